@@ -43,7 +43,7 @@ struct AdjArgs {
   const float* dzx2;                  // crest mode: the second jumps, else NULL
   const float* dzy2;
   const unsigned long long* n_steps;  // per design: steps of the forward run
-  const double* seg;                  // per design [K][3]: (dt, rain, t) of this segment's steps
+  const double* seg;                  // per design [K][kLog]: the records of this segment's steps
   int K;
   unsigned long long step0;           // global index of the segment's first step
   const float* tape;                  // [K][n_designs][3][N]: state at step step0 + j
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kTileThreads, 6) k_adj_replay(const AdjArgs A,
   const size_t N = (size_t)nx * ny, SX = (size_t)ny * (nx + 1), SY = (size_t)(ny + 1) * nx;
   const float* X = A.tape + ((size_t)j * A.n_designs + d) * 3 * N;
   float* Y = const_cast<float*>(A.tape) + ((size_t)(j + 1) * A.n_designs + d) * 3 * N;
-  const double* sg = A.seg + ((size_t)d * A.K + j) * 3;
+  const double* sg = A.seg + ((size_t)d * A.K + j) * kLog;
   const StepK k = step_consts(A.P, sg[0], sg[1]);
   const float* dzx = A.dzx + d * SX;
   const float* dzy = A.dzy + d * SY;
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(kTileThreads) k_adj_step(const AdjArgs A, int 
     return;
   }
   const float* X = A.tape + ((size_t)j * A.n_designs + d) * 3 * N;
-  const double* sg = A.seg + ((size_t)d * A.K + j) * 3;
+  const double* sg = A.seg + ((size_t)d * A.K + j) * kLog;
   const StepK k = step_consts(A.P, sg[0], sg[1]);
   const float* dzx = A.dzx + d * SX;
   const float* dzy = A.dzy + d * SY;

@@ -78,7 +78,7 @@ inline int adj_rows_for(int nx, int ny, int n_designs, int sm_count) {
 __global__ void k_adj_plan(const AdjArgs A, PlainCtl* ctl) {
   const int j = blockIdx.x, d = blockIdx.y;
   PlainCtl* c = ctl + (size_t)j * A.n_designs + d;
-  const double* sg = A.seg + ((size_t)d * A.K + j) * 3;
+  const double* sg = A.seg + ((size_t)d * A.K + j) * kLog;
   const bool live = A.step0 + j < A.n_steps[d];
   if ((int)threadIdx.x < A.P.inflow.n)
     c->inf[threadIdx.x] = live ? inflow_values(A.P.inflow, threadIdx.x, sg[2], A.P.g) : make_float2(0.0f, 0.0f);
@@ -87,6 +87,7 @@ __global__ void k_adj_plan(const AdjArgs A, PlainCtl* ctl) {
     c->par = 0;
     c->step = A.step0 + j;
     c->k = step_consts(A.P, sg[0], sg[1]);
+    c->k.exact = sg[3] != 0.0 ? 1u : 0u;
     c->pl.dt = sg[0]; c->pl.rain = sg[1]; c->pl.t_new = sg[2] + sg[0]; c->pl.hits = false;
   }
 }
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, ITR_ADJ_MIN_BLOCKS) k_adj_band
     return;
   }
   const float* X = A.tape + ((size_t)j * A.n_designs + d) * 3 * N;
-  const double* sg = A.seg + ((size_t)d * A.K + j) * 3;
+  const double* sg = A.seg + ((size_t)d * A.K + j) * kLog;
   const StepK k = step_consts(A.P, sg[0], sg[1]);
   const float* dzx = A.dzx + d * SX;
   const float* dzy = A.dzy + d * SY;

@@ -34,6 +34,7 @@
 // so an aborted design stops at once.
 #pragma once
 #include <cooperative_groups.h>
+#include <type_traits>
 #include "itr_device.cuh"
 
 namespace itr {
@@ -77,7 +78,7 @@ struct BatchArgs {
   int max_rows;
   DesignOut* out;     // n_designs
   unsigned long long max_steps;
-  unsigned exact;     // 1: every paired reciprocal through the IEEE routine (checking)
+  unsigned exact;     // 1: every step through the scalar path (checking)
   unsigned wait_limit;   // try_wait rounds of a single-CTA design's barrier wait before status 5
   unsigned stall_test;   // 1: that barrier expects one arrival more than the CTA makes (timeout test)
   const WarmStart* warm;   // optional, per design (state NULL: cold start)
@@ -350,13 +351,6 @@ ITR_DEV Cell2 cell2_of(const Cell& a, const Cell& b) {
 }
 ITR_DEV Cell cx(const Cell2& a) { Cell c; c.h = a.h.x; c.qx = a.qx.x; c.qy = a.qy.x; c.u = a.u.x; c.v = a.v.x; c.c = a.c.x; return c; }
 ITR_DEV Cell cy(const Cell2& a) { Cell c; c.h = a.h.y; c.qx = a.qx.y; c.qy = a.qy.y; c.u = a.u.y; c.v = a.v.y; c.c = a.c.y; return c; }
-ITR_DEV FaceF fx_(const Face2& f) { FaceF r; r.m = f.m.x; r.nl = f.nl.x; r.nr = f.nr.x; r.t = f.t.x; return r; }
-ITR_DEV FaceF fy_(const Face2& f) { FaceF r; r.m = f.m.y; r.nl = f.nl.y; r.nr = f.nr.y; r.t = f.t.y; return r; }
-ITR_DEV Face2 face2_of(const FaceF& a, const FaceF& b) {
-  Face2 f;
-  f.m = make_float2(a.m, b.m); f.nl = make_float2(a.nl, b.nl); f.nr = make_float2(a.nr, b.nr); f.t = make_float2(a.t, b.t);
-  return f;
-}
 ITR_DEV Cell2 shfl_up_cell2(const Cell2& c) {
   Cell2 o;
   o.h = make_float2(__shfl_up_sync(0xffffffffu, c.h.x, 1), __shfl_up_sync(0xffffffffu, c.h.y, 1));
@@ -510,6 +504,15 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
   const WarmStart* WS = (A.warm && A.warm[d].state) ? &A.warm[d] : nullptr;
   const double t_start = WS ? WS->t : 0.0;
   double s0_l = 0.0, v0_l = 0.0;
+  bool uns_l = false, neg_l = false;   // initial depths out of the bounds of the branch-free step; a jump or stage out of them
+  if (CREST) {
+    for (size_t i = (size_t)ra * nxp1 + tid; i < (size_t)rb * nxp1; i += blockDim.x)
+      neg_l = neg_l || !jump_safe(A.dzx[(size_t)d * ny * nxp1 + i]) || !jump_safe(A.dzx2[(size_t)d * ny * nxp1 + i]);
+    for (size_t i = (size_t)ra * nx + tid; i < (size_t)(rb + 1) * nx; i += blockDim.x)
+      neg_l = neg_l || !jump_safe(A.dzy[(size_t)d * (ny + 1) * nx + i]) || !jump_safe(A.dzy2[(size_t)d * (ny + 1) * nx + i]);
+  }
+  if (BND && A.bh)
+    for (int i = tid; i < nbc; i += blockDim.x) neg_l = neg_l || !stage_safe(A.bc[i], bh[i]);
   for (int idx = tid; idx < nr * nx; idx += blockDim.x) {
     const int r = ra + idx / nx, c = idx % nx;
     if (WS) {
@@ -528,6 +531,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
     sm.S4[idx] = make_float4(h, 0.0f, 0.0f, u);
     sm.S2[idx] = make_float2(v, cc);
     sm.PK[idx] = 0.0f;
+    uns_l = uns_l || !depth_safe(P, h);
     const double hd = (double)h;
     v0_l += hd;
     if (hd > P.h_dry) {  // initial_smax (solver.rs:314-332) with q = 0
@@ -555,14 +559,16 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) { double t = __shfl_xor_sync(0xffffffffu, sw, o); sw = sw > t ? sw : t; }
     const double vw = warp_sum_d(v0_l);
-    if (lane == 0) { sm.red[wid * 8 + 0] = sw; sm.red[wid * 8 + 1] = vw; }
+    const bool un = __any_sync(0xffffffffu, uns_l), ng = __any_sync(0xffffffffu, neg_l);
+    if (lane == 0) { sm.red[wid * 8 + 0] = sw; sm.red[wid * 8 + 1] = vw; sm.red[wid * 8 + 2] = (un ? 1.0 : 0.0) + (ng ? 2.0 : 0.0); }
   }
   if (CLUSTERED) { cluster_arrive(); cluster_wait(); } else __syncthreads();
   if (SKIP) row_flags(sm, 0, nr, nr_max, nx, W, wid, nwarps, lane);   // wetness of the initial state (parity 0)
   double s0 = 0.0, v0 = 0.0;
+  int flags = 0;
   for (int qq = 0; qq < C; ++qq) {
     const double* rr = CLUSTERED ? remote(sm.red, qq) : sm.red;
-    for (int w = 0; w < nwarps; ++w) { const double a = rr[w * 8 + 0]; s0 = s0 > a ? s0 : a; v0 += rr[w * 8 + 1]; }
+    for (int w = 0; w < nwarps; ++w) { const double a = rr[w * 8 + 0]; s0 = s0 > a ? s0 : a; v0 += rr[w * 8 + 1]; flags |= (int)rr[w * 8 + 2]; }
   }
   v0 *= P.area;
   if (WS) v0 = WS->v0;
@@ -574,6 +580,10 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
   unsigned sync_index = WS ? WS->sync_index : 0u;
   double dt_cfl = WS ? WS->dt_cfl : (s0 > 0.0 ? dmin_num(P.cfl / s0, P.dt_max) : P.dt_max);
   double acc_rain = WS ? WS->acc_rain : 0.0;
+  // Scalar-path steps: always (checking, a jump or stage depth out of bounds), or until the state is known to be
+  // bounded (a warm start's from the dt its wave rate gave).
+  const bool always_exact = A.exact != 0u || (flags & 2) != 0;
+  bool unsafe = WS ? !(P.cfl <= 0.99 * (double)P.s_safe * dt_cfl) : (flags & 1) != 0;
   int status = 0;
   unsigned breach_cell = 0, breach_sync = 0;
   double violation = 0.0, lower_bound = 0.0, volume = WS ? WS->volume : v0, rel_res = WS ? WS->rel_res : 0.0;
@@ -663,6 +673,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
           }
           if (q == 0 && tid == 0) A.fallback_t[d] = t;
           locked_live = false;
+          unsafe = true;   // (the snapshot's bound is not kept: one step through the scalar path)
           gs.full();   // the restored state of every CTA visible before the next step
           continue;
         }
@@ -670,7 +681,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
     }
     const StepPlan pl = LOCKED ? plan_step_dt_c(P, t, sync_index, dt_pick, rcur) : plan_step_c(P, t, sync_index, dt_cfl, rcur);
     StepK k = step_consts(P, pl.dt, pl.rain);
-    k.exact = A.exact;
+    k.exact = always_exact || unsafe ? 1u : 0u;
     const int sp = (int)(step & 1ull);
     if (BND) {
       inf_cur = sm.INF + sp * kMaxInflow;
@@ -684,8 +695,8 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
         }
       }
     }
-    float smax_l = 0.0f, infil_l = 0.0f, fix_l = 0.0f;
-    bool bad_l = false;
+    float smax_l = 0.0f, infil_l = 0.0f, fix_l = 0.0f, low_l = 0.0f;
+    bool uns_l = false;
     int par = 0;
 
     // ---- strip pre-phase: first row, its west faces, the strip's top y-faces ----
@@ -721,8 +732,13 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
       const Cell2 above = cell2_of(a0, a1);
       const float2 dy0 = make_float2(__ldg(A.dzy + oy0 + fy), __ldg(A.dzy + oy1 + fy));
       const float2 dy1 = CREST ? make_float2(__ldg(A.dzy2 + oy0 + fy), __ldg(A.dzy2 + oy1 + fy)) : f2(0.0f);
-      fW = face2<true, CREST>(left.h, left.u, left.v, left.c, cur.h, cur.u, cur.v, cur.c, dx0, dx1, k);
-      fN = face2<false, CREST>(above.h, above.u, above.v, above.c, cur.h, cur.u, cur.v, cur.c, dy0, dy1, k);
+      if (!k.exact) {
+        fW = face2<true, CREST>(left.h, left.u, left.v, left.c, cur.h, cur.u, cur.v, cur.c, dx0, dx1, k);
+        fN = face2<false, CREST>(above.h, above.u, above.v, above.c, cur.h, cur.u, cur.v, cur.c, dy0, dy1, k);
+      } else {
+        fW = face2_exact<true, CREST>(left.h, left.u, left.v, left.c, cur.h, cur.u, cur.v, cur.c, dx0, dx1, k);
+        fN = face2_exact<false, CREST>(above.h, above.u, above.v, above.c, cur.h, cur.u, cur.v, cur.c, dy0, dy1, k);
+      }
       if (lane == 0) {
         sm.XB[CK(((par * S + s) * W + wis) * 2 + 0, sm.nxb, 7)] = f4(fx_(fW));
         sm.XB[CK(((par * S + s) * W + wis) * 2 + 1, sm.nxb, 7)] = f4(fy_(fW));
@@ -803,7 +819,8 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
         if (!last && !skip_next) {   // the next row's west faces
           nxt = load_pair(lr + 1, r + 1);
           const Cell2 left = left_pair(nxt, lr + 1, r + 1);
-          fWn = face2<true, CREST>(left.h, left.u, left.v, left.c, nxt.h, nxt.u, nxt.v, nxt.c, d_xn, d_xn2, k);
+          fWn = k.exact ? face2_exact<true, CREST>(left.h, left.u, left.v, left.c, nxt.h, nxt.u, nxt.v, nxt.c, d_xn, d_xn2, k)
+                        : face2<true, CREST>(left.h, left.u, left.v, left.c, nxt.h, nxt.u, nxt.v, nxt.c, d_xn, d_xn2, k);
           if (lane == 0) {
             sm.XB[CK((((par ^ 1) * S + s) * W + wis) * 2 + 0, sm.nxb, 9)] = f4(fx_(fWn));
             sm.XB[CK((((par ^ 1) * S + s) * W + wis) * 2 + 1, sm.nxb, 9)] = f4(fy_(fWn));
@@ -854,27 +871,37 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
         if (cell1) b1 = ghost_y(cy(cur), bc_s + col1, false);
         below = cell2_of(b0, b1);
       }
-      // new faces and the cell update; every lane of the strip computes (lanes past the grid
-      // on zeros or ghost values), so the warp-uniform reciprocal fallback sees all 32 lanes
+      // new faces and the cell update; every lane of the strip computes (lanes past the grid on
+      // zeros or ghost values: finite). One branch per row picks the branch-free arithmetic or the
+      // scalar path, so the row's two faces, update and velocities are one straight-line block.
       CellNew2 o;
       float2 uu, vv;
-      if (!last) {
-        // (the next row's west faces are computed even when that row will be skipped: one
-        // straight-line body keeps both faces' instructions interleaved)
-        fS = face2<false, CREST>(cur.h, cur.u, cur.v, cur.c, nxt.h, nxt.u, nxt.v, nxt.c, d_s, d_s2, k);
-        fWn = face2<true, CREST>(left.h, left.u, left.v, left.c, nxt.h, nxt.u, nxt.v, nxt.c, d_xn, d_xn2, k);
-      } else if (bottom) {
-        fS = face2<false, CREST>(cur.h, cur.u, cur.v, cur.c, below.h, below.u, below.v, below.c, d_s, d_s2, k);
+      if (!k.exact) {
+        if (!last) {
+          // (the next row's west faces are computed even when that row will be skipped: one
+          // straight-line body keeps both faces' instructions interleaved)
+          fS = face2<false, CREST>(cur.h, cur.u, cur.v, cur.c, nxt.h, nxt.u, nxt.v, nxt.c, d_s, d_s2, k);
+          fWn = face2<true, CREST>(left.h, left.u, left.v, left.c, nxt.h, nxt.u, nxt.v, nxt.c, d_xn, d_xn2, k);
+        } else if (bottom) {
+          fS = face2<false, CREST>(cur.h, cur.u, cur.v, cur.c, below.h, below.u, below.v, below.c, d_s, d_s2, k);
+        } else {
+          fS = fS_in;
+        }
+        o = update_cell2(cur.h, cur.qx, cur.qy, fW, fE, fN, fS, wet_r, gn2_r, k);
+        vel2(o.h, o.qx, o.qy, k, uu, vv);
       } else {
-        fS = fS_in;
-      }
-      o = update_cell2(cur.h, cur.qx, cur.qy, fW, fE, fN, fS, wet_r, gn2_r, k);
-      {
-        const float2 h2 = mul2(o.h, o.h, k.nz);
-        const float2 inv = rcp2f(add2(h2, max2(h2, f2(heps2))), k.exact);
-        const float2 tt = mul2(add2(o.h, o.h), inv, k.nz);
-        uu = mul2(o.qx, tt, k.nz);
-        vv = mul2(o.qy, tt, k.nz);
+        if (!last) {
+          fS = face2_exact<false, CREST>(cur.h, cur.u, cur.v, cur.c, nxt.h, nxt.u, nxt.v, nxt.c, d_s, d_s2, k);
+          fWn = face2_exact<true, CREST>(left.h, left.u, left.v, left.c, nxt.h, nxt.u, nxt.v, nxt.c, d_xn, d_xn2, k);
+        } else if (bottom) {
+          fS = face2_exact<false, CREST>(cur.h, cur.u, cur.v, cur.c, below.h, below.u, below.v, below.c, d_s, d_s2, k);
+        } else {
+          fS = fS_in;
+        }
+        o = update_cell2_exact(cur.h, cur.qx, cur.qy, fW, fE, fN, fS, wet_r, gn2_r, k);
+        const Vel2 w = vel2_exact(o.h, o.qx, o.qy, P.g_f, heps2);
+        uu = w.u; vv = w.v;
+        uns_l = uns_l || (cell0 && !state_safe(P, o.s.x)) || (cell1 && !state_safe(P, o.s.y));
       }
       if (!last && lane == 0) {
         sm.XB[CK((((par ^ 1) * S + s) * W + wis) * 2 + 0, sm.nxb, 9)] = f4(fx_(fWn));
@@ -895,7 +922,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
         const float pk = sm.PK[li];
         if (o.h.x > pk) sm.PK[li] = o.h.x;
         smax_l = rmax(smax_l, o.s.x);
-        bad_l = bad_l || o.bad.x;
+        low_l = fminf(low_l, o.low.x);
         infil_l += o.infil.x;
         fix_l += o.fix.x;
       }
@@ -906,7 +933,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
         const float pk = sm.PK[li];
         if (o.h.y > pk) sm.PK[li] = o.h.y;
         smax_l = rmax(smax_l, o.s.y);
-        bad_l = bad_l || o.bad.y;
+        low_l = fminf(low_l, o.low.y);
         infil_l += o.infil.y;
         fix_l += o.fix.y;
       }
@@ -923,11 +950,12 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
     // ---- end of step: CFL max, health, per-warp ledger partials ----
     {
       const float m = warp_max_f(smax_l);
-      const unsigned b = __any_sync(0xffffffffu, bad_l) ? 1u : 0u;
+      const bool bad_l = low_l < -k.h_dry || __float_as_uint(low_l) == 0xff800000u;
+      const unsigned b = (__any_sync(0xffffffffu, bad_l) ? 1u : 0u) | (__any_sync(0xffffffffu, uns_l) ? 2u : 0u);
       const float wi = warp_sum_f(infil_l), wf = warp_sum_f(fix_l);
       if (lane == 0) {
         if (m > 0.0f) atomicMax(&sm.slot[sp], __float_as_uint(m));
-        if (b) atomicOr(&sm.slot[2 + sp], 1u);
+        if (b) atomicOr(&sm.slot[2 + sp], b);
         sm.WS[(sp * nwarps + wid) * 2 + 0] = wi;
         sm.WS[(sp * nwarps + wid) * 2 + 1] = wf;
       }
@@ -985,7 +1013,8 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
     step += 1;
     t = pl.t_new;
     acc_rain += pl.rain * P.area * P.wet_count;
-    if (badv) { status = 3; break; }
+    if (badv & 1u) { status = 3; break; }
+    unsafe = !state_safe(P, __uint_as_float(smax_bits)) || (badv & 2u) != 0u;
     dt_cfl = smax > 0.0 ? P.cfl / smax : P.dt_max;
     if constexpr (LOCKED) s_cur = smax;
     if (pl.hits) {

@@ -455,9 +455,44 @@ static RunParams make_run_params(const itr_params* p, const itr_grid* g) {
   P.inv_dx_f = (float)(1.0 / g->dx); P.inv_dy_f = (float)(1.0 / g->dy);
   P.h_dry_f = (float)p->h_dry; P.heps2_f = (float)(p->h_eps * p->h_eps); P.q_min_f = (float)1e-30;
   P.nz = -0.0f;
+  P.s_safe = -1.0f;   // safe_rate_limit, where the kernels have a branch-free step
   P.inflow.n = 0;   // build_boundaries fills the groups
   P.inflow.scale = p->inflow_scale;
   return P;
+}
+
+// RunParams::s_safe: the largest wave rate s = max (|u| + c) / dx + (|v| + c) / dy of a state whose
+// step may take the branch-free square roots and reciprocals (itr_device.cuh, sqrt2 and rcp2), or
+// -1 when these parameters bound no state (every step then takes the scalar path).
+// With V = s max(dx, dy): |u| + 2 c <= V, so h <= V^2 / 4 g, |q| <= V^3 / 27 g, a face's momentum
+// flux (HLL's star flux included) <= 0.3 V^4 / g, and the momentum after the flux update
+// <= V^3 / 27 g + 4 (dt / dx) 0.3 V^4 / g, which must stay below 2^39 so that the sum of two
+// squares stays below sqrt2's 2^80. A stage ghost copies q into its own depth hs (0, or 2^-15 m to
+// 2^10 m, else the kernels flag the design): its flux is <= 6 q^2 / hs. The other operands follow:
+// HLL's denominator is a difference of speeds of opposite sign, 2^-97 .. 3 V; the friction term is
+// at most 1 + dt g n^2 2^40 h_dry^(-7/3); the velocity's h^2 + max(h^2, h_eps^2) is at least
+// h_eps^2 and at most 2^81. dt_most: the longest step (dt_max or the locked schedule's longest).
+static float safe_rate_limit(const RunParams& P, const float* wet, const float* gn2, size_t N, bool bnd, double dt_most) {
+  auto in = [](double v, double lo, double hi) { return v >= lo && v <= hi; };   // false for NaN
+  bool ok = in(P.g, 0.25, 64.0) && in(P.dx, 1e-3, 1e6) && in(P.dy, 1e-3, 1e6) && in(dt_most, 0.0, 4096.0) && in(P.sync, 0.0, 1e9) &&
+            in(P.h_dry, 0x1p-24, 1024.0) && in(P.h_eps, 0x1p-48, 1024.0) && in(P.infil, 0.0, 1.0);
+  for (int i = 0; i < P.rain.n; ++i) ok = ok && in(P.rain.r[i], -1.0, 1.0);
+  for (int g = 0; g < P.inflow.n; ++g)
+    for (int i = P.inflow.off[g]; i < P.inflow.off[g + 1]; ++i) ok = ok && in(P.inflow.q[i] * P.inflow.inv_len[g] * P.inflow.scale, -256.0, 256.0);
+  float wl = 0.0f, wh = 0.0f, gl = 0.0f, gh = 0.0f;
+  bool num = true;
+  for (size_t i = 0; i < N; ++i) {
+    wl = std::min(wl, wet[i]); wh = std::max(wh, wet[i]);
+    gl = std::min(gl, gn2[i]); gh = std::max(gh, gn2[i]);
+    num = num & (wet[i] == wet[i]) & (gn2[i] == gn2[i]);
+  }
+  ok = ok && num && wl >= 0.0f && wh <= 1.0f && gl >= 0.0f && gh <= 1024.0f;
+  if (!ok) return -1.0f;
+  const double r = (dt_most + 1e-9 * P.sync) / std::min(P.dx, P.dy);
+  if (!(dt_most * gh * 0x1p40 * std::pow(P.h_dry, -7.0 / 3.0) < 0x1p120) || !(r <= 4096.0)) return -1.0f;
+  double V = std::min(1024.0, std::pow(0x1p38 * P.g / (1.2 * r + 1.0), 0.25));
+  if (bnd) V = std::min(V, std::pow(0x1p38 * 729.0 * P.g * P.g / (24.0 * 0x1p15 * r + 1.0), 1.0 / 6.0));
+  return (float)(0.99 * V / std::max(P.dx, P.dy));
 }
 
 // Device boundary codes and inflow groups of a grid (boundary.rs:12-87): an inflow cell's
@@ -726,7 +761,7 @@ static int run_plain_design(itr_ctx* ctx, PlainArgs& A, int n_blocks, dim3 grid,
 // Adjoint request: while set, run_batch takes the tiled path and records a tape.
 struct Vjp {
   int K;                                  // checkpoint interval (steps)
-  std::vector<std::vector<double>> dt;    // per design: (dt, rain, t) of every step taken
+  std::vector<std::vector<double>> dt;    // per design: the record (kLog values) of every step taken
   uint64_t blocks = 0;                    // checkpoints written (one per block of K steps)
   double* gx;                             // host outputs
   double* gy;
@@ -807,17 +842,15 @@ static int run_tiled_batch(itr_ctx* ctx, PlainArgs& A, int n, dim3 tgrid, int* l
     cudaError_t e = cudaMemcpyAsync(hc, A.ctl, (size_t)n * sizeof(PlainCtl), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) { rc = fail(ctx, ITR_DEVICE_ERROR, "tiled run: %s", cudaGetErrorString(e)); break; }
-    if (tape) {   // (dt, rain, t) of this block's steps, from the ring of 2K slots
+    if (tape) {   // the records of this block's steps, from the ring of 2K slots
       double* ring = ctx->aRingH.as<double>();
-      e = cudaMemcpy(ring, A.dt_log, (size_t)n * 2 * K * 3 * 8, cudaMemcpyDeviceToHost);
+      e = cudaMemcpy(ring, A.dt_log, (size_t)n * 2 * K * kLog * 8, cudaMemcpyDeviceToHost);
       if (e != cudaSuccess) { rc = fail(ctx, ITR_DEVICE_ERROR, "tape: %s", cudaGetErrorString(e)); break; }
       const uint64_t s0 = polls * (uint64_t)K;
       for (int d = 0; d < n; ++d)
         for (uint64_t s = s0; s < s0 + K && s < hc[d].step; ++s) {
-          const double* q = ring + ((size_t)d * 2 * K + (size_t)(s % (2 * K))) * 3;
-          tape->dt[d].push_back(q[0]);
-          tape->dt[d].push_back(q[1]);
-          tape->dt[d].push_back(q[2]);
+          const double* q = ring + ((size_t)d * 2 * K + (size_t)(s % (2 * K))) * kLog;
+          tape->dt[d].insert(tape->dt[d].end(), q, q + kLog);
         }
     }
     bool all = true;
@@ -898,8 +931,8 @@ static int vjp_backward(itr_ctx* ctx, const PlainArgs& F, const itr_objective* o
   CU(ctx->aTape.ensure((size_t)K * S3 * 4));
   CU(ctx->aLA.ensure(S3 * 4)); CU(ctx->aLB.ensure(S3 * 4));
   CU(ctx->aGx.ensure((size_t)n * SX * 8)); CU(ctx->aGy.ensure((size_t)n * SY * 8));
-  // (dt, rain, t) of every segment, laid out [segment][design][K][3], uploaded once
-  const size_t seg_elems = (size_t)n * K * 3;
+  // the step records of every segment, laid out [segment][design][K][kLog], uploaded once
+  const size_t seg_elems = (size_t)n * K * kLog;
   CU(ctx->aSeg.ensure(nblocks * seg_elems * 8));
   CU(ctx->aRingH.ensure(nblocks * seg_elems * 8));
   CU(cudaMemsetAsync(ctx->aLA.p, 0, S3 * 4, st));
@@ -935,10 +968,8 @@ static int vjp_backward(itr_ctx* ctx, const PlainArgs& F, const itr_objective* o
       for (int j = 0; j < K; ++j) {
         const uint64_t s = b * K + j;
         const bool have = s < nst[d];
-        double* q = segh + b * seg_elems + ((size_t)d * K + j) * 3;
-        q[0] = have ? V->dt[d][3 * s] : 0.0;
-        q[1] = have ? V->dt[d][3 * s + 1] : 0.0;
-        q[2] = have ? V->dt[d][3 * s + 2] : 0.0;
+        double* q = segh + b * seg_elems + ((size_t)d * K + j) * kLog;
+        for (int v = 0; v < kLog; ++v) q[v] = have ? V->dt[d][kLog * s + v] : 0.0;
       }
   CU(cudaMemcpyAsync(ctx->aSeg.p, segh, nblocks * seg_elems * 8, cudaMemcpyHostToDevice, st));
   // Two tapes: segment b's replay fills tape b % 2 on the second stream while the backward
@@ -1254,6 +1285,11 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
   rc = build_boundaries(ctx, g, P.inflow, st + o_bc);
   if (rc != ITR_OK) return rc;
   const bool bnd = has_stage || P.inflow.n > 0;
+  {
+    double dt_most = P.dt_max;
+    if (!ctx->recording) for (double v : ctx->locked_dt) dt_most = std::max(dt_most, v);
+    P.s_safe = safe_rate_limit(P, g->wet, g->gn2, N, bnd, dt_most);
+  }
   if (has_stage && !M)
     for (int d = 0; d < n; ++d) stage_depths(g, ds[d].z_edge, reinterpret_cast<float*>(st + o_bh) + d * NB);
   if (M) {
@@ -1420,6 +1456,7 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
     if (e == cudaSuccess) e = ctx->tctl.ensure((size_t)n * sizeof(PlainCtl));
     memset(&A, 0, sizeof(A));
     A.P = P; A.nx = nx; A.ny = ny; A.mode = g->mode; A.n_designs = n;
+    if (ctx->exact_special) A.P.s_safe = -1.0f;
     A.wet = reinterpret_cast<const float*>(dv + o_wet);
     A.gn2 = reinterpret_cast<const float*>(dv + o_gn2);
     A.bc = reinterpret_cast<const uint8_t*>(dv + o_bc);
@@ -1615,8 +1652,8 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
     if (ctx->vjp) {
       const int K = ctx->vjp->K;
       CU(ctx->aTpk.ensure((size_t)n * N * 4));
-      CU(ctx->aRing.ensure((size_t)n * 2 * K * 3 * 8));
-      CU(ctx->aRingH.ensure((size_t)n * 2 * K * 3 * 8));
+      CU(ctx->aRing.ensure((size_t)n * 2 * K * kLog * 8));
+      CU(ctx->aRingH.ensure((size_t)n * 2 * K * kLog * 8));
       A.tpk = ctx->aTpk.as<unsigned>();
       A.dt_log = ctx->aRing.as<double>();
       A.max_log = 2 * K;
@@ -1906,6 +1943,7 @@ extern "C" int itr_gpu_record_baseline(itr_ctx* ctx, const itr_params* p, const 
     R->open_rows[row] = 1;
   }
   if (has_stage) { R->bh.resize(NB); stage_depths(g, base->z_edge, R->bh.data()); }
+  R->P.s_safe = safe_rate_limit(R->P, g->wet, g->gn2, N, has_stage || R->P.inflow.n > 0, R->P.dt_max);
   // the base's run on the tiled path, checkpointed every K steps, with its whole ledger
   const int max_rows = (int)R->P.n_sync;
   std::vector<double> led((size_t)(max_rows > 0 ? max_rows : 1) * 8);

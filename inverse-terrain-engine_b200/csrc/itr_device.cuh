@@ -43,7 +43,7 @@ ITR_DEV float rcbrt(float x) {
 struct StepK {
   float g, g_half, dt, dtdx, dtdy, inv_dx, inv_dy, h_dry, heps2, q_min, rain, cap;
   float nz;   // -0.0f read from the kernel parameters at run time (see mul2)
-  unsigned exact;   // 1: paired reciprocals always through the IEEE routine (checking)
+  unsigned exact;   // 1: this step through the scalar path (state or parameters not known to be bounded, or checking)
 };
 
 // A face flux tuple: mass, normal momentum seen from the low-index (n_l) and high-index
@@ -379,7 +379,19 @@ struct RunParams {
   // step-invariant f32 constants (solver.rs:269-285), rounded once on the host
   float g_f, g_half_f, inv_dx_f, inv_dy_f, h_dry_f, heps2_f, q_min_f;
   float nz;   // -0.0f, supplied at run time (see mul2)
+  float s_safe;   // largest wave rate of a state whose step may take the branch-free roots (safe_rate_limit)
 };
+
+// Whether a state with this largest wave rate (|u| + c) / dx + (|v| + c) / dy is bounded (NaN is not).
+ITR_DEV bool state_safe(const RunParams& P, float smax) { return smax <= P.s_safe; }
+// The same of an initial depth (at rest): finite, not negative (-0 neither), celerity within the limit.
+ITR_DEV bool depth_safe(const RunParams& P, float h) {
+  return !(__float_as_uint(h) >> 31) && sqrtf(P.g_f * h) * (P.inv_dx_f + P.inv_dy_f) <= P.s_safe;
+}
+// A crest jump is a height above a cell; a negative one would deepen the water.
+ITR_DEV bool jump_safe(float d) { return !(d < 0.0f); }
+// A stage ghost's depth (boundary code 2): 0, or not so small that the momentum it copies becomes a huge velocity.
+ITR_DEV bool stage_safe(int code, float hs) { return code != 2 || hs == 0.0f || (hs >= 0x1p-15f && hs <= 1024.0f); }
 
 ITR_DEV double dmin_num(double a, double b) { return a < b ? a : b; }  // operands never NaN here
 
@@ -520,20 +532,22 @@ struct DesignOut {
 }  // namespace itr
 
 // --------------------------------------------------------------- two cells at once ----
-// The same arithmetic on pairs of cells: every add and multiply is a paired FP32
-// instruction (__fadd2_rn / __fmul2_rn: each component is the IEEE round-to-nearest
-// result of the scalar operation), every compare, select, square root and reciprocal is
-// done per component. Association order is the scalar code's, so each component has the
-// same bits as the scalar path (and as the reference's f32 kernel).
+// The same arithmetic on pairs of cells: adds and multiplies are paired FP32 instructions,
+// compares, selects and the estimates behind square roots and reciprocals are done per
+// component. Association order is the scalar code's, so each component has the same bits as the
+// scalar path (and as the reference's f32 kernel).
+//
+// Two forms. The *_exact functions call the scalar path, right for every input. The others run
+// branch-free square roots and reciprocals whose operands must lie in stated ranges; a kernel
+// takes them for a whole step when StepK::exact is 0, which the integrator sets only when the
+// state it starts from and the run's parameters are bounded (safe_rate_limit below).
 namespace itr {
 
 struct B2 { bool x, y; };
 struct Face2 { float2 m, nl, nr, t; };
 
 ITR_DEV float2 f2(float a) { return make_float2(a, a); }
-// Packed FP32 pairs through PTX with an explicit .rn rounding modifier: such instructions are
-// never contracted into fused multiply-adds (the float2 intrinsics may be), so each component
-// is exactly the scalar IEEE result.
+// Packed FP32 pairs through PTX with an explicit .rn rounding modifier.
 ITR_DEV unsigned long long pk2(float2 a) {
   unsigned long long r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
@@ -555,109 +569,104 @@ ITR_DEV float2 sub2(float2 a, float2 b) {
   return upk2(r);
 }
 // Paired product as fma(a, b, -0): exactly round(a*b) for every input (x + -0 == x, zeros
-// keep their sign). The -0 must not be a compile-time constant, else the compiler turns the
-// fma back into a multiply and fuses it with the next add (observed on sm_100a), which
-// would round once instead of twice; it is the kernel parameter StepK::nz.
+// keep their sign). mul.rn.f32x2 followed by an add is fused on sm_100a in spite of its .rn
+// (measured: 42 % of random a*b+c differ from the twice-rounded value), and so is an fma whose
+// -0 is a compile-time constant; -0 is therefore the kernel parameter StepK::nz.
 ITR_DEV float2 mul2(float2 a, float2 b, float nz) {
   unsigned long long r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pk2(a)), "l"(pk2(b)), "l"(pk2(make_float2(nz, nz))));
   return upk2(r);
 }
-ITR_DEV float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
-ITR_DEV float2 sel2(B2 c, float2 a, float2 b) { return make_float2(c.x ? a.x : b.x, c.y ? a.y : b.y); }
-ITR_DEV float2 max2(float2 a, float2 b) { return make_float2(rmax(a.x, b.x), rmax(a.y, b.y)); }
-ITR_DEV float2 min2(float2 a, float2 b) { return make_float2(rmin(a.x, b.x), rmin(a.y, b.y)); }
-ITR_DEV B2 gt2(float2 a, float b) { return B2{a.x > b, a.y > b}; }
-ITR_DEV B2 ge2(float2 a, float b) { return B2{a.x >= b, a.y >= b}; }
-ITR_DEV B2 le2(float2 a, float b) { return B2{a.x <= b, a.y <= b}; }
-ITR_DEV B2 lt2(float2 a, float b) { return B2{a.x < b, a.y < b}; }
-ITR_DEV B2 not2(B2 a) { return B2{!a.x, !a.y}; }
-ITR_DEV B2 and2(B2 a, B2 b) { return B2{a.x && b.x, a.y && b.y}; }
-ITR_DEV B2 or2(B2 a, B2 b) { return B2{a.x || b.x, a.y || b.y}; }
-ITR_DEV float2 sqrt2(float2 a) { return make_float2(sqrt_rn(a.x), sqrt_rn(a.y)); }
-ITR_DEV float2 rcp2(float2 a) { return make_float2(rcp(a.x), rcp(a.y)); }
+// The plain paired product, for results that no addition reads (only products, estimates and
+// selects of these) and for exact ones (a power of two), where fusing changes nothing.
+ITR_DEV float2 mulp2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pk2(a)), "l"(pk2(b)));
+  return upk2(r);
+}
 ITR_DEV float2 fma2(float2 a, float2 b, float2 c) {
   unsigned long long r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pk2(a)), "l"(pk2(b)), "l"(pk2(c)));
   return upk2(r);
 }
-
-// ---- Reciprocal without the IEEE routine's per-lane slow-path branch ----
-// 1/x as one Newton step from the hardware estimate (textbook FMA refinement: P. Markstein,
-// IBM J. Res. Dev. 34(1), 1990; J.-M. Muller et al., Handbook of Floating-Point Arithmetic,
-// 2nd ed., 2018, ch. 4): y = est(1/x); e = fma(-x, y, 1); y + y e. Checked against CUDA's
-// IEEE reciprocal on every 32-bit input with |x| in [2^-125, 2^126): identical. An operand
-// outside that range (zero, infinity, NaN, tiny or huge) sends the whole warp through the
-// IEEE routine for that call, as does k.exact; the branch is warp-uniform, so the common
-// path carries no divergence point. Results are the IEEE ones for every input. The step
-// kernel's reciprocals (HLL denominator, friction, velocity) are in range for every
-// healthy state: the fallback is for NaN/infinite states and for checking.
-ITR_DEV float rcp_est(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
-// In range: |x| in [2^-125, 2^126), i.e. biased exponent 2 .. 252. Two compares of |x| (the
-// absolute value is an operand modifier); NaN, zero and infinity fail them.
-ITR_DEV bool rcp_in(float x) { return fabsf(x) >= 0x1p-125f && fabsf(x) < 0x1p126f; }
-
-ITR_DEV float2 rcp2f(float2 x, unsigned exact) {
-  const float2 y = make_float2(rcp_est(x.x), rcp_est(x.y));
-  const float2 e = fma2(neg2(x), y, f2(1.0f));
-  float2 r = fma2(y, e, y);
-  if (__any_sync(0xffffffffu, !(rcp_in(x.x) && rcp_in(x.y)) || exact)) r = rcp2(x);
-  return r;
-}
-// canon (a == 0 ? +0 : a) as one paired add of +0: x + 0 is x for every x except -0, which
-// rounds to +0; a NaN stays a NaN (its payload may differ, which no result depends on).
-ITR_DEV float2 canon2(float2 a) { return add2(a, f2(0.0f)); }
+ITR_DEV float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+ITR_DEV float2 sel2(B2 c, float2 a, float2 b) { return make_float2(c.x ? a.x : b.x, c.y ? a.y : b.y); }
+ITR_DEV float2 max2(float2 a, float2 b) { return make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y)); }
+ITR_DEV float2 min2(float2 a, float2 b) { return make_float2(fminf(a.x, b.x), fminf(a.y, b.y)); }
 // max(a, 0) with the reference's NaN rule (a > 0 ? a : 0): the hardware maximum with +0 gives
-// the same bits for all 2^32 inputs of each component (checked exhaustively on the B200,
-// NaN and -0 included), in one instruction per component instead of a compare and a select.
+// the same bits for all 2^32 inputs of each component.
 ITR_DEV float2 max2z(float2 a) { return make_float2(fmaxf(a.x, 0.0f), fmaxf(a.y, 0.0f)); }
-ITR_DEV float2 abs2(float2 a) { return make_float2(rabs(a.x), rabs(a.y)); }
+ITR_DEV B2 gt2(float2 a, float b) { return B2{a.x > b, a.y > b}; }
+
+// 1/x for |x| in [2^-125, 2^126): one Newton step from the hardware estimate (textbook FMA
+// refinement: P. Markstein, IBM J. Res. Dev. 34(1), 1990; J.-M. Muller et al., Handbook of
+// Floating-Point Arithmetic, 2nd ed., 2018, ch. 4): y = est(1/x); e = fma(-x, y, 1); y + y e.
+// Equal to CUDA's IEEE reciprocal on every 32-bit input of that range (checked on the B200).
+ITR_DEV float rcp_est(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+ITR_DEV float2 rcp2(float2 x) {
+  const float2 y = make_float2(rcp_est(x.x), rcp_est(x.y));
+  return fma2(y, fma2(neg2(x), y, f2(1.0f)), y);
+}
+// sqrt(x) for x = +0 or x in [2^-149, 2^80): one Newton step from the hardware estimate of
+// 1/sqrt (same sources: s = x y, d = fma(-s, s, x), s + d (y / 2)), on x 2^48 so that the
+// residual d is exact for the smallest subnormals too (wetting fronts have depths down to them).
+// The 2^-126 added for the estimate alone keeps it finite at 0 and vanishes in rounding
+// elsewhere. Equal to CUDA's IEEE square root on every 32-bit input of that range (checked on the
+// B200); about half its time, and without the branch that would end the basic block.
+ITR_DEV float rsqrt_est(float x) { float r; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+ITR_DEV float2 sqrt2(float2 x) {
+  const float2 xs = mulp2(x, f2(0x1p48f));
+  const float2 xt = add2(xs, f2(0x1p-126f));
+  const float2 y = make_float2(rsqrt_est(xt.x), rsqrt_est(xt.y));
+  const float2 s = mulp2(xs, y), h = mulp2(y, f2(0x1p-25f));
+  return fma2(fma2(neg2(s), s, xs), h, mulp2(s, f2(0x1p-24f)));
+}
 
 ITR_DEV float2 rcbrt2(float2 x, float nz) {
   float2 r = make_float2(__uint_as_float(0x54A23280u - __float_as_uint(x.x) / 3u),
                          __uint_as_float(0x54A23280u - __float_as_uint(x.y) / 3u));
-  const float2 x3 = mul2(x, f2((float)(1.0 / 3.0)), nz);
+  const float2 x3 = mulp2(x, f2((float)(1.0 / 3.0)));
   const float2 c43 = f2((float)(4.0 * (1.0 / 3.0)));
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const float2 r2 = mul2(r, r, nz);
-    r = sub2(mul2(r, c43, nz), mul2(x3, mul2(r2, r2, nz), nz));
+    const float2 r2 = mulp2(r, r);
+    r = sub2(mul2(r, c43, nz), mul2(x3, mulp2(r2, r2), nz));
   }
   return r;
 }
 
-// hll (numerics.rs:56-93) on two faces.
-ITR_DEV Face2 hll2(float2 hl, float2 ul, float2 tl, float2 cl, float2 hr, float2 ur, float2 tr, float2 cr, float g_half, float nz,
-                   unsigned exact) {
+// hll (numerics.rs:56-93) on two faces with finite, bounded states. Three places differ from the
+// scalar text and give the same bits: 0.5 a + b and 2 a + b as one fma (the product is exact
+// unless |a| < 2^-125, where it vanishes beside b: a wet side's celerity is above 2^-73); min and
+// max as instructions (the sign of a zero wave speed is not read); and no test for two dry
+// sides: their celerities are 0, so the wave speeds are equal and one of the upwind fluxes, a
+// zero, is taken (its sign is lost in the cell update, whose states are never -0).
+ITR_DEV Face2 hll2(float2 hl, float2 ul, float2 tl, float2 cl, float2 hr, float2 ur, float2 tr, float2 cr, float g_half, float nz) {
   const float NZ = nz;
-  const B2 dry_l = not2(gt2(hl, 0.0f));
-  const B2 dry_r = not2(gt2(hr, 0.0f));
-  const float2 ustar = sub2(add2(mul2(f2(0.5f), add2(ul, ur), NZ), cl), cr);
-  const float2 cstar = add2(mul2(f2(0.5f), add2(cl, cr), NZ), mul2(f2(0.25f), sub2(ul, ur), NZ));
+  const B2 wet_l = gt2(hl, 0.0f), wet_r = gt2(hr, 0.0f);
+  const float2 ustar = sub2(fma2(f2(0.5f), add2(ul, ur), cl), cr);
+  const float2 cstar = fma2(f2(0.25f), sub2(ul, ur), mulp2(f2(0.5f), add2(cl, cr)));
   const float2 ul_cl = sub2(ul, cl);
   const float2 ur_cr = add2(ur, cr);
   const float2 slw = min2(ul_cl, sub2(ustar, cstar));
   const float2 srw = max2(ur_cr, add2(ustar, cstar));
-  const float2 sl = sel2(dry_l, sub2(ur, mul2(f2(2.0f), cr, NZ)), sel2(dry_r, ul_cl, slw));
-  const float2 sr = sel2(dry_l, ur_cr, sel2(dry_r, add2(ul, mul2(f2(2.0f), cl, NZ)), srw));
+  const float2 sl = sel2(wet_l, sel2(wet_r, slw, ul_cl), fma2(f2(-2.0f), cr, ur));
+  const float2 sr = sel2(wet_l, sel2(wet_r, srw, fma2(f2(2.0f), cl, ul)), ur_cr);
   const float2 ml = mul2(hl, ul, NZ);
   const float2 mr = mul2(hr, ur, NZ);
   const float2 gh = f2(g_half);
-  const float2 pl_ = mul2(mul2(gh, hl, NZ), hl, NZ);
-  const float2 pr_ = mul2(mul2(gh, hr, NZ), hr, NZ);
+  const float2 pl_ = mul2(mulp2(gh, hl), hl, NZ);
+  const float2 pr_ = mul2(mulp2(gh, hr), hr, NZ);
   const float2 pl = add2(mul2(ml, ul, NZ), pl_);
   const float2 pr = add2(mul2(mr, ur, NZ), pr_);
-  const B2 both_dry = and2(dry_l, dry_r);
-  const B2 use_l = ge2(sl, 0.0f);
-  const B2 use_r = le2(sr, 0.0f);
-  const B2 trivial = or2(or2(both_dry, use_l), use_r);
-  const float2 den = sel2(trivial, f2(1.0f), sub2(sr, sl));
-  const float2 inv = rcp2f(den, exact);
-  const float2 slsr = mul2(sl, sr, NZ);
+  const B2 use_l = B2{sl.x >= 0.0f, sl.y >= 0.0f}, use_r = B2{sr.x <= 0.0f, sr.y <= 0.0f};
+  const B2 trivial = B2{use_l.x || use_r.x, use_l.y || use_r.y};
+  const float2 inv = rcp2(sel2(trivial, f2(1.0f), sub2(sr, sl)));
+  const float2 slsr = mulp2(sl, sr);
   const float2 fm_star = mul2(add2(sub2(mul2(sr, ml, NZ), mul2(sl, mr, NZ)), mul2(slsr, sub2(hr, hl), NZ)), inv, NZ);
   const float2 fn_star = mul2(add2(sub2(mul2(sr, pl, NZ), mul2(sl, pr, NZ)), mul2(slsr, sub2(mr, ml), NZ)), inv, NZ);
-  const float2 fm = sel2(both_dry, f2(0.0f), sel2(use_l, ml, sel2(use_r, mr, fm_star)));
-  const float2 fn = sel2(both_dry, f2(0.0f), sel2(use_l, pl, sel2(use_r, pr, fn_star)));
+  const float2 fm = sel2(use_l, ml, sel2(use_r, mr, fm_star));
+  const float2 fn = sel2(use_l, pl, sel2(use_r, pr, fn_star));
   Face2 f;
   f.m = fm;
   f.nl = sub2(fn, pl_);
@@ -687,49 +696,91 @@ ITR_DEV Face2 face2(float2 hl, float2 ul, float2 vl, float2 cl, float2 hr, float
     csl = sel2(pl, sl, cl);
     csr = sel2(pr, sr, cr);
   }
-  if (NORMAL_X) return hll2(hsl, ul, vl, csl, hsr, ur, vr, csr, k.g_half, NZ, k.exact);
-  return hll2(hsl, vl, ul, csl, hsr, vr, ur, csr, k.g_half, NZ, k.exact);
+  if (NORMAL_X) return hll2(hsl, ul, vl, csl, hsr, ur, vr, csr, k.g_half, NZ);
+  return hll2(hsl, vl, ul, csl, hsr, vr, ur, csr, k.g_half, NZ);
 }
 
+// low: the depth before the positivity fix; a cell is unhealthy when low < -h_dry.
 struct CellNew2 {
-  float2 h, qx, qy, s, infil, fix, c;
-  B2 bad;
+  float2 h, qx, qy, s, infil, fix, c, low;
 };
 
-// flux_update then sources (numerics.rs:144-195) on two cells.
+// flux_update then sources (numerics.rs:144-195) on two cells with finite, bounded states.
+// Momentum: the reference multiplies by keep = 0 where the new depth is below h_dry and then
+// flushes |q| < q_min to 0; both are one select here (a dry cell's q is 0 either way).
 ITR_DEV CellNew2 update_cell2(float2 h, float2 qx, float2 qy, const Face2& w, const Face2& e, const Face2& n,
                               const Face2& s, float2 wet, float2 gn2, const StepK& k) {
   const float NZ = k.nz;
   const float2 dtdx = f2(k.dtdx), dtdy = f2(k.dtdy);
-  float2 h1 = sub2(sub2(h, mul2(dtdx, sub2(e.m, w.m), NZ)), mul2(dtdy, sub2(s.m, n.m), NZ));
+  CellNew2 o;
+  const float2 h1 = sub2(sub2(h, mul2(dtdx, sub2(e.m, w.m), NZ)), mul2(dtdy, sub2(s.m, n.m), NZ));
   const float2 qx1 = sub2(sub2(qx, mul2(dtdx, sub2(e.nl, w.nr), NZ)), mul2(dtdy, sub2(s.t, n.t), NZ));
   const float2 qy1 = sub2(sub2(qy, mul2(dtdx, sub2(e.t, w.t), NZ)), mul2(dtdy, sub2(s.nl, n.nr), NZ));
-  CellNew2 o;
-  B2 bad = not2(B2{h1.x >= -k.h_dry, h1.y >= -k.h_dry});
-  const B2 neg = lt2(h1, 0.0f);
-  o.fix = max2z(neg2(h1));   // h1 < 0 ? -h1 : 0, the same bits for every h1
-  h1 = sel2(neg, f2(0.0f), h1);
-  const float2 h2 = add2(h1, mul2(f2(k.rain), wet, NZ));
-  o.infil = min2(mul2(f2(k.cap), wet, NZ), h2);
+  o.low = h1;
+  const float2 hc = max2z(h1);
+  o.fix = sub2(hc, h1);
+  const float2 h2 = add2(hc, mul2(f2(k.rain), wet, NZ));
+  o.infil = min2(mulp2(f2(k.cap), wet), h2);
   const float2 h3 = sub2(h2, o.infil);
-  const B2 dry = lt2(h3, k.h_dry);
+  const B2 dry = B2{h3.x < k.h_dry, h3.y < k.h_dry};
   const float2 r = rcbrt2(sel2(dry, f2(1.0f), h3), NZ);
-  const float2 r3 = mul2(mul2(r, r, NZ), r, NZ);
-  const float2 r7 = mul2(mul2(r3, r3, NZ), r, NZ);
+  const float2 r3 = mulp2(mulp2(r, r), r);
+  const float2 r7 = mulp2(mulp2(r3, r3), r);
   const float2 qm = sqrt2(add2(mul2(qx1, qx1, NZ), mul2(qy1, qy1, NZ)));
-  const float2 inv = rcp2f(add2(f2(1.0f), mul2(mul2(mul2(f2(k.dt), gn2, NZ), qm, NZ), r7, NZ)), k.exact);
-  const float2 keep = sel2(dry, f2(0.0f), f2(1.0f));
-  float2 qx2 = mul2(mul2(qx1, inv, NZ), keep, NZ);
-  float2 qy2 = mul2(mul2(qy1, inv, NZ), keep, NZ);
-  qx2 = sel2(lt2(abs2(qx2), k.q_min), f2(0.0f), qx2);
-  qy2 = sel2(lt2(abs2(qy2), k.q_min), f2(0.0f), qy2);
+  const float2 inv = rcp2(add2(f2(1.0f), mul2(mulp2(mulp2(f2(k.dt), gn2), qm), r7, NZ)));
+  const float2 tx = mulp2(qx1, inv), ty = mulp2(qy1, inv);
+  o.qx = make_float2(fabsf(tx.x) >= k.q_min && !dry.x ? tx.x : 0.0f, fabsf(tx.y) >= k.q_min && !dry.y ? tx.y : 0.0f);
+  o.qy = make_float2(fabsf(ty.x) >= k.q_min && !dry.x ? ty.x : 0.0f, fabsf(ty.y) >= k.q_min && !dry.y ? ty.y : 0.0f);
   const float2 c = sqrt2(mul2(f2(k.g), h3, NZ));
-  o.s = add2(mul2(add2(mul2(abs2(qx2), r3, NZ), c), f2(k.inv_dx), NZ), mul2(add2(mul2(abs2(qy2), r3, NZ), c), f2(k.inv_dy), NZ));
-  o.bad = B2{bad.x || !(qm.x == qm.x), bad.y || !(qm.y == qm.y)};
-  o.h = canon2(h3);
-  o.qx = canon2(qx2);
-  o.qy = canon2(qy2);
+  const float2 ax = mul2(o.qx, r3, NZ), ay = mul2(o.qy, r3, NZ);   // |q| r3 = |q r3|
+  const float2 sx = make_float2(fabsf(ax.x) + c.x, fabsf(ax.y) + c.y), sy = make_float2(fabsf(ay.x) + c.x, fabsf(ay.y) + c.y);
+  o.s = add2(mul2(sx, f2(k.inv_dx), NZ), mul2(sy, f2(k.inv_dy), NZ));
+  o.h = add2(h3, f2(0.0f));   // canon: -0 becomes +0
   o.c = c;
+  return o;
+}
+
+// Paired desingularised velocity and celerity (cell_vel on two cells).
+ITR_DEV void vel2(float2 h, float2 qx, float2 qy, const StepK& k, float2& u, float2& v) {
+  const float2 h2 = mul2(h, h, k.nz);
+  const float2 t = mulp2(add2(h, h), rcp2(add2(h2, max2(h2, f2(k.heps2)))));
+  u = mul2(qx, t, k.nz);
+  v = mul2(qy, t, k.nz);
+}
+ITR_DEV float2 cel2(float2 h, const StepK& k) { return sqrt2(mul2(f2(k.g), h, k.nz)); }
+
+// The same through the scalar path, for steps with StepK::exact set (rare: not inlined).
+ITR_DEV Face2 face2_of(const FaceF& a, const FaceF& b) {
+  Face2 f;
+  f.m = make_float2(a.m, b.m); f.nl = make_float2(a.nl, b.nl); f.nr = make_float2(a.nr, b.nr); f.t = make_float2(a.t, b.t);
+  return f;
+}
+ITR_DEV FaceF fx_(const Face2& f) { FaceF r; r.m = f.m.x; r.nl = f.nl.x; r.nr = f.nr.x; r.t = f.t.x; return r; }
+ITR_DEV FaceF fy_(const Face2& f) { FaceF r; r.m = f.m.y; r.nl = f.nl.y; r.nr = f.nr.y; r.t = f.t.y; return r; }
+
+template <bool NORMAL_X, bool CREST>
+__device__ __noinline__ Face2 face2_exact(float2 hl, float2 ul, float2 vl, float2 cl, float2 hr, float2 ur, float2 vr, float2 cr,
+                                          float2 d0, float2 d1, StepK k) {
+  return face2_of(face<NORMAL_X, CREST>(hl.x, ul.x, vl.x, cl.x, hr.x, ur.x, vr.x, cr.x, d0.x, d1.x, k),
+                  face<NORMAL_X, CREST>(hl.y, ul.y, vl.y, cl.y, hr.y, ur.y, vr.y, cr.y, d0.y, d1.y, k));
+}
+// low: -infinity for an unhealthy cell (a NaN is not below -h_dry).
+static __device__ __noinline__ CellNew2 update_cell2_exact(float2 h, float2 qx, float2 qy, Face2 w, Face2 e, Face2 n, Face2 s,
+                                                           float2 wet, float2 gn2, StepK k) {
+  const CellNew a = update_cell(h.x, qx.x, qy.x, fx_(w), fx_(e), fx_(n), fx_(s), wet.x, gn2.x, k);
+  const CellNew b = update_cell(h.y, qx.y, qy.y, fy_(w), fy_(e), fy_(n), fy_(s), wet.y, gn2.y, k);
+  CellNew2 o;
+  o.h = make_float2(a.h, b.h); o.qx = make_float2(a.qx, b.qx); o.qy = make_float2(a.qy, b.qy); o.s = make_float2(a.s, b.s);
+  o.infil = make_float2(a.infil, b.infil); o.fix = make_float2(a.fix, b.fix); o.c = make_float2(a.c, b.c);
+  const float inf = __int_as_float(0x7f800000);
+  o.low = make_float2(a.bad ? -inf : 0.0f, b.bad ? -inf : 0.0f);
+  return o;
+}
+struct Vel2 { float2 u, v, c; };
+static __device__ __noinline__ Vel2 vel2_exact(float2 h, float2 qx, float2 qy, float g, float heps2) {
+  Vel2 o;
+  cell_vel(h.x, qx.x, qy.x, g, heps2, o.u.x, o.v.x, o.c.x);
+  cell_vel(h.y, qx.y, qy.y, g, heps2, o.u.y, o.v.y, o.c.y);
   return o;
 }
 

@@ -28,6 +28,8 @@ static_assert(kTileThreads >= 17 * 16, "one x-face and one y-face per thread");
 // mass fluxes (signed: the reference nets a y-edge over its whole row before splitting it
 // into inflow and outflow, kernel.rs:452-472).
 constexpr int kPart = 7;
+// A step's record for the adjoint: dt, rain, start time, StepK::exact.
+constexpr int kLog = 4;
 // The update kernels ask for 6 resident blocks per SM (32 registers a thread): with the
 // 18x18 halo loads waiting on HBM, more resident warps beat fewer registers (measured +10%).
 
@@ -53,6 +55,7 @@ struct PlainCtl {
   int locked_live;
   int copy_req;
   unsigned long long rows_skipped;   // dry rows skipped so far (kernel.rs:605-612)
+  unsigned unsafe;   // bit 0: the state is not known to be bounded, bit 1: never will be (StepK::exact)
 };
 
 struct PlainArgs {
@@ -84,7 +87,7 @@ struct PlainArgs {
   int max_rows;
   unsigned long long max_steps;
   unsigned* tpk;      // optional, per design nx*ny: index of the state that last raised PK
-  double* dt_log;     // optional, per design a ring of max_log (dt, rain, t): slot step % max_log
+  double* dt_log;     // optional, per design a ring of max_log records [kLog]: slot step % max_log
   int max_log;
   const WarmStart* warm;   // optional, per design (state NULL: cold)
   // Baseline-locked dt (SolverParams::locked_dt / cfl_hard, solver.rs:42-46); read only by
@@ -150,7 +153,7 @@ ITR_DEV PlainDesign plain_design(const PlainArgs& A, int d, int n_tiles) {
   v.ctl = A.ctl + d;
   v.ledger = A.ledger ? A.ledger + (size_t)d * A.max_rows * 8 : nullptr;
   v.tpk = A.tpk ? A.tpk + d * N : nullptr;
-  v.dt_log = A.dt_log ? A.dt_log + (size_t)d * A.max_log * 3 : nullptr;
+  v.dt_log = A.dt_log ? A.dt_log + (size_t)d * A.max_log * kLog : nullptr;
   v.cut = A.cut_d ? A.cut_d[d] : A.cut;
   v.fill = A.fill_d ? A.fill_d[d] : A.fill;
   const size_t R = (size_t)A.ny + 2;
@@ -237,7 +240,7 @@ __global__ void __launch_bounds__(kTileThreads, 6) k_plain_update(const PlainArg
   }
   __syncthreads();
   float smax = 0.0f;
-  bool bad = false;
+  bool bad = false, uns = false;
   double acc[5] = {0, 0, 0, 0, 0};
   if (cv) {
     const FaceF w = fx[ly * 17 + lx], e = fx[ly * 17 + lx + 1];
@@ -252,6 +255,7 @@ __global__ void __launch_bounds__(kTileThreads, 6) k_plain_update(const PlainArg
     }
     smax = o.s;
     bad = o.bad;
+    uns = !state_safe(A.P, o.s);
     acc[0] = (double)o.infil; acc[1] = (double)o.fix;
     if (hits) acc[4] = (double)o.h;
     // boundary faces: x-edges split per face (kernel.rs:435-450), y-edges summed first
@@ -263,7 +267,7 @@ __global__ void __launch_bounds__(kTileThreads, 6) k_plain_update(const PlainArg
   // block reductions, fixed order
   float m = smax;
   for (int o = 16; o > 0; o >>= 1) m = rmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  unsigned b = __any_sync(0xffffffffu, bad) ? 1u : 0u;
+  unsigned b = (__any_sync(0xffffffffu, bad) ? 1u : 0u) | (__any_sync(0xffffffffu, uns) ? 2u : 0u);
   for (int j = 0; j < 5; ++j)
     for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
   const int wid = li >> 5;
@@ -282,7 +286,7 @@ __global__ void __launch_bounds__(kTileThreads, 6) k_plain_update(const PlainArg
     float mm = 0.0f; unsigned bb = 0u; double ss[5] = {0, 0, 0, 0, 0};
     for (int w = 0; w < kTileThreads / 32; ++w) { mm = rmax(mm, wmax[w]); bb |= wbad[w]; for (int j = 0; j < 5; ++j) ss[j] += wsum[w][j]; }
     if (mm > 0.0f) atomicMax(&D.ctl->smax_bits, __float_as_uint(mm));
-    if (bb) atomicOr(&D.ctl->bad, 1u);
+    if (bb) atomicOr(&D.ctl->bad, bb);
     double* p = D.part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kPart;
     for (int j = 0; j < 5; ++j) p[j] = ss[j];
     p[5] = yt; p[6] = yb;
@@ -358,13 +362,15 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int n_blocks, int first) {
     if (lane == 0) {
       c.tot_infil += tot[0]; c.tot_fix += tot[1]; c.tot_in += tot[2]; c.tot_out += tot[3];
       c.smax_bits = 0u;
+      c.bad = 0u;
+      c.unsafe = (c.unsafe & 2u) | (!state_safe(P, (float)smax) || (badv & 2u) ? 1u : 0u);
       c.step += 1;
       c.t = c.pl.t_new;
       c.acc_rain += c.pl.rain * P.area * P.wet_count;
       c.par ^= 1;
     }
     __syncwarp();
-    if (badv) { if (lane == 0) { c.status = 3; c.done = 1; } return; }
+    if (badv & 1u) { if (lane == 0) { c.status = 3; c.done = 1; } return; }
     if (lane == 0) c.dt_cfl = smax > 0.0 ? P.cfl / smax : P.dt_max;
     if constexpr (LOCKED) { if (lane == 0) c.s_cur = smax; }
     __syncwarp();
@@ -451,6 +457,7 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int n_blocks, int first) {
       const double dt = c.locked_live ? A.locked_dt[c.step] : dmin_num(c.dt_cfl, P.dt_max);
       c.pl = plan_step_dt(P, c.t, c.sync_index, dt);
       c.k = step_consts(P, c.pl.dt, c.pl.rain);
+      c.k.exact = c.unsafe ? 1u : 0u;
     }
     return;
   }
@@ -463,11 +470,12 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int n_blocks, int first) {
     if (!(c.t < P.duration && c.sync_index < P.n_sync)) { c.done = 1; return; }
     if (c.step >= A.max_steps) { c.status = 4; c.done = 1; return; }
     c.pl = plan_step(P, c.t, c.sync_index, c.dt_cfl);
-    if (D.dt_log) {   // ring of max_log entries, slot step mod max_log
-      const size_t slot = (size_t)(c.step % (unsigned long long)A.max_log);
-      D.dt_log[3 * slot] = c.pl.dt; D.dt_log[3 * slot + 1] = c.pl.rain; D.dt_log[3 * slot + 2] = c.t;
-    }
     c.k = step_consts(P, c.pl.dt, c.pl.rain);
+    c.k.exact = c.unsafe ? 1u : 0u;
+    if (D.dt_log) {   // ring of max_log entries, slot step mod max_log
+      double* q = D.dt_log + (size_t)(c.step % (unsigned long long)A.max_log) * kLog;
+      q[0] = c.pl.dt; q[1] = c.pl.rain; q[2] = c.t; q[3] = (double)c.k.exact;
+    }
   }
 }
 
@@ -518,6 +526,15 @@ __global__ void k_plain_init(const PlainArgs A) {
     for (int j = threadIdx.x; j < 2 * (ny + 2); j += blockDim.x) D.rowwet[j] = 0u;
     __syncthreads();
   }
+  // a crest jump or stage depth out of the branch-free step's bounds keeps the run on the scalar path
+  bool neg = false;
+  if (A.mode == 1) {
+    for (size_t i = threadIdx.x; i < (size_t)ny * (nx + 1); i += blockDim.x) neg = neg || !jump_safe(D.dzx[i]) || !jump_safe(D.dzx2[i]);
+    for (size_t i = threadIdx.x; i < (size_t)(ny + 1) * nx; i += blockDim.x) neg = neg || !jump_safe(D.dzy[i]) || !jump_safe(D.dzy2[i]);
+  }
+  if (D.bh)
+    for (int i = threadIdx.x; i < 2 * (nx + ny); i += blockDim.x) neg = neg || !stage_safe(A.bc[i], D.bh[i]);
+  const unsigned never = __syncthreads_or(neg ? 1 : 0) ? 2u : 0u;
   if (W) {
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
       D.H[i] = W->state[i]; D.QX[i] = W->state[n + i]; D.QY[i] = W->state[2 * n + i]; D.PK[i] = W->state[3 * n + i];
@@ -530,17 +547,20 @@ __global__ void k_plain_init(const PlainArgs A) {
       c.t = W->t; c.dt_cfl = W->dt_cfl; c.acc_rain = W->acc_rain; c.v0 = W->v0; c.volume = W->volume; c.rel_res = W->rel_res;
       c.tot_infil = W->tot_infil; c.tot_fix = W->tot_fix; c.tot_in = W->tot_in; c.tot_out = W->tot_out;
       c.step = W->step; c.sync_index = W->sync_index; c.n_rows = W->n_rows;
+      c.unsafe = never | (P.cfl <= 0.99 * (double)P.s_safe * W->dt_cfl ? 0u : 1u);   // dt_cfl = cfl / largest wave rate
       *D.ctl = c;
     }
     return;
   }
   __shared__ double ss[32], sv[32];
   double s0 = 0.0, v0 = 0.0;
+  bool uns = false;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     float h = D.h0[i];
     D.H[i] = h; D.QX[i] = 0.0f; D.QY[i] = 0.0f; D.PK[i] = 0.0f;
     if (D.tpk) D.tpk[i] = 0u;
     if (D.rowwet && h != 0.0f) D.rowwet[1 + i / nx] = 1u;
+    uns = uns || !depth_safe(P, h);
     double hd = (double)h;
     v0 += hd;
     if (hd > P.h_dry) {
@@ -554,7 +574,7 @@ __global__ void k_plain_init(const PlainArgs A) {
     v0 += __shfl_xor_sync(0xffffffffu, v0, o);
   }
   if ((threadIdx.x & 31) == 0) { ss[threadIdx.x >> 5] = s0; sv[threadIdx.x >> 5] = v0; }
-  __syncthreads();
+  const unsigned unsafe = never | (__syncthreads_or(uns ? 1 : 0) ? 1u : 0u);
   if (threadIdx.x == 0) {
     double s = 0.0, v = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { s = s > ss[w] ? s : ss[w]; v += sv[w]; }
@@ -563,6 +583,7 @@ __global__ void k_plain_init(const PlainArgs A) {
     c.v0 = v * P.area; c.volume = c.v0;
     c.dt_cfl = s > 0.0 ? dmin_num(P.cfl / s, P.dt_max) : P.dt_max;
     c.s_cur = s;
+    c.unsafe = unsafe;
     *D.ctl = c;
   }
 }
