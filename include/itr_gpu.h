@@ -197,8 +197,8 @@ int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_grid* g, int3
  *              take the tiled path), 1 = plain one-design-per-launch kernel, 2 = tiled
  *              batched path: all designs per launch, state in HBM, a CUDA graph per
  *              steps_per_submit steps
- *   "threads"  threads per CTA of the batched kernel (0 = autotune)
- *   "cluster"  CTAs per design of the batched kernel (0 = autotune)
+ *   "threads"  threads per CTA of the batched kernel, at most 512 used (0 = by the grid and population)
+ *   "cluster"  CTAs per design of the batched kernel (0 = by the grid and population, 1 .. 8)
  *   "graph"    tiled path: 1 = replay each block of steps as one CUDA graph (default 1)
  *   "steps_per_submit"  plain and tiled paths: steps between host polls (default 64)
  *   "warm_start"  1 = start each design from the baseline record (itr_gpu_record_baseline) where
@@ -254,7 +254,7 @@ int itr_gpu_rerun_resident(itr_ctx* ctx);
  * evaluator.rs:218-266 runs one batch per level). Each group is one grid with its designs,
  * monitors and objective, exactly the arguments of itr_gpu_run_batch; every group's
  * persistent cluster kernel runs as one branch of a single CUDA graph launch, each with
- * the launch shape autotuned for its grid, per-design adaptive dt and per-design aborts.
+ * its launch shape chosen for its grid, per-design adaptive dt and per-design aborts.
  * results holds sum(n_designs) entries in group order. */
 typedef struct itr_group {
   const itr_grid* grid;

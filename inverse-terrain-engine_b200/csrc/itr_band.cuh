@@ -234,6 +234,8 @@ ITR_DEV void band_sweep(const PlainArgs& A, const PlainDesign& D, const PlainCtl
   __syncwarp();
 
   // ---- row sweep ----
+  UpdK uk;
+  uk.dtdx = f2(k.dtdx); uk.dtdy = f2(k.dtdy); uk.inv_dx = f2(k.inv_dx); uk.inv_dy = f2(k.inv_dy);
   const float* dzx = D.dzx + c0;
   const float* dzy = D.dzy + c0;
   auto load_in = [&](int r) -> RowIn {   // inputs of row r (r < r1)
@@ -341,7 +343,7 @@ ITR_DEV void band_sweep(const PlainArgs& A, const PlainDesign& D, const PlainCtl
     }
     CellNew2 o;
     if constexpr (EX) o = update_cell2_exact(cur.h, cur.qx, cur.qy, fW, fE, fN, fS, q.wet, q.gn2, k);
-    else o = update_cell2(cur.h, cur.qx, cur.qy, fW, fE, fN, fS, q.wet, q.gn2, k);
+    else o = update_cell2(cur.h, cur.qx, cur.qy, fW, fE, fN, fS, q.wet, q.gn2, k, uk);
     const size_t ci = (size_t)r * nx + c0;
     if (vec) {
       *reinterpret_cast<float2*>(D.H + pout + ci) = o.h;

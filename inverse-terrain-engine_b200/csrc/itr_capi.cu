@@ -22,6 +22,7 @@
 #include "itr_device.cuh"
 #include "itr_batched.cuh"
 #include "itr_batched_table.cuh"
+#include "itr_pack.cuh"
 #include "itr_plain.cuh"
 #include "itr_band.cuh"
 #include "itr_adjoint.cuh"
@@ -70,9 +71,9 @@ struct LaunchCfg {
   int C = 1, T = 512, W = 1, S = 1;
   size_t smem = 0;
   bool ok = false;
-  bool tiled = false;   // the measured choice was the tiled HBM path
-  int band = 1;         // ... with the row-band kernel (1) or the 16x16 tiles (0)
+  bool tiled = false;   // the tiled HBM path instead
   bool bnd = false;     // the grid has stage or inflow cells (k_batched<..., BND>)
+  double us = 0.0;      // predicted time of a step
 };
 
 }  // namespace
@@ -125,7 +126,6 @@ struct itr_ctx {
   std::string err;
   // options
   int impl = 0, threads = 0, cluster = 0, graph = 1, steps_per_submit = 64;
-  int autotune = 1, autotune_top = 6, probe_steps = 200;
   int exact_special = 0;
   int band = 1;           // tiled path update kernel: 1 = row-band sweep (k_band), 0 = 16x16 tiles
   int adj_band = -1;      // adjoint kernels on row bands: bit 0 the replay, bit 1 the backward step (else 16x16 tiles);
@@ -133,13 +133,13 @@ struct itr_ctx {
   int adj_trim = 1;       // adjoint: skip the steps after a design's latest asset maximum (zero adjoint there)
   unsigned wait_limit = 1u << 22;   // bounded barrier wait of single-CTA designs (try_wait rounds)
   int stall_wait_test = 0;          // test of the timeout path: that wait never completes
-  float tune_ms = 0.0f;
   // baseline-locked dt (itr_gpu_set_locked_dt): the schedule, its limit, the snapshot buffers
   // and, per design of the last batch, the fallback time (-1: none)
   std::vector<double> locked_dt;
   double cfl_hard = 0.5;
   bool locked_run = false;
-  DevBuf lDt, lS4, lS2, lSk, lSs, lFb;
+  DevBuf lDt, lS4, lSs, lFb;
+  DevBuf bG, bJ, bJ2, bNever;   // cluster kernel: packed inputs (k_pack_inputs)
   std::vector<double> fallback;
   // device buffers (batched path)
   DevBuf wet, gn2, bc, dzx, dzy, dzx2, dzy2, h0, cut, fill, mon, obj_i, obj_d, peak, depth, ledger, out, mmax;
@@ -188,7 +188,7 @@ struct itr_ctx {
   PlainArgs last_tiled;
   dim3 last_tgrid;
   int last_band = 1;   // the tiled update kernel of the last tiled batch (option band)
-  // autotune cache: (nx, ny, n_designs, mode) -> cfg
+  // launch shapes by (nx, ny, n_designs, mode)
   std::map<std::tuple<int, int, int, int>, LaunchCfg> tuned;
   cudaGraphExec_t gexec = nullptr;
 };
@@ -228,24 +228,23 @@ static BatchedFn batched_fn(bool crest, bool clustered, int maxt, bool bnd, bool
   return bnd ? batched_fn_01(clustered, maxt, locked, skip) : batched_fn_00(clustered, maxt, locked, skip);
 }
 
-static int maxt_bucket(int T) { return T <= 256 ? 256 : T <= 512 ? 512 : T <= 768 ? 768 : 1024; }
+static int maxt_bucket(int T) { return T <= 256 ? 256 : T <= 384 ? 384 : 512; }
 
 // Geometry of the batched kernel for (nx, ny) with C CTAs per design and about T threads.
-static LaunchCfg make_cfg(const itr_ctx* ctx, int nx, int ny, int C, int T_target, bool crest, bool bnd) {
+static LaunchCfg make_cfg(const itr_ctx* ctx, int nx, int ny, int C, int T_target, bool bnd) {
   LaunchCfg c;
   c.C = C;
   c.bnd = bnd;
-  c.W = (nx + 1 + 63) / 64;   // warps per strip row; each lane holds two columns
-  if (C < 1 || ny < C) return c;
+  c.W = windows(nx);   // warps per strip row
+  if (C < 1 || ny < C || nx < 2) return c;   // (one column: its west and east faces share a lane; the tiled path takes it)
   const int nr_min = ny / C, nr_max = (ny + C - 1) / C;
-  int S = T_target / (32 * c.W);
-  if (c.W > 1 && S > 15) S = 15;   // one named barrier per strip (ids 1..15)
+  int S = std::min(T_target, 512) / (32 * c.W);   // (more threads leave too few registers each: below)
   if (S > nr_min) S = nr_min;
   if (S < 1) return c;
   c.S = S;
   c.T = S * 32 * c.W;
-  if (c.T > 1024) return c;
-  c.smem = batched_smem_bytes(nr_max, nx, S, c.W, c.T / 32, crest ? 1 : 0, bnd ? 1 : 0, ny);
+  if (c.T > 512) return c;
+  c.smem = smem_plan(nr_max, nx, S, c.W, c.T / 32, bnd ? 1 : 0, ny).total;
   c.ok = c.smem <= ctx->smem_optin;
   return c;
 }
@@ -291,59 +290,38 @@ static int max_active_clusters(itr_ctx* ctx, const LaunchCfg& cfg, bool crest) {
   return n;
 }
 
-// Candidate configurations, best-first by a simple model: time ~ waves * work per CTA.
-static std::vector<LaunchCfg> candidates(itr_ctx* ctx, int nx, int ny, int n_designs, bool crest, bool bnd) {
-  std::vector<std::pair<double, LaunchCfg>> v;
-  for (int C : {1, 2, 4, 8}) {
-    for (int T : {256, 384, 512, 640, 768, 896, 1024}) {
-      LaunchCfg c = make_cfg(ctx, nx, ny, C, T, crest, bnd);
-      if (!c.ok) continue;
-      bool dup = false;
-      for (auto& e : v) if (e.second.C == c.C && e.second.T == c.T) dup = true;
-      if (dup) continue;
-      int act = max_active_clusters(ctx, c, crest);
+// The launch shape of the cluster kernel for n designs of an nx x ny grid: the least predicted time per
+// step over all cluster sizes and block sizes. A rule on sizes alone, so that the same batch always
+// runs in the same shape (its ledger sums to the same bits); it replaces timing a few candidates on
+// the first call, which cost up to 13 probe launches and, between near shapes, did not always end alike.
+//   step = waves (F + (L + 1/2) r): F the barrier, the CFL reduction and the integrator, L the rows of a
+//   strip, r a row's time with w warps on each of an SM's four schedulers.
+// The constants are a fit to 31 populations (24x20 .. 700x20, 1 .. 500 designs) x all shapes, 200 steps
+// each: the shape chosen is the fastest or within 6 % of it on all but one (45x35 x64: 12 %), 0.8 %
+// on average. Blocks above 256 threads hold 168 registers a thread, too few for the sweep that runs the
+// faces a row ahead (x 1.15 per row), but three windows divide 12 warps and not 8; above 384 (128
+// registers) only for grids that need more windows than 12.
+static LaunchCfg batched_shape(itr_ctx* ctx, int nx, int ny, int n, bool crest, bool bnd) {
+  LaunchCfg best;
+  double best_us = 1e300;
+  for (int C = 1; C <= 8; ++C) {
+    int last_S = 0;
+    for (int T = 32; T <= 512; T += 32) {
+      if (T > 384 && 32 * windows(nx) <= 384) break;
+      const LaunchCfg c = make_cfg(ctx, nx, ny, C, T, bnd);
+      if (!c.ok || c.S == last_S) continue;
+      last_S = c.S;
+      const int act = max_active_clusters(ctx, c, crest);
       if (act <= 0) continue;
-      double waves = std::ceil((double)n_designs / act);
-      double rows = std::ceil((double)ny / C);
-      // per-CTA cost ~ cells per thread; small penalty per cluster barrier
-      double per_step = rows * nx / (double)c.T * (1.0 + 0.02 * (C - 1)) + 0.5;
-      double cost = waves * per_step;
-      v.push_back({cost, c});
+      const double waves = std::ceil((double)n / act);
+      const int ctas = std::min(n, act) * C, per_sm = (ctas + ctx->sm_count - 1) / ctx->sm_count;
+      const double w = std::max(1.0, per_sm * c.T / 128.0), rows = std::ceil(std::ceil((double)ny / C) / c.S);
+      const double r = c.T <= 256 ? 0.75 * (1.0 + 0.25 * (w - 1.0)) : 0.8625 * (1.0 + 0.3 * (w - 1.0));
+      const double us = waves * ((C > 1 ? 1.5 : 0.9) + (rows + 0.5) * r);
+      if (us < best_us) { best_us = us; best = c; best.us = us; }
     }
   }
-  std::sort(v.begin(), v.end(), [](const std::pair<double, LaunchCfg>& a, const std::pair<double, LaunchCfg>& b) { return a.first < b.first; });
-  std::vector<LaunchCfg> out;
-  for (auto& p : v) out.push_back(p.second);
-  return out;
-}
-
-// Time `probe_steps` steps of the batch under each candidate shape (CUDA events on the
-// context stream) and return the fastest. The probe runs write only scratch outputs.
-static int autotune(itr_ctx* ctx, const BatchArgs& A0, const std::vector<LaunchCfg>& cands, int n, LaunchCfg* best) {
-  BatchArgs A = A0;
-  A.max_steps = (unsigned long long)ctx->probe_steps;
-  A.warm = nullptr;   // probe the cold start: the shapes compare the same
-  A.ledger_out = nullptr;
-  A.max_rows = 0;
-  A.obj.enabled = 0;
-  float best_ms = 1e30f;
-  const size_t k = cands.size() < (size_t)ctx->autotune_top ? cands.size() : (size_t)ctx->autotune_top;
-  for (size_t i = 0; i < k; ++i) {
-    LaunchCfg c = cands[i];
-    A.C = c.C; A.W = c.W; A.S = c.S;
-    float ms = 0.0f;
-    for (int rep = 0; rep < 2; ++rep) {   // first launch warms the instruction cache
-      CU(cudaEventRecord(ctx->ev[1], ctx->stream));
-      int rc = launch_batched(ctx, A, c, n);
-      if (rc != ITR_OK) return rc;
-      CU(cudaEventRecord(ctx->ev[2], ctx->stream));
-      CU(cudaEventSynchronize(ctx->ev[2]));
-      CU(cudaEventElapsedTime(&ms, ctx->ev[1], ctx->ev[2]));
-    }
-    if (ms < best_ms) { best_ms = ms; *best = c; }
-  }
-  ctx->tune_ms = best_ms;
-  return ITR_OK;
+  return best;
 }
 
 // ------------------------------------------------------------------ input checks ------
@@ -440,13 +418,23 @@ static RunParams make_run_params(const itr_params* p, const itr_grid* g) {
   memset(&P, 0, sizeof(P));
   P.duration = p->duration_s; P.sync = p->sync_interval_s; P.cfl = p->cfl; P.dt_max = p->dt_max_s;
   P.h_dry = p->h_dry; P.h_eps = p->h_eps; P.infil = p->infil_capacity; P.initial_depth = p->initial_depth;
-  P.dx = g->dx; P.dy = g->dy; P.g = g->g; P.area = g->dx * g->dy; P.wet_count = (double)g->wet_count;
+  P.dx = g->dx; P.dy = g->dy; P.g = g->g; P.area = g->dx * g->dy; P.rdx = 1.0 / g->dx; P.rdy = 1.0 / g->dy; P.wet_count = (double)g->wet_count;
   P.n_sync = (uint32_t)std::ceil(p->duration_s / p->sync_interval_s);
   P.skip_dry = p->skip_dry;
   P.rain.n = p->n_rain;
   for (int i = 0; i < p->n_rain; ++i) { P.rain.t[i] = p->rain_t[i]; P.rain.r[i] = p->rain_rate[i]; }
   P.rain_sorted = 1;
   for (int i = 1; i < p->n_rain; ++i) if (!(p->rain_t[i] >= p->rain_t[i - 1])) P.rain_sorted = 0;
+  for (int i = 0; i <= p->n_rain; ++i) {   // the storm's linear pieces
+    RainSeg& s = P.rain.seg[i];
+    const bool first = i == 0, last = i == p->n_rain, any = p->n_rain > 0;
+    s.t0 = any ? p->rain_t[first ? 0 : i - 1] : 0.0;
+    s.r0 = any ? p->rain_rate[first ? 0 : i - 1] : 0.0;
+    s.dr = first || last ? 0.0 : p->rain_rate[i] - p->rain_rate[i - 1];
+    s.den = first || last ? 1.0 : p->rain_t[i] - p->rain_t[i - 1];
+    s.rden = 1.0 / s.den;
+    s.end = last ? HUGE_VAL : p->rain_t[i];
+  }
   // Dry-row skipping can act only on a step without rain: keep it on only when the storm has
   // a rain-free stretch inside the run (no skipping is possible otherwise, and the kernels
   // then leave out its bookkeeping; the results are the same either way).
@@ -609,7 +597,7 @@ void itr_gpu_destroy(itr_ctx* ctx) {
                     &ctx->tpart, &ctx->tctl, &ctx->tRow, &ctx->tGw, &ctx->tSnapRow, &ctx->aTpk, &ctx->aRing, &ctx->aTape, &ctx->aTape2, &ctx->aLA, &ctx->aLB, &ctx->aGx, &ctx->aGy, &ctx->aGx2, &ctx->aGy2,
                     &ctx->aSeg, &ctx->aNst, &ctx->aSeedC, &ctx->aSeedS, &ctx->aSeedW, &ctx->aSeedN, &ctx->aTmon,
                     &ctx->mDz, &ctx->mZe, &ctx->mAux, &ctx->mJp, &ctx->mJob, &ctx->mOut, &ctx->wsb, &ctx->rIn, &ctx->rOut,
-                    &ctx->lDt, &ctx->lS4, &ctx->lS2, &ctx->lSk, &ctx->lSs, &ctx->lFb})
+                    &ctx->lDt, &ctx->lS4, &ctx->lSs, &ctx->lFb, &ctx->bG, &ctx->bJ, &ctx->bJ2, &ctx->bNever})
     b->release();
   for (DevBuf& b : ctx->aCkpt) b.release();
   for (itr_ctx* c : ctx->children) itr_gpu_destroy(c);
@@ -658,7 +646,7 @@ int itr_gpu_set_option(itr_ctx* ctx, const char* key, int64_t value) {
   else if (k == "cluster") { if (!(value == 0 || value == 1 || value == 2 || value == 4 || value == 8)) return fail(ctx, ITR_INVALID_ARG, "cluster must be 0,1,2,4,8"); ctx->cluster = (int)value; }
   else if (k == "graph") ctx->graph = value != 0;
   else if (k == "steps_per_submit") { if (value < 1) return fail(ctx, ITR_INVALID_ARG, "steps_per_submit must be >= 1"); ctx->steps_per_submit = (int)value; }
-  else if (k == "autotune") { ctx->autotune = value != 0; ctx->tuned.clear(); }
+  else if (k == "autotune") {}   // (the launch shape follows from the sizes: batched_shape)
   else if (k == "exact_special") ctx->exact_special = value != 0;
   else if (k == "warm_start") ctx->warm_start = value != 0;
   else if (k == "band") ctx->band = value != 0;
@@ -666,7 +654,7 @@ int itr_gpu_set_option(itr_ctx* ctx, const char* key, int64_t value) {
   else if (k == "adj_band") { if (value < -1 || value > 3) return fail(ctx, ITR_INVALID_ARG, "adj_band is -1 .. 3"); ctx->adj_band = (int)value; }
   else if (k == "wait_limit") { if (value < 1 || value > 0x7fffffff) return fail(ctx, ITR_INVALID_ARG, "wait_limit out of range"); ctx->wait_limit = (unsigned)value; }
   else if (k == "stall_wait_test") ctx->stall_wait_test = value != 0;
-  else if (k == "probe_steps") { if (value < 1) return fail(ctx, ITR_INVALID_ARG, "probe_steps must be >= 1"); ctx->probe_steps = (int)value; }
+  else if (k == "probe_steps") { if (value < 1) return fail(ctx, ITR_INVALID_ARG, "probe_steps must be >= 1"); }
   else return fail(ctx, ITR_INVALID_ARG, "unknown option '%s'", key);
   if (k == "threads" || k == "cluster") ctx->tuned.clear();
   return ITR_OK;
@@ -1135,7 +1123,8 @@ static int collect_results(itr_ctx* ctx, const Collect& c) {
   }
 #endif
   float k_ms = 0, t_ms = 0;
-  cudaEventElapsedTime(&k_ms, ctx->ev[1], ctx->ev[2]);
+  // (a ladder group's kernel runs in the ladder's graph: its own events are not recorded)
+  if (cudaEventElapsedTime(&k_ms, ctx->ev[1], ctx->ev[2]) != cudaSuccess) { k_ms = 0; cudaGetLastError(); }
   cudaEventElapsedTime(&t_ms, ctx->ev[0], ctx->ev[3]);
   ctx->kernel_ms = k_ms; ctx->total_ms = t_ms; ctx->launches = launches;
   uint64_t cu = 0;
@@ -1445,7 +1434,6 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
   bool tiled = ctx->impl == 2 || ctx->vjp != nullptr;
   dim3 tgrid = tiled_grid(ctx, nx, ny, n);   // blocks per design of the tiled path's update
   int n_tiles = (int)(tgrid.x * tgrid.y);
-  const int band0 = ctx->band;
   const int max_tiles = std::max((nx + kTile - 1) / kTile * ((ny + kTile - 1) / kTile), n_tiles);
   const bool bnd_grid = has_stage || P.inflow.n > 0;   // stage or inflow ghosts
   auto tiled_args = [&](PlainArgs& A) -> cudaError_t {
@@ -1504,19 +1492,12 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
     }
     return e;
   };
-  int tiled_band = ctx->band;   // the tiled path's update kernel for this batch (the autotuner may pick)
   if (ctx->impl == 0 && !tiled) {
     BatchArgs A;
     memset(&A, 0, sizeof(A));
     A.P = P; A.nx = nx; A.ny = ny; A.mode = g->mode; A.n_designs = n;
-    A.wet = reinterpret_cast<const float*>(dv + o_wet);
-    A.gn2 = reinterpret_cast<const float*>(dv + o_gn2);
     A.bc = reinterpret_cast<const uint8_t*>(dv + o_bc);
     A.bh = has_stage ? reinterpret_cast<const float*>(dv + o_bh) : nullptr;
-    A.dzx = reinterpret_cast<const float*>(dv + o_dzx);
-    A.dzy = reinterpret_cast<const float*>(dv + o_dzy);
-    A.dzx2 = crest ? reinterpret_cast<const float*>(dv + o_dzx2) : nullptr;
-    A.dzy2 = crest ? reinterpret_cast<const float*>(dv + o_dzy2) : nullptr;
     A.h0 = reinterpret_cast<const float*>(dv + o_h0);
     A.cut = reinterpret_cast<const double*>(dv + o_cut);
     A.fill = reinterpret_cast<const double*>(dv + o_fill);
@@ -1535,82 +1516,57 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
     A.warm = warm_dev;
     // launch configuration
     LaunchCfg cfg;
-    // (the dry-row instantiation is tuned apart: its bookkeeping changes the best shape)
-    auto key = std::make_tuple(nx, ny, n, (int)g->mode + (bnd ? 2 : 0) + (A.P.skip_dry ? 4 : 0));
+    auto pack = [&]() -> cudaError_t {   // the kernel's copy of the inputs
+      const size_t PJ = (size_t)pairs(nx) + 2, rec = (size_t)(ny + 1) * PJ;
+      cudaError_t e = ctx->bG.ensure(ny * PJ * 16);
+      if (e == cudaSuccess) e = ctx->bJ.ensure(n * rec * 16);
+      if (e == cudaSuccess && crest) e = ctx->bJ2.ensure(n * rec * 16);
+      if (e == cudaSuccess) e = ctx->bNever.ensure((size_t)n * 4);
+      if (e == cudaSuccess) e = cudaMemsetAsync(ctx->bNever.p, 0, (size_t)n * 4, ctx->stream);
+      if (e != cudaSuccess) return e;
+      PackArgs K;
+      memset(&K, 0, sizeof(K));
+      K.nx = nx; K.ny = ny; K.n = n;
+      K.wet = reinterpret_cast<const float*>(dv + o_wet); K.gn2 = reinterpret_cast<const float*>(dv + o_gn2);
+      K.dzx = reinterpret_cast<const float*>(dv + o_dzx); K.dzy = reinterpret_cast<const float*>(dv + o_dzy);
+      if (crest) { K.dzx2 = reinterpret_cast<const float*>(dv + o_dzx2); K.dzy2 = reinterpret_cast<const float*>(dv + o_dzy2); }
+      K.bc = A.bc; K.bh = A.bh;
+      K.G = ctx->bG.as<float4>(); K.J = ctx->bJ.as<float4>(); K.J2 = crest ? ctx->bJ2.as<float4>() : nullptr;
+      K.never = ctx->bNever.as<unsigned>();
+      k_pack_inputs<<<dim3((unsigned)((rec + 255) / 256), (unsigned)n), 256, 0, ctx->stream>>>(K);
+      launches += 1;
+      A.G = K.G; A.J = K.J; A.J2 = K.J2; A.never = K.never;
+      return cudaGetLastError();
+    };
+    auto key = std::make_tuple(nx, ny, n, (int)g->mode + (bnd ? 2 : 0));
     if (ctx->cluster > 0 || ctx->threads > 0) {
-      cfg = make_cfg(ctx, nx, ny, ctx->cluster > 0 ? ctx->cluster : 1, ctx->threads > 0 ? ctx->threads : 512, crest, bnd);
+      cfg = make_cfg(ctx, nx, ny, ctx->cluster > 0 ? ctx->cluster : 1, ctx->threads > 0 ? ctx->threads : 512, bnd);
       if (!cfg.ok) return fail(ctx, ITR_UNSUPPORTED, "cluster=%d threads=%d does not fit a %dx%d grid in shared memory", ctx->cluster, ctx->threads, nx, ny);
-    } else if (ctx->tuned.count(key) && !(locked && ctx->tuned[key].tiled)) {
+      CU(pack());
+    } else if (ctx->tuned.count(key)) {
       cfg = ctx->tuned[key];
       tiled = cfg.tiled;
-      if (tiled) tiled_band = cfg.band;
+      if (!tiled) CU(pack());
     } else {
-      std::vector<LaunchCfg> cands = candidates(ctx, nx, ny, n, crest, bnd);
-      if (cands.empty()) {
-        tiled = true;   // a design needs more shared memory than 8 CTAs hold
-      } else {
-        // Measured autotuning: time a short probe (the first steps of this very batch) of
-        // the best few shapes by the model and keep the fastest for this (grid, population).
-        cfg = cands[0];
-        if (ctx->autotune) {   // (a single candidate is timed too: the tiled path is compared with it)
-          rc = autotune(ctx, A, cands, n, &cfg);
-          if (rc != ITR_OK) return rc;
-        }
-        if (ctx->autotune && !locked && !ctx->defer) {
-          // the tiled HBM path as one more candidate, timed over the same probe steps (not for
-          // a ladder group: the ladder runs every group's cluster kernel in one graph launch)
-          PlainArgs T;
-          CU(tiled_args(T));   // (no locked schedule here: the tiled candidate is timed only unlocked)
-          T.max_steps = (unsigned long long)ctx->probe_steps;
-          T.warm = nullptr;
-          T.obj.enabled = 0; T.ledger = nullptr; T.max_rows = 0;
-          int dummy = 0;
-          // both update kernels of the tiled path, row bands and 16x16 tiles; direct launches
-          // and one poll: no graph build or host round trips in the timing
-          const int g0 = ctx->graph, k0 = ctx->steps_per_submit;
-          ctx->graph = 0; ctx->steps_per_submit = ctx->probe_steps;
-          for (int bk = 1; bk >= 0 && rc == ITR_OK; --bk) {
-            ctx->band = bk;
-            const dim3 tg = tiled_grid(ctx, nx, ny, n);
-            float t_ms = 0.0f;
-            cudaError_t e = tiled_args(T);
-            T.max_steps = (unsigned long long)ctx->probe_steps;
-            T.warm = nullptr;
-            T.obj.enabled = 0; T.ledger = nullptr; T.max_rows = 0;
-            if (e == cudaSuccess) e = cudaEventRecord(ctx->ev[1], ctx->stream);
-            if (e != cudaSuccess) { rc = fail(ctx, ITR_DEVICE_ERROR, "tiled probe: %s", cudaGetErrorString(e)); break; }
-            rc = run_tiled_batch(ctx, T, n, tg, &dummy);
-            if (rc != ITR_OK) break;
-            e = cudaEventRecord(ctx->ev[2], ctx->stream);
-            if (e == cudaSuccess) e = cudaEventSynchronize(ctx->ev[2]);
-            if (e == cudaSuccess) e = cudaEventElapsedTime(&t_ms, ctx->ev[1], ctx->ev[2]);
-            if (e != cudaSuccess) { rc = fail(ctx, ITR_DEVICE_ERROR, "tiled probe: %s", cudaGetErrorString(e)); break; }
-            if (t_ms < ctx->tune_ms) { cfg.tiled = true; cfg.band = bk; ctx->tune_ms = t_ms; }
-          }
-          ctx->graph = g0; ctx->steps_per_submit = k0;
-          ctx->band = band0;
-          if (rc != ITR_OK) return rc;
-        }
-        if (!(locked && ctx->tuned.count(key))) ctx->tuned[key] = cfg;   // a locked run keeps a cached tiled choice
-        tiled = cfg.tiled;
-        if (tiled) tiled_band = cfg.band;
-      }
+      cfg = batched_shape(ctx, nx, ny, n, crest, bnd);
+      if (!cfg.ok) cfg.tiled = true;   // a design needs more shared memory than 8 CTAs hold
+      ctx->tuned[key] = cfg;
+      tiled = cfg.tiled;
+      if (!tiled) CU(pack());
     }
     if (!tiled) {
       A.C = cfg.C; A.W = cfg.W; A.S = cfg.S;
       if (locked) {
         const size_t nl = ctx->locked_dt.size();
         CU(ctx->lDt.ensure(nl * 8));
-        CU(ctx->lS4.ensure((size_t)n * N * 16));
-        CU(ctx->lS2.ensure((size_t)n * N * 8));
-        CU(ctx->lSk.ensure((size_t)n * N * 4));
+        CU(ctx->lS4.ensure((size_t)n * cfg.C * smem_plan((ny + cfg.C - 1) / cfg.C, nx, cfg.S, cfg.W, cfg.T / 32, bnd ? 1 : 0, ny).state));
         CU(ctx->lSs.ensure((size_t)n * cfg.C * sizeof(LockedSnap)));
         CU(ctx->lFb.ensure((size_t)n * 8));
         CU(cudaMemcpyAsync(ctx->lDt.p, ctx->locked_dt.data(), nl * 8, cudaMemcpyHostToDevice, ctx->stream));
         A.locked_dt = ctx->lDt.as<double>();
         A.n_locked = (unsigned long long)nl;
         A.cfl_hard = ctx->cfl_hard;
-        A.snap4 = ctx->lS4.as<float4>(); A.snap2 = ctx->lS2.as<float2>(); A.snapk = ctx->lSk.as<float>();
+        A.snap = ctx->lS4.as<float4>();
         A.snap_s = ctx->lSs.as<LockedSnap>();
         A.fallback_t = ctx->lFb.as<double>();
         ctx->locked_run = true;
@@ -1639,13 +1595,6 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
     }
   }
   if (tiled) {
-    struct BandScope {   // the tuned kernel choice for this batch; the option stays the caller's
-      itr_ctx* c; int v;
-      ~BandScope() { c->band = v; }
-    } band_scope{ctx, band0};
-    ctx->band = tiled_band;
-    tgrid = tiled_grid(ctx, nx, ny, n);
-    n_tiles = (int)(tgrid.x * tgrid.y);
     const int nb = n_tiles;
     PlainArgs A;
     CU(tiled_args(A));
@@ -1734,7 +1683,7 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
 
 // Uneven batch: several grid groups (the fidelity ladder's coarse, native and half-cell
 // grids) in one CUDA graph launch. Each group is prepared on its own child context (inputs
-// uploaded, launch shape autotuned for its grid) and its persistent cluster kernel becomes
+// uploaded, launch shape chosen for its grid) and its persistent cluster kernel becomes
 // one parallel branch of the graph; a group whose grid needs the tiled path runs on its own
 // before the graph. Results come back per group, in group order.
 extern "C" int itr_gpu_run_ladder(itr_ctx* ctx, const itr_params* p, int32_t n_groups, const itr_group* groups,
@@ -1755,8 +1704,7 @@ extern "C" int itr_gpu_run_ladder(itr_ctx* ctx, const itr_params* p, int32_t n_g
   for (int gi = 0; gi < n_groups; ++gi) {
     itr_ctx* c = ctx->children[gi];
     c->impl = ctx->impl; c->threads = ctx->threads; c->cluster = ctx->cluster; c->graph = ctx->graph;
-    c->steps_per_submit = ctx->steps_per_submit; c->autotune = ctx->autotune; c->autotune_top = ctx->autotune_top;
-    c->probe_steps = ctx->probe_steps; c->exact_special = ctx->exact_special;
+    c->steps_per_submit = ctx->steps_per_submit; c->exact_special = ctx->exact_special;
     c->wait_limit = ctx->wait_limit; c->stall_wait_test = ctx->stall_wait_test;
     if (!c->ev_fork) CU(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
     c->defer = true;

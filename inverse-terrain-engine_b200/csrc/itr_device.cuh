@@ -186,11 +186,36 @@ ITR_DEV CellNew update_cell(float h, float qx, float qy, const FaceF& w, const F
 // every thread of a design redundantly (identical inputs, identical bits).
 constexpr int kMaxRain = 32;
 
+// One linear piece of the rate: r0 + dr (x - t0) / den for x <= end (rden = 1 / den rounded). Piece 0 is
+// the constant before the first point, piece n the constant after the last.
+struct RainSeg { double t0, r0, dr, den, rden, end; };
+
 struct Rain {
   int n;
   double t[kMaxRain];
   double r[kMaxRain];
+  RainSeg seg[kMaxRain + 1];
 };
+
+// a / b rounded to nearest from y = 1 / b rounded to nearest, as fused multiply-adds: a y is within two
+// units of the last place, one correction by the exact residual makes it faithful, a second one
+// rounds it right (P. Markstein, IBM J. Res. Dev. 34(1), 1990; Muller et al., Handbook of
+// Floating-Point Arithmetic, 2nd ed., 2018, ch. 4). Operands and quotient in the normal range, or a = 0.
+ITR_DEV double div_rn(double a, double b, double y) {
+  double q = a * y;
+  q = __fma_rn(__fma_rn(-b, q, a), y, q);
+  return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+// The same for a b that is an f32 above 0: the reciprocal by Newton steps from the hardware's estimate.
+// The last step starts within a unit of 1 / b, so it rounds it right unless b's 53-bit significand is
+// all ones (same sources), which an f32's is not.
+ITR_DEV double div_by_f32(double a, double b) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+#pragma unroll
+  for (int i = 0; i < 3; ++i) y = __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+  return div_rn(a, b, y);
+}
 
 ITR_DEV double rain_rate(const Rain& R, double x) {
   if (R.n == 0) return 0.0;
@@ -378,6 +403,7 @@ struct RunParams {
   Inflow inflow;
   // step-invariant f32 constants (solver.rs:269-285), rounded once on the host
   float g_f, g_half_f, inv_dx_f, inv_dy_f, h_dry_f, heps2_f, q_min_f;
+  double rdx, rdy;   // 1 / dx, 1 / dy rounded (div_rn)
   float nz;   // -0.0f, supplied at run time (see mul2)
   float s_safe;   // largest wave rate of a state whose step may take the branch-free roots (safe_rate_limit)
 };
@@ -425,6 +451,23 @@ ITR_DEV StepPlan plan_step_c(const RunParams& P, double t, uint32_t sync_index, 
   return s;
 }
 
+// The same schedule split for a kernel that overlaps it with work that needs no dt. The rate at the
+// step's start is known from the step before; while no breakpoint lies inside the step the integral is
+// one trapezoid of the piece `seg`, else (or for an unsorted storm) `rare` is set and the general
+// integral replaces s.rain.
+ITR_DEV double rain_piece(const RainSeg& g, double x) { return g.r0 + div_rn(g.dr * (x - g.t0), g.den, g.rden); }
+ITR_DEV StepPlan plan_step_fast(const RunParams& P, double t, double t_sync, double t_hit, double dt_pick, double rate_t, int seg,
+                                bool& rare) {
+  StepPlan s;
+  s.hits = t + dt_pick >= t_hit;
+  s.dt = s.hits ? t_sync - t : dt_pick;
+  const double b = t + s.dt;
+  s.rain = 0.5 * (rate_t + rain_piece(P.rain.seg[seg], b)) * (b - t);
+  rare = b > P.rain.seg[seg].end || !P.rain_sorted;
+  s.t_new = s.hits ? t_sync : b;
+  return s;
+}
+
 // plan_step for a step whose dt before the sync clip is given (the baseline-locked dt).
 ITR_DEV StepPlan plan_step_dt(const RunParams& P, double t, uint32_t sync_index, double dt) {
   StepPlan s;
@@ -456,27 +499,8 @@ ITR_DEV StepK step_consts(const RunParams& P, double dt, double rain) {
   k.g = P.g_f; k.g_half = P.g_half_f; k.inv_dx = P.inv_dx_f; k.inv_dy = P.inv_dy_f;
   k.h_dry = P.h_dry_f; k.heps2 = P.heps2_f; k.q_min = P.q_min_f;
   k.dt = (float)dt;
-  k.dtdx = (float)(dt / P.dx);
-  k.dtdy = (float)(dt / P.dy);
-  k.rain = (float)rain;
-  k.cap = (float)(P.infil * dt);
-  k.nz = P.nz;
-  k.exact = 0u;
-  return k;
-}
-
-ITR_DEV StepK make_consts(const RunParams& P, double dt, double rain) {
-  StepK k;
-  k.g = (float)P.g;
-  k.g_half = (float)(0.5 * P.g);
-  k.dt = (float)dt;
-  k.dtdx = (float)(dt / P.dx);
-  k.dtdy = (float)(dt / P.dy);
-  k.inv_dx = (float)(1.0 / P.dx);
-  k.inv_dy = (float)(1.0 / P.dy);
-  k.h_dry = (float)P.h_dry;
-  k.heps2 = (float)(P.h_eps * P.h_eps);
-  k.q_min = (float)1e-30;
+  k.dtdx = (float)div_rn(dt, P.dx, P.rdx);
+  k.dtdy = (float)div_rn(dt, P.dy, P.rdy);
   k.rain = (float)rain;
   k.cap = (float)(P.infil * dt);
   k.nz = P.nz;
@@ -589,6 +613,11 @@ ITR_DEV float2 fma2(float2 a, float2 b, float2 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pk2(a)), "l"(pk2(b)), "l"(pk2(c)));
   return upk2(r);
 }
+// Products, sums and fused products with a constant or a value shared by all lanes, per component: the
+// pair instruction would hold the constant in a register pair of each lane.
+ITR_DEV float2 mulc2(float c, float2 a) { return make_float2(__fmul_rn(c, a.x), __fmul_rn(c, a.y)); }
+ITR_DEV float2 addc2(float2 a, float c) { return make_float2(__fadd_rn(a.x, c), __fadd_rn(a.y, c)); }
+ITR_DEV float2 fmac2(float c, float2 a, float2 b) { return make_float2(__fmaf_rn(c, a.x, b.x), __fmaf_rn(c, a.y, b.y)); }
 ITR_DEV float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 ITR_DEV float2 sel2(B2 c, float2 a, float2 b) { return make_float2(c.x ? a.x : b.x, c.y ? a.y : b.y); }
 ITR_DEV float2 max2(float2 a, float2 b) { return make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y)); }
@@ -605,7 +634,8 @@ ITR_DEV B2 gt2(float2 a, float b) { return B2{a.x > b, a.y > b}; }
 ITR_DEV float rcp_est(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 ITR_DEV float2 rcp2(float2 x) {
   const float2 y = make_float2(rcp_est(x.x), rcp_est(x.y));
-  return fma2(y, fma2(neg2(x), y, f2(1.0f)), y);
+  const float2 e = make_float2(__fmaf_rn(-x.x, y.x, 1.0f), __fmaf_rn(-x.y, y.y, 1.0f));
+  return fma2(y, e, y);
 }
 // sqrt(x) for x = +0 or x in [2^-149, 2^80): one Newton step from the hardware estimate of
 // 1/sqrt (same sources: s = x y, d = fma(-s, s, x), s + d (y / 2)), on x 2^48 so that the
@@ -615,22 +645,22 @@ ITR_DEV float2 rcp2(float2 x) {
 // B200); about half its time, and without the branch that would end the basic block.
 ITR_DEV float rsqrt_est(float x) { float r; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 ITR_DEV float2 sqrt2(float2 x) {
-  const float2 xs = mulp2(x, f2(0x1p48f));
-  const float2 xt = add2(xs, f2(0x1p-126f));
+  const float2 xs = mulc2(0x1p48f, x);
+  const float2 xt = addc2(xs, 0x1p-126f);
   const float2 y = make_float2(rsqrt_est(xt.x), rsqrt_est(xt.y));
-  const float2 s = mulp2(xs, y), h = mulp2(y, f2(0x1p-25f));
-  return fma2(fma2(neg2(s), s, xs), h, mulp2(s, f2(0x1p-24f)));
+  const float2 s = mulp2(xs, y), h = mulc2(0x1p-25f, y);
+  return fma2(fma2(neg2(s), s, xs), h, mulc2(0x1p-24f, s));
 }
 
 ITR_DEV float2 rcbrt2(float2 x, float nz) {
   float2 r = make_float2(__uint_as_float(0x54A23280u - __float_as_uint(x.x) / 3u),
                          __uint_as_float(0x54A23280u - __float_as_uint(x.y) / 3u));
-  const float2 x3 = mulp2(x, f2((float)(1.0 / 3.0)));
-  const float2 c43 = f2((float)(4.0 * (1.0 / 3.0)));
+  const float2 x3 = mulc2((float)(1.0 / 3.0), x);
+  const float c43 = (float)(4.0 * (1.0 / 3.0));
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const float2 r2 = mulp2(r, r);
-    r = sub2(mul2(r, c43, nz), mul2(x3, mulp2(r2, r2), nz));
+    r = sub2(mulc2(c43, r), mul2(x3, mulp2(r2, r2), nz));
   }
   return r;
 }
@@ -644,24 +674,22 @@ ITR_DEV float2 rcbrt2(float2 x, float nz) {
 ITR_DEV Face2 hll2(float2 hl, float2 ul, float2 tl, float2 cl, float2 hr, float2 ur, float2 tr, float2 cr, float g_half, float nz) {
   const float NZ = nz;
   const B2 wet_l = gt2(hl, 0.0f), wet_r = gt2(hr, 0.0f);
-  const float2 ustar = sub2(fma2(f2(0.5f), add2(ul, ur), cl), cr);
-  const float2 cstar = fma2(f2(0.25f), sub2(ul, ur), mulp2(f2(0.5f), add2(cl, cr)));
+  const float2 ustar = sub2(fmac2(0.5f, add2(ul, ur), cl), cr);
+  const float2 cstar = fmac2(0.25f, sub2(ul, ur), mulc2(0.5f, add2(cl, cr)));
   const float2 ul_cl = sub2(ul, cl);
   const float2 ur_cr = add2(ur, cr);
   const float2 slw = min2(ul_cl, sub2(ustar, cstar));
   const float2 srw = max2(ur_cr, add2(ustar, cstar));
-  const float2 sl = sel2(wet_l, sel2(wet_r, slw, ul_cl), fma2(f2(-2.0f), cr, ur));
-  const float2 sr = sel2(wet_l, sel2(wet_r, srw, fma2(f2(2.0f), cl, ul)), ur_cr);
+  const float2 sl = sel2(wet_l, sel2(wet_r, slw, ul_cl), fmac2(-2.0f, cr, ur));
+  const float2 sr = sel2(wet_l, sel2(wet_r, srw, fmac2(2.0f, cl, ul)), ur_cr);
   const float2 ml = mul2(hl, ul, NZ);
   const float2 mr = mul2(hr, ur, NZ);
-  const float2 gh = f2(g_half);
-  const float2 pl_ = mul2(mulp2(gh, hl), hl, NZ);
-  const float2 pr_ = mul2(mulp2(gh, hr), hr, NZ);
+  const float2 pl_ = mul2(mulc2(g_half, hl), hl, NZ);
+  const float2 pr_ = mul2(mulc2(g_half, hr), hr, NZ);
   const float2 pl = add2(mul2(ml, ul, NZ), pl_);
   const float2 pr = add2(mul2(mr, ur, NZ), pr_);
   const B2 use_l = B2{sl.x >= 0.0f, sl.y >= 0.0f}, use_r = B2{sr.x <= 0.0f, sr.y <= 0.0f};
-  const B2 trivial = B2{use_l.x || use_r.x, use_l.y || use_r.y};
-  const float2 inv = rcp2(sel2(trivial, f2(1.0f), sub2(sr, sl)));
+  const float2 inv = rcp2(sub2(sr, sl));   // (not read where an upwind flux is taken)
   const float2 slsr = mulp2(sl, sr);
   const float2 fm_star = mul2(add2(sub2(mul2(sr, ml, NZ), mul2(sl, mr, NZ)), mul2(slsr, sub2(hr, hl), NZ)), inv, NZ);
   const float2 fn_star = mul2(add2(sub2(mul2(sr, pl, NZ), mul2(sl, pr, NZ)), mul2(slsr, sub2(mr, ml), NZ)), inv, NZ);
@@ -685,14 +713,14 @@ ITR_DEV Face2 face2(float2 hl, float2 ul, float2 vl, float2 cl, float2 hr, float
     const B2 pos = gt2(d0, 0.0f);
     hsl = max2z(sub2(hl, max2z(d0)));
     hsr = max2z(sub2(hr, max2z(neg2(d0))));
-    const float2 cred = sqrt2(mul2(f2(k.g), sel2(pos, hsl, hsr), NZ));
+    const float2 cred = sqrt2(mulc2(k.g, sel2(pos, hsl, hsr)));
     csl = sel2(pos, cred, cl);
     csr = sel2(pos, cr, cred);
   } else {
     hsl = max2z(sub2(hl, d0));
     hsr = max2z(sub2(hr, d1));
     const B2 pl = gt2(d0, 0.0f), pr = gt2(d1, 0.0f);
-    const float2 sl = sqrt2(mul2(f2(k.g), hsl, NZ)), sr = sqrt2(mul2(f2(k.g), hsr, NZ));
+    const float2 sl = sqrt2(mulc2(k.g, hsl)), sr = sqrt2(mulc2(k.g, hsr));
     csl = sel2(pl, sl, cl);
     csr = sel2(pr, sr, cr);
   }
@@ -705,13 +733,17 @@ struct CellNew2 {
   float2 h, qx, qy, s, infil, fix, c, low;
 };
 
+// The step's dt / dx, dt / dy and the grid's 1 / dx, 1 / dy per component: 0 for a component whose
+// cell stays as it is and adds nothing to the step's sums (a lane's idle columns).
+struct UpdK { float2 dtdx, dtdy, inv_dx, inv_dy; };
+
 // flux_update then sources (numerics.rs:144-195) on two cells with finite, bounded states.
 // Momentum: the reference multiplies by keep = 0 where the new depth is below h_dry and then
 // flushes |q| < q_min to 0; both are one select here (a dry cell's q is 0 either way).
 ITR_DEV CellNew2 update_cell2(float2 h, float2 qx, float2 qy, const Face2& w, const Face2& e, const Face2& n,
-                              const Face2& s, float2 wet, float2 gn2, const StepK& k) {
+                              const Face2& s, float2 wet, float2 gn2, const StepK& k, const UpdK& uk) {
   const float NZ = k.nz;
-  const float2 dtdx = f2(k.dtdx), dtdy = f2(k.dtdy);
+  const float2 dtdx = uk.dtdx, dtdy = uk.dtdy;
   CellNew2 o;
   const float2 h1 = sub2(sub2(h, mul2(dtdx, sub2(e.m, w.m), NZ)), mul2(dtdy, sub2(s.m, n.m), NZ));
   const float2 qx1 = sub2(sub2(qx, mul2(dtdx, sub2(e.nl, w.nr), NZ)), mul2(dtdy, sub2(s.t, n.t), NZ));
@@ -719,23 +751,23 @@ ITR_DEV CellNew2 update_cell2(float2 h, float2 qx, float2 qy, const Face2& w, co
   o.low = h1;
   const float2 hc = max2z(h1);
   o.fix = sub2(hc, h1);
-  const float2 h2 = add2(hc, mul2(f2(k.rain), wet, NZ));
-  o.infil = min2(mulp2(f2(k.cap), wet), h2);
+  const float2 h2 = add2(hc, mulc2(k.rain, wet));
+  o.infil = min2(mulc2(k.cap, wet), h2);
   const float2 h3 = sub2(h2, o.infil);
   const B2 dry = B2{h3.x < k.h_dry, h3.y < k.h_dry};
   const float2 r = rcbrt2(sel2(dry, f2(1.0f), h3), NZ);
   const float2 r3 = mulp2(mulp2(r, r), r);
   const float2 r7 = mulp2(mulp2(r3, r3), r);
   const float2 qm = sqrt2(add2(mul2(qx1, qx1, NZ), mul2(qy1, qy1, NZ)));
-  const float2 inv = rcp2(add2(f2(1.0f), mul2(mulp2(mulp2(f2(k.dt), gn2), qm), r7, NZ)));
+  const float2 inv = rcp2(addc2(mul2(mulp2(mulc2(k.dt, gn2), qm), r7, NZ), 1.0f));
   const float2 tx = mulp2(qx1, inv), ty = mulp2(qy1, inv);
   o.qx = make_float2(fabsf(tx.x) >= k.q_min && !dry.x ? tx.x : 0.0f, fabsf(tx.y) >= k.q_min && !dry.y ? tx.y : 0.0f);
   o.qy = make_float2(fabsf(ty.x) >= k.q_min && !dry.x ? ty.x : 0.0f, fabsf(ty.y) >= k.q_min && !dry.y ? ty.y : 0.0f);
-  const float2 c = sqrt2(mul2(f2(k.g), h3, NZ));
+  const float2 c = sqrt2(mulc2(k.g, h3));
   const float2 ax = mul2(o.qx, r3, NZ), ay = mul2(o.qy, r3, NZ);   // |q| r3 = |q r3|
   const float2 sx = make_float2(fabsf(ax.x) + c.x, fabsf(ax.y) + c.y), sy = make_float2(fabsf(ay.x) + c.x, fabsf(ay.y) + c.y);
-  o.s = add2(mul2(sx, f2(k.inv_dx), NZ), mul2(sy, f2(k.inv_dy), NZ));
-  o.h = add2(h3, f2(0.0f));   // canon: -0 becomes +0
+  o.s = add2(mul2(sx, uk.inv_dx, NZ), mul2(sy, uk.inv_dy, NZ));
+  o.h = addc2(h3, 0.0f);   // canon: -0 becomes +0
   o.c = c;
   return o;
 }
@@ -743,11 +775,11 @@ ITR_DEV CellNew2 update_cell2(float2 h, float2 qx, float2 qy, const Face2& w, co
 // Paired desingularised velocity and celerity (cell_vel on two cells).
 ITR_DEV void vel2(float2 h, float2 qx, float2 qy, const StepK& k, float2& u, float2& v) {
   const float2 h2 = mul2(h, h, k.nz);
-  const float2 t = mulp2(add2(h, h), rcp2(add2(h2, max2(h2, f2(k.heps2)))));
+  const float2 t = mulp2(add2(h, h), rcp2(add2(h2, make_float2(fmaxf(h2.x, k.heps2), fmaxf(h2.y, k.heps2)))));
   u = mul2(qx, t, k.nz);
   v = mul2(qy, t, k.nz);
 }
-ITR_DEV float2 cel2(float2 h, const StepK& k) { return sqrt2(mul2(f2(k.g), h, k.nz)); }
+ITR_DEV float2 cel2(float2 h, const StepK& k) { return sqrt2(mulc2(k.g, h)); }
 
 // The same through the scalar path, for steps with StepK::exact set (rare: not inlined).
 ITR_DEV Face2 face2_of(const FaceF& a, const FaceF& b) {
