@@ -2,7 +2,7 @@
 //
 // The design's state stays in the ping-pong planes of the tiled path (PlainArgs: H, QX, QY
 // [2][nx*ny], running peaks PK), the integrator in its control block (PlainCtl, advanced by
-// k_plain_finalize); only the per-step update differs from k_plain_update. It is the row
+// plain_finalize_body in the last block, or by k_plain_finalize_locked); only the per-step update differs from k_plain_update. It is the row
 // sweep of the cluster kernel (itr_batched.cuh) and of the reference's fused CPU kernel
 // (crates/itr-hydro/src/kernel.rs:637-697), laid out for a state that is read from HBM:
 //   * a warp owns a segment of 64 columns of a band of kBandRows rows; lane l holds the two
@@ -21,6 +21,13 @@
 //   * the old state is read-only during a step (ping-pong), so warps never synchronise with
 //     each other inside a step: row r + 1 is loaded while row r is updated, and the only
 //     block barrier is the final reduction of the per-block partials.
+// What bounds it: the row arithmetic (56 % of the issue slots, register-file reads; a step of 16 designs
+// of 1024 x 1024 moves 48 B per cell in 0.29 ms, 2.7 TB/s). So a row's inputs come as two records
+// (jumps, wet | g n^2) of 16 B per pair, the columns past the grid are masked once per step instead of
+// once per row, a row's ghosts are filled in when it is used (filled in at the load they made every
+// row wait for memory: 285 ms against 238 ms of 16 designs x 959 steps; the layout with separate arrays
+// took 256 ms), and the last block of a design advances its integrator, so that a step is one
+// launch: one design of 1024 x 1024, 681 steps, 21.5 ms -> 19.3 ms.
 // Outputs are k_plain_update's: the new plane, PK (and the argmax state index tpk), the
 // per-block partials [kPart] in the finalize's layout, and the atomic smax / bad words.
 // TAPE: the adjoint's replay of a recorded step (itr_adjoint_band.cuh): the same update, writing
@@ -118,33 +125,8 @@ ITR_DEV void band_cell(const PlainArgs& A, const PlainDesign& D, const float2* i
   else ghost_state<false>(code, h, qx, qy, hs, fi, gyn);
 }
 
-// Raw (not yet velocity-complemented) state of the lane's two cells of row r.
+// Raw (not yet velocity-complemented) state of the lane's two cells of a row.
 struct Raw2 { float2 h, qx, qy; };
-
-template <bool BND>
-ITR_DEV Raw2 band_row(const PlainArgs& A, const PlainDesign& D, const float2* inf, size_t plane, int r, int c0, bool interior) {
-  Raw2 o;
-  if (interior) {   // both columns inside the grid and r a grid row: plain loads
-    const size_t i = plane + (size_t)r * A.nx + c0;
-    if ((A.nx & 1) == 0) {   // even rows: the pair is 8-byte aligned (c0 and the plane size are even)
-      o.h = *reinterpret_cast<const float2*>(D.H + i);
-      o.qx = *reinterpret_cast<const float2*>(D.QX + i);
-      o.qy = *reinterpret_cast<const float2*>(D.QY + i);
-    } else {
-      o.h = make_float2(D.H[i], D.H[i + 1]);
-      o.qx = make_float2(D.QX[i], D.QX[i + 1]);
-      o.qy = make_float2(D.QY[i], D.QY[i + 1]);
-    }
-    return o;
-  }
-  band_cell<BND>(A, D, inf, plane, r, c0, o.h.x, o.qx.x, o.qy.x);
-  band_cell<BND>(A, D, inf, plane, r, c0 + 1, o.h.y, o.qx.y, o.qy.y);
-  return o;
-}
-
-// Inputs of one row for the lane's two columns: south y-face jumps (face row r + 1), x-face
-// jumps of row r + 1, wet and g n^2 of row r.
-struct RowIn { float2 dys, dys2, dxn, dxn2, wet, gn2, pk; };
 
 // Sums of one warp's sweep (one step): the finalize's partials, the largest wave rate, the lowest
 // depth before the positivity fix, and whether a cell left the bounds of the branch-free step
@@ -157,8 +139,9 @@ struct BandAcc {
 };
 
 // A warp's segment of one band. EX: every root and reciprocal through the scalar path (k.exact).
-template <bool EX, bool CREST, bool BND, bool TAPE>
-ITR_DEV void band_sweep(const PlainArgs& A, const PlainDesign& D, const PlainCtl& cl, const StepK& k, int s, int r0, int r1,
+// SKIP: with the dry-row test (only launched where the storm leaves a rain-free step).
+template <bool EX, bool CREST, bool BND, bool TAPE, bool SKIP>
+ITR_DEV void band_sweep(const PlainArgs& A, const PlainDesign& D, const PlainCtl& cl, const StepK& k, int d, int s, int r0, int r1,
                         float4* edge_w, float4* edge_e, BandAcc& acc) {
   const int par = cl.par;
   const bool hits = cl.pl.hits;
@@ -170,19 +153,29 @@ ITR_DEV void band_sweep(const PlainArgs& A, const PlainDesign& D, const PlainCtl
   const int lane = threadIdx.x & 31;
   const int L = r1 - r0;
   const int cw = 64 * s, ce = cw + 64;              // the segment's edge x-faces
-  const int c0 = cw + 2 * lane, c1 = c0 + 1;
-  const bool v0 = c0 < nx, v1 = c1 < nx;            // cells of the lane
-  const bool interior = c1 < nx;                    // both columns are grid cells
-  const bool vec = interior && (nx & 1) == 0;       // their pairs are 8-byte aligned in every plane
+  // The lane's pair of columns; a pair past the grid reads the last one, whose mirror is the east ghost.
+  const int P2 = pairs(nx), PJ = P2 + 2, p = 32 * s + lane, pl = p < P2 ? p : P2 - 1;
+  const int c0 = 2 * p;
+  const bool even = (nx & 1) == 0;                   // pairs are 8-byte aligned in every plane
+  const bool v0 = p < P2, v1 = c0 + 1 < nx;         // cells of the lane
+  const bool y_in = 2 * pl + 1 < nx;                 // the pair read has two cells
+  const bool mir_x = even && p >= P2, mir_y = !even && p >= P2 - 1;   // ghost from the pair's other column
+  const bool edge = mir_x || mir_y;
   const bool last_seg = ce > nx;                    // the east domain edge lies inside this segment
+  const float2 mask = make_float2(v0 ? 1.0f : 0.0f, v1 ? 1.0f : 0.0f);
+  const int jr = p + 1 <= P2 + 1 ? p + 1 : 0, gr = v0 ? p + 1 : 0;    // the pair's records (0: zeros)
+  const float4* const Jl = A.J + (size_t)d * (ny + 1) * PJ + jr;
+  const float4* const J2l = CREST ? A.J2 + (size_t)d * (ny + 1) * PJ + jr : nullptr;
+  const float4* const Gl = A.G + gr;
+
   // Dry-row skipping (kernel.rs:605-612): with no rain this step, grid row r is skipped when
   // padded rows r, r + 1, r + 2 (grid rows r - 1, r, r + 1 and their ghosts) held no water
   // in the old state. Its faces are then exactly 0 and its cells keep their (zero) state, so
   // skipping changes no result. Bit p of skipm: grid row r0 + p; bit i of m: padded row r0 + i.
   unsigned long long skipm = 0ull;
-  const unsigned* rw_old = D.rowwet ? D.rowwet + (size_t)par * (ny + 2) : nullptr;
-  unsigned* rw_new = D.rowwet ? D.rowwet + (size_t)(par ^ 1) * (ny + 2) : nullptr;
-  if (!TAPE && rw_old && A.P.skip_dry && !(k.rain > 0.0f)) {
+  const unsigned* rw_old = SKIP ? D.rowwet + (size_t)par * (ny + 2) : nullptr;
+  unsigned* rw_new = SKIP ? D.rowwet + (size_t)(par ^ 1) * (ny + 2) : nullptr;
+  if (SKIP && !(k.rain > 0.0f)) {
     const int ja = r0 + lane, jb = r0 + 32 + lane;
     const bool da = ja <= ny + 1 && plain_row_dry(rw_old, D.gwet, ja);
     const bool db = lane < 2 && jb <= ny + 1 && plain_row_dry(rw_old, D.gwet, jb);
@@ -193,29 +186,65 @@ ITR_DEV void band_sweep(const PlainArgs& A, const PlainDesign& D, const PlainCtl
   // Rows the sweep needs: row p is updated unless skipped, and its state and inputs are also
   // read for the next row's west faces; need(p) is false when rows p and p + 1 (or the band's
   // end) are both skipped, and then nothing of row p is loaded.
-  auto skipped = [&](int p) -> bool { return p >= L || ((skipm >> p) & 1ull); };
-  auto need = [&](int p) -> bool { return !(skipped(p) && skipped(p + 1)); };
+  auto skipped = [&](int q) -> bool { return SKIP && (q >= L || ((skipm >> q) & 1ull)); };
+  auto need = [&](int q) -> bool { return !SKIP || !(skipped(q) && skipped(q + 1)); };
+
+  // A row's raw state: the pair of the nearest grid row, and what the loads leave out (the rows
+  // beyond the domain's edges, the column beyond the east edge). The second half waits for the loads, so it
+  // runs when the row is used, a row of arithmetic after they were issued.
+  auto load_row = [&](int r) -> Raw2 {
+    const int rr = r < 0 ? 0 : r >= ny ? ny - 1 : r;
+    const size_t i = pin + (size_t)rr * nx + 2 * pl;
+    Raw2 o;
+    if (even) {
+      o.h = *reinterpret_cast<const float2*>(D.H + i);
+      o.qx = *reinterpret_cast<const float2*>(D.QX + i);
+      o.qy = *reinterpret_cast<const float2*>(D.QY + i);
+    } else {
+      o.h = make_float2(D.H[i], y_in ? D.H[i + 1] : 0.0f);
+      o.qx = make_float2(D.QX[i], y_in ? D.QX[i + 1] : 0.0f);
+      o.qy = make_float2(D.QY[i], y_in ? D.QY[i + 1] : 0.0f);
+    }
+    return o;
+  };
+  auto ghosts = [&](Raw2& o, int r) {
+    if (r < 0 || r >= ny) {   // north or south ghost row (its east ghost is not read)
+      for (int e = 0; e < 2; ++e) {
+        float &h = e ? o.h.y : o.h.x, &qx = e ? o.qx.y : o.qx.x, &qy = e ? o.qy.y : o.qy.x;
+        const int pos = (r < 0 ? 0 : nx) + 2 * pl + e;
+        const int code = e == 0 || y_in ? A.bc[pos] : 1;
+        const float hs = BND && code == 2 ? D.bh[pos] : 0.0f;
+        const float2 fi = BND && code >= 3 ? inf[code - 3] : make_float2(0.0f, 0.0f);
+        ghost_state<false>(code, h, qx, qy, hs, fi, r < 0);
+      }
+    } else if (edge) {
+      float h = mir_x ? o.h.y : o.h.x, qx = mir_x ? o.qx.y : o.qx.x, qy = mir_x ? o.qy.y : o.qy.x;
+      const int pos = 2 * nx + ny + r, code = A.bc[pos];
+      const float hs = BND && code == 2 ? D.bh[pos] : 0.0f;
+      const float2 fi = BND && code >= 3 ? inf[code - 3] : make_float2(0.0f, 0.0f);
+      ghost_state<true>(code, h, qx, qy, hs, fi, false);
+      if (mir_x) { o.h.x = h; o.qx.x = qx; o.qy.x = qy; } else { o.h.y = h; o.qx.y = qx; o.qy.y = qy; }
+    }
+  };
+
   // ---- pre-pass: the segment's two edge x-faces of every row of the band (skipped rows:
   //      zero faces, which they are) ----
   {
     const int r = r0 + lane;
     Raw2 lf, rt;
     float2 d0 = f2(0.0f), d1 = f2(0.0f);
+    lf.h = lf.qx = lf.qy = rt.h = rt.qx = rt.qy = f2(0.0f);
     if (r < r1 && !skipped(lane)) {
       band_cell<BND>(A, D, inf, pin, r, cw - 1, lf.h.x, lf.qx.x, lf.qy.x);
       band_cell<BND>(A, D, inf, pin, r, cw, rt.h.x, rt.qx.x, rt.qy.x);
       if (ce <= nx) {
         band_cell<BND>(A, D, inf, pin, r, ce - 1, lf.h.y, lf.qx.y, lf.qy.y);
         band_cell<BND>(A, D, inf, pin, r, ce, rt.h.y, rt.qx.y, rt.qy.y);
-      } else {
-        lf.h.y = lf.qx.y = lf.qy.y = rt.h.y = rt.qx.y = rt.qy.y = 0.0f;
       }
       const size_t xo = (size_t)r * nxp1;
       d0.x = D.dzx[xo + cw];
       d0.y = ce <= nx ? D.dzx[xo + ce] : 0.0f;
       if (CREST) { d1.x = D.dzx2[xo + cw]; d1.y = ce <= nx ? D.dzx2[xo + ce] : 0.0f; }
-    } else {
-      lf.h = lf.qx = lf.qy = rt.h = rt.qx = rt.qy = f2(0.0f);
     }
     const Cell2 a = cells_of<EX>(lf.h, lf.qx, lf.qy, k), b = cells_of<EX>(rt.h, rt.qx, rt.qy, k);
     const Face2 f = band_face<EX, true, CREST>(a, b, d0, d1, k);
@@ -235,161 +264,140 @@ ITR_DEV void band_sweep(const PlainArgs& A, const PlainDesign& D, const PlainCtl
 
   // ---- row sweep ----
   UpdK uk;
-  uk.dtdx = f2(k.dtdx); uk.dtdy = f2(k.dtdy); uk.inv_dx = f2(k.inv_dx); uk.inv_dy = f2(k.inv_dy);
-  const float* dzx = D.dzx + c0;
-  const float* dzy = D.dzy + c0;
-  auto load_in = [&](int r) -> RowIn {   // inputs of row r (r < r1)
-    RowIn q;
-    const int rn = r + 1 < ny ? r + 1 : ny - 1;   // next row's x-faces (unused for the last row)
-    const size_t fy = (size_t)(r + 1) * nx, fx = (size_t)rn * nxp1, fc = (size_t)r * nx;
-    q.dxn = make_float2(c0 <= nx ? dzx[fx] : 0.0f, c1 <= nx ? dzx[fx + 1] : 0.0f);
-    q.dys2 = q.dxn2 = f2(0.0f);
-    if (CREST) {
-      q.dys2 = make_float2(v0 ? D.dzy2[c0 + fy] : 0.0f, v1 ? D.dzy2[c0 + fy + 1] : 0.0f);
-      q.dxn2 = make_float2(c0 <= nx ? D.dzx2[c0 + fx] : 0.0f, c1 <= nx ? D.dzx2[c0 + fx + 1] : 0.0f);
-    }
-    const size_t ci = fc + c0;
-    if (vec) {   // 8-byte aligned pairs (even nx, both columns in the grid)
-      q.wet = *reinterpret_cast<const float2*>(A.wet + ci);
-      q.gn2 = *reinterpret_cast<const float2*>(A.gn2 + ci);
-      q.pk = TAPE ? f2(0.0f) : *reinterpret_cast<const float2*>(D.PK + ci);
-      q.dys = *reinterpret_cast<const float2*>(dzy + fy);
-    } else {
-      q.dys = make_float2(v0 ? dzy[fy] : 0.0f, v1 ? dzy[fy + 1] : 0.0f);
-      q.wet = make_float2(v0 ? A.wet[ci] : 0.0f, v1 ? A.wet[ci + 1] : 0.0f);
-      q.gn2 = make_float2(v0 ? A.gn2[ci] : 0.0f, v1 ? A.gn2[ci + 1] : 0.0f);
-      q.pk = TAPE ? f2(0.0f) : make_float2(v0 ? D.PK[ci] : 0.0f, v1 ? D.PK[ci + 1] : 0.0f);
-    }
-    return q;
-  };
-  auto xfaces = [&](const Cell2& c, float2 d, float2 d2, int p) -> Face2 {
-    // west faces of the lane's two columns: (c0 - 1 | c0) and (c0 | c1); lane 0's first
+  uk.dtdx = mulc2(k.dtdx, mask); uk.dtdy = mulc2(k.dtdy, mask); uk.inv_dx = mulc2(k.inv_dx, mask); uk.inv_dy = mulc2(k.inv_dy, mask);
+  auto xfaces = [&](const Cell2& c, float2 j, float2 j2, int q) -> Face2 {
+    // west faces of the lane's two columns: (c0 - 1 | c0) and (c0 | c0 + 1); lane 0's first
     // one is the segment's west edge face from the pre-pass
     Cell2 left;
-    left.h = make_float2(__shfl_up_sync(0xffffffffu, c.h.y, 1), c.h.x);
-    left.u = make_float2(__shfl_up_sync(0xffffffffu, c.u.y, 1), c.u.x);
-    left.v = make_float2(__shfl_up_sync(0xffffffffu, c.v.y, 1), c.v.x);
-    left.c = make_float2(__shfl_up_sync(0xffffffffu, c.c.y, 1), c.c.x);
+    left.h = west2(c.h); left.u = west2(c.u); left.v = west2(c.v); left.c = west2(c.c);
     left.qx = left.qy = f2(0.0f);
-    Face2 f = band_face<EX, true, CREST>(left, c, d, d2, k);
+    Face2 f = band_face<EX, true, CREST>(left, c, j, j2, k);
     if (lane == 0) {
-      const FaceF w = ff(edge_w[p]);
+      const FaceF w = ff(edge_w[q]);
       f.m.x = w.m; f.nl.x = w.nl; f.nr.x = w.nr; f.t.x = w.t;
     }
     return f;
   };
-  // the row above the band (old state; the north ghost row at the domain edge) and row r0
-  const bool int_lane = interior;
+  const float4 zero4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   Cell2 cur{}, nxt{};
   Face2 fN{}, fW{};
   if (!skipped(0)) {
-    const Raw2 ta = band_row<BND>(A, D, inf, pin, r0 - 1, c0, int_lane && r0 > 0);
-    const Raw2 ca = band_row<BND>(A, D, inf, pin, r0, c0, int_lane);
+    Raw2 ta = load_row(r0 - 1), ca = load_row(r0);   // the row above the band and its first
+    ghosts(ta, r0 - 1);
+    ghosts(ca, r0);
     const Cell2 top = cells_of<EX>(ta.h, ta.qx, ta.qy, k);
     cur = cells_of<EX>(ca.h, ca.qx, ca.qy, k);
-    const size_t fy = (size_t)r0 * nx, fx = (size_t)r0 * nxp1;
-    const float2 dy0 = make_float2(v0 ? dzy[fy] : 0.0f, v1 ? dzy[fy + 1] : 0.0f);
-    const float2 dy1 = CREST ? make_float2(v0 ? D.dzy2[c0 + fy] : 0.0f, v1 ? D.dzy2[c0 + fy + 1] : 0.0f) : f2(0.0f);
-    const float2 dx0 = make_float2(c0 <= nx ? dzx[fx] : 0.0f, c1 <= nx ? dzx[fx + 1] : 0.0f);
-    const float2 dx1 = CREST ? make_float2(c0 <= nx ? D.dzx2[c0 + fx] : 0.0f, c1 <= nx ? D.dzx2[c0 + fx + 1] : 0.0f) : f2(0.0f);
-    fN = band_face<EX, false, CREST>(top, cur, dy0, dy1, k);
-    fW = xfaces(cur, dx0, dx1, 0);
-    if (!TAPE && r0 == 0) {   // y_boundary top (kernel.rs:452-472): summed over the row first
+    const float4 j = __ldg(Jl + (size_t)r0 * PJ), j2 = CREST ? __ldg(J2l + (size_t)r0 * PJ) : zero4;
+    fN = band_face<EX, false, CREST>(top, cur, lo2(j), lo2(j2), k);
+    fW = xfaces(cur, hi2(j), hi2(j2), 0);
+    if (!TAPE && r0 == 0)   // y_boundary top (kernel.rs:452-472): summed over the row first
       acc.ytop += (v0 ? (double)fN.m.x : 0.0) + (v1 ? (double)fN.m.y : 0.0);
+  }
+  // inputs of row r, the jumps below it and west of row r + 1
+  float4 jn = zero4, jn2 = zero4, gn = zero4;
+  float2 pn = f2(0.0f);
+  Raw2 raw;
+  raw.h = raw.qx = raw.qy = f2(0.0f);
+  auto load_in = [&](int r) {
+    jn = __ldg(Jl + (size_t)(r + 1) * PJ);
+    if (CREST) jn2 = __ldg(J2l + (size_t)(r + 1) * PJ);
+    gn = __ldg(Gl + (size_t)r * PJ);
+    if (!TAPE) {
+      const size_t i = (size_t)r * nx + 2 * pl;
+      if (even) pn = *reinterpret_cast<const float2*>(D.PK + i);
+      else pn = make_float2(D.PK[i], y_in ? D.PK[i + 1] : 0.0f);
     }
-  }
-  RowIn in{};
-  Raw2 raw{};
-  if (need(0)) {
-    in = load_in(r0);
-    raw = band_row<BND>(A, D, inf, pin, r0 + 1, c0, int_lane && r0 + 1 < ny);
-  }
+    raw = load_row(r + 1);
+  };
+  if (need(0)) load_in(r0);
 #pragma unroll 1
-  for (int p = 0; p < L; ++p) {
-    const int r = r0 + p;
-    const RowIn q = in;
-    const bool skip = skipped(p);
-    if (need(p)) nxt = cells_of<EX>(raw.h, raw.qx, raw.qy, k);
-    if (p + 1 < L && need(p + 1)) {   // next row's operands, in flight while this row is updated
-      in = load_in(r + 1);
-      raw = band_row<BND>(A, D, inf, pin, r + 2, c0, int_lane && r + 2 < ny);
+  for (int q = 0; q < L; ++q) {
+    const int r = r0 + q;
+    const float4 j = jn, j2 = jn2, g = gn;
+    const float2 pk = pn;
+    if (need(q)) {
+      ghosts(raw, r + 1);
+      nxt = cells_of<EX>(raw.h, raw.qx, raw.qy, k);
     }
+    if (q + 1 < L && need(q + 1)) load_in(r + 1);   // next row's operands, in flight while this row is updated
     Face2 fWn{};
-    if (!skipped(p + 1)) fWn = xfaces(nxt, q.dxn, q.dxn2, p + 1);
-    if (skip) {   // a dry row between dry rows: zero faces, the (zero) state carried over
-      const size_t ci = (size_t)r * nx + c0;
-      if (vec) {
-        *reinterpret_cast<float2*>(D.H + pout + ci) = f2(0.0f);
-        *reinterpret_cast<float2*>(D.QX + pout + ci) = f2(0.0f);
-        *reinterpret_cast<float2*>(D.QY + pout + ci) = f2(0.0f);
-      } else {
-        if (v0) { D.H[pout + ci] = 0.0f; D.QX[pout + ci] = 0.0f; D.QY[pout + ci] = 0.0f; }
-        if (v1) { D.H[pout + ci + 1] = 0.0f; D.QX[pout + ci + 1] = 0.0f; D.QY[pout + ci + 1] = 0.0f; }
-      }
+    const size_t ci = (size_t)r * nx + c0;
+    if (SKIP && skipped(q)) {   // a dry row between dry rows: zero faces, the (zero) state carried over
+      if (!skipped(q + 1)) fWn = xfaces(nxt, hi2(j), hi2(j2), q + 1);
+      if (v0) { D.H[pout + ci] = 0.0f; D.QX[pout + ci] = 0.0f; D.QY[pout + ci] = 0.0f; }
+      if (v1) { D.H[pout + ci + 1] = 0.0f; D.QX[pout + ci + 1] = 0.0f; D.QY[pout + ci + 1] = 0.0f; }
       cur = nxt; fN = Face2{}; fW = fWn;
       continue;
     }
-    const Face2 fS = band_face<EX, false, CREST>(cur, nxt, q.dys, q.dys2, k);
+    const Face2 fS = band_face<EX, false, CREST>(cur, nxt, lo2(j), lo2(j2), k);
+    // (the row after the band's last is faced too, and not read: one straight-line body)
+    fWn = xfaces(nxt, hi2(j), hi2(j2), q + 1 < L ? q + 1 : q);
     // east faces: the second column's west face, and lane + 1's first (lane 31: the edge)
     Face2 fE;
-    fE.m.x = fW.m.y; fE.nl.x = fW.nl.y; fE.nr.x = fW.nr.y; fE.t.x = fW.t.y;
-    fE.m.y = __shfl_down_sync(0xffffffffu, fW.m.x, 1);
-    fE.nl.y = __shfl_down_sync(0xffffffffu, fW.nl.x, 1);
-    fE.nr.y = __shfl_down_sync(0xffffffffu, fW.nr.x, 1);
-    fE.t.y = __shfl_down_sync(0xffffffffu, fW.t.x, 1);
+    fE.m = east2(fW.m); fE.nl = east2(fW.nl); fE.nr = east2(fW.nr); fE.t = east2(fW.t);
     if (lane == 31) {
-      const FaceF e = ff(edge_e[p]);
+      const FaceF e = ff(edge_e[q]);
       fE.m.y = e.m; fE.nl.y = e.nl; fE.nr.y = e.nr; fE.t.y = e.t;
     }
     CellNew2 o;
-    if constexpr (EX) o = update_cell2_exact(cur.h, cur.qx, cur.qy, fW, fE, fN, fS, q.wet, q.gn2, k);
-    else o = update_cell2(cur.h, cur.qx, cur.qy, fW, fE, fN, fS, q.wet, q.gn2, k, uk);
-    const size_t ci = (size_t)r * nx + c0;
-    if (vec) {
-      *reinterpret_cast<float2*>(D.H + pout + ci) = o.h;
-      *reinterpret_cast<float2*>(D.QX + pout + ci) = o.qx;
-      *reinterpret_cast<float2*>(D.QY + pout + ci) = o.qy;
+    if constexpr (EX) {
+      o = update_cell2_exact(cur.h, cur.qx, cur.qy, fW, fE, fN, fS, lo2(g), hi2(g), k);
+      if (!v0) { o.s.x = o.low.x = o.infil.x = o.fix.x = 0.0f; }   // (idle columns need not be finite here)
+      if (!v1) { o.s.y = o.low.y = o.infil.y = o.fix.y = 0.0f; }
+      acc.uns = acc.uns || !state_safe(A.P, o.s.x) || !state_safe(A.P, o.s.y);
+    } else {
+      o = update_cell2(cur.h, cur.qx, cur.qy, fW, fE, fN, fS, lo2(g), hi2(g), k, uk);
+    }
+    if (even) {
+      if (v0) {
+        *reinterpret_cast<float2*>(D.H + pout + ci) = o.h;
+        *reinterpret_cast<float2*>(D.QX + pout + ci) = o.qx;
+        *reinterpret_cast<float2*>(D.QY + pout + ci) = o.qy;
+      }
     } else {
       if (v0) { D.H[pout + ci] = o.h.x; D.QX[pout + ci] = o.qx.x; D.QY[pout + ci] = o.qy.x; }
       if (v1) { D.H[pout + ci + 1] = o.h.y; D.QX[pout + ci + 1] = o.qx.y; D.QY[pout + ci + 1] = o.qy.y; }
     }
     if constexpr (!TAPE) {
-      if (v0) {
-        if (o.h.x > q.pk.x) { D.PK[ci] = o.h.x; if (D.tpk) D.tpk[ci] = (unsigned)(cl.step + 1); }
-        acc.smax = rmax(acc.smax, o.s.x);
-        acc.low = fminf(acc.low, o.low.x);
-        if (EX) acc.uns = acc.uns || !state_safe(A.P, o.s.x);
+      const bool up0 = v0 && o.h.x > pk.x, up1 = v1 && o.h.y > pk.y;
+      if (up0) D.PK[ci] = o.h.x;
+      if (up1) D.PK[ci + 1] = o.h.y;
+      if (D.tpk) {   // the state that raised the peak last
+        if (up0) D.tpk[ci] = (unsigned)(cl.step + 1);
+        if (up1) D.tpk[ci + 1] = (unsigned)(cl.step + 1);
       }
-      if (v1) {
-        if (o.h.y > q.pk.y) { D.PK[ci + 1] = o.h.y; if (D.tpk) D.tpk[ci + 1] = (unsigned)(cl.step + 1); }
-        acc.smax = rmax(acc.smax, o.s.y);
-        acc.low = fminf(acc.low, o.low.y);
-        if (EX) acc.uns = acc.uns || !state_safe(A.P, o.s.y);
-      }
+      acc.smax = fmaxf(acc.smax, fmaxf(o.s.x, o.s.y));
+      acc.low = fminf(acc.low, fminf(o.low.x, o.low.y));
       // row partials: f32 over the lane's pair, f64 across rows
-      acc.infil += (double)((v0 ? o.infil.x : 0.0f) + (v1 ? o.infil.y : 0.0f));
-      acc.fix += (double)((v0 ? o.fix.x : 0.0f) + (v1 ? o.fix.y : 0.0f));
+      acc.infil += (double)(o.infil.x + o.infil.y);
+      acc.fix += (double)(o.fix.x + o.fix.y);
       if (hits) acc.vol += (v0 ? (double)o.h.x : 0.0) + (v1 ? (double)o.h.y : 0.0);
       if (last_seg) {   // x_boundary: the east domain face inside this segment (kernel.rs:435-450)
-        if (c0 == nx - 1) { const double ve = (double)fE.m.x * dt_dy; if (ve > 0.0) acc.out += ve; else acc.in -= ve; }
-        if (c1 == nx - 1) { const double ve = (double)fE.m.y * dt_dy; if (ve > 0.0) acc.out += ve; else acc.in -= ve; }
+        if (c0 == nx - 1 || c0 == nx - 2) {
+          const double ve = (double)(c0 == nx - 1 ? fE.m.x : fE.m.y) * dt_dy;
+          if (ve > 0.0) acc.out += ve; else acc.in -= ve;
+        }
       }
       if (r == ny - 1) acc.ybot += (v0 ? (double)fS.m.x : 0.0) + (v1 ? (double)fS.m.y : 0.0);
-      if (rw_new && __any_sync(0xffffffffu, (v0 && o.h.x > 0.0f) || (v1 && o.h.y > 0.0f)) && lane == 0)
+      if (SKIP && __any_sync(0xffffffffu, (v0 && o.h.x > 0.0f) || (v1 && o.h.y > 0.0f)) && lane == 0)
         rw_new[r + 1] = 1u;   // the row holds water in the new state (every writer stores 1)
     }
     cur = nxt; fN = fS; fW = fWn;
   }
 }
 
-template <bool CREST, bool BND, bool TAPE = false>
-__global__ void __launch_bounds__(kBandWarps * 32, 3) k_band(const PlainArgs A) {
+// One step of every design: bands of rows x groups of segments x designs. fin: the last block of a
+// design to finish its band advances the design's integrator (plain_finalize_body), instead of a
+// launch of its own.
+template <bool CREST, bool BND, bool TAPE, bool SKIP>
+__global__ void __launch_bounds__(kBandWarps * 32, 3) k_band(const PlainArgs A, int fin) {
   __shared__ float4 edge_w[kBandWarps][kBandRows], edge_e[kBandWarps][kBandRows];
   __shared__ float wmax[kBandWarps];
   __shared__ unsigned wbad[kBandWarps];
   __shared__ double wsum[kBandWarps][kPart];
-  const int nblk = gridDim.x * gridDim.y;
-  const PlainDesign D = plain_design(A, blockIdx.z, nblk);
+  __shared__ unsigned s_last;
+  const int nblk = gridDim.x * gridDim.y, d = blockIdx.z;
+  const PlainDesign D = plain_design(A, d, nblk);
   const PlainCtl& cl = *D.ctl;
   if (cl.done) return;
   const StepK k = cl.k;
@@ -400,30 +408,47 @@ __global__ void __launch_bounds__(kBandWarps * 32, 3) k_band(const PlainArgs A) 
   const int r1 = r0 + R < A.ny ? r0 + R : A.ny;
   BandAcc t;
   if (s < (A.nx + 63) / 64) {
-    if (!k.exact) band_sweep<false, CREST, BND, TAPE>(A, D, cl, k, s, r0, r1, edge_w[wid], edge_e[wid], t);
-    else band_sweep<true, CREST, BND, TAPE>(A, D, cl, k, s, r0, r1, edge_w[wid], edge_e[wid], t);
+    if (!k.exact) band_sweep<false, CREST, BND, TAPE, SKIP>(A, D, cl, k, d, s, r0, r1, edge_w[wid], edge_e[wid], t);
+    else band_sweep<true, CREST, BND, TAPE, SKIP>(A, D, cl, k, d, s, r0, r1, edge_w[wid], edge_e[wid], t);
   }
   if constexpr (TAPE) return;
-  // ---- block reduction into the finalize's partials (fixed order) ----
-  const float m = warp_max_f(t.smax);
+  // ---- block reduction into the finalize's partials (fixed order). What only some blocks or steps
+  //      have (the edges' fluxes, the volume of a sync step) is summed only there. ----
+  const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(t.smax));
   const bool low = t.low < -k.h_dry || __float_as_uint(t.low) == 0xff800000u;
   const unsigned b = (__any_sync(0xffffffffu, low) ? 1u : 0u) | (__any_sync(0xffffffffu, t.uns) ? 2u : 0u);
+  const bool xedge = blockIdx.x == 0 || blockIdx.x == gridDim.x - 1, yedge = r0 == 0 || r1 == A.ny;
   double acc[kPart] = {t.infil, t.fix, t.in, t.out, t.vol, t.ytop, t.ybot};
 #pragma unroll
-  for (int j = 0; j < kPart; ++j) acc[j] = warp_sum_d(acc[j]);
+  for (int j = 0; j < kPart; ++j)
+    if (j < 2 || ((j == 2 || j == 3) && xedge) || (j == 4 && cl.pl.hits) || (j > 4 && yedge)) acc[j] = warp_sum_d(acc[j]);
   if (lane == 0) {
-    wmax[wid] = m; wbad[wid] = b;
+    wmax[wid] = __uint_as_float(m); wbad[wid] = b;
     for (int j = 0; j < kPart; ++j) wsum[wid][j] = acc[j];
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float mm = 0.0f; unsigned bb = 0u; double ss[kPart] = {0, 0, 0, 0, 0, 0, 0};
-    for (int w = 0; w < wpb; ++w) { mm = rmax(mm, wmax[w]); bb |= wbad[w]; for (int j = 0; j < kPart; ++j) ss[j] += wsum[w][j]; }
-    if (mm > 0.0f) atomicMax(&D.ctl->smax_bits, __float_as_uint(mm));
-    if (bb) atomicOr(&D.ctl->bad, bb);
-    double* pp = D.part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kPart;
-    for (int j = 0; j < kPart; ++j) pp[j] = ss[j];
+  if (wid == 0) {
+    if (lane == 0) {
+      float mm = 0.0f; unsigned bb = 0u;
+      for (int w = 0; w < wpb; ++w) { mm = fmaxf(mm, wmax[w]); bb |= wbad[w]; }
+      if (mm > 0.0f) atomicMax(&D.ctl->smax_bits, __float_as_uint(mm));
+      if (bb) atomicOr(&D.ctl->bad, bb);
+    }
+    if (lane < kPart) {
+      double ss = 0.0;
+      for (int w = 0; w < wpb; ++w) ss += wsum[w][lane];
+      D.part[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kPart + lane] = ss;
+    }
   }
+  if (!fin) return;
+  // the design's last block: its partials, maxima and row flags are in memory before the count
+  if (SKIP || wid == 0) __threadfence();   // (the threads that wrote them)
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicInc(A.arrive + d, (unsigned)nblk - 1u) == (unsigned)nblk - 1u ? 1u : 0u;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  plain_finalize_body<false>(A, d, nblk, 0);
 }
 
 }  // namespace itr

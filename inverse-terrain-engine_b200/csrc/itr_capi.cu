@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <chrono>
 #include <mutex>
+#include <type_traits>
 #include "../../include/itr_gpu.h"
 #include "itr_device.cuh"
 #include "itr_batched.cuh"
@@ -147,6 +148,7 @@ struct itr_ctx {
   DevBuf pH, pQX, pQY, pPK, ppart, pctl;
   // tiled batched path: state planes, tile partials, control blocks of all designs
   DevBuf tH, tQX, tQY, tpart, tctl;
+  DevBuf tArr;                  // row-band path: blocks done with a design's step
   DevBuf tRow, tGw, tSnapRow;   // row-band path: dry-row flags, ghost wetness, flags at the locked snapshot
   // adjoint: argmax states, (dt, rain) ring, checkpoints, tape, adjoint state, gradients
   DevBuf aTpk, aRing, aTape, aTape2, aLA, aLB, aGx, aGy, aGx2, aGy2, aSeg, aNst, aSeedC, aSeedS, aSeedW, aSeedN, aTmon;
@@ -594,7 +596,7 @@ void itr_gpu_destroy(itr_ctx* ctx) {
   for (DevBuf* b : {&ctx->wet, &ctx->gn2, &ctx->bc, &ctx->dzx, &ctx->dzy, &ctx->dzx2, &ctx->dzy2, &ctx->h0, &ctx->cut, &ctx->fill,
                     &ctx->mon, &ctx->obj_i, &ctx->obj_d, &ctx->peak, &ctx->depth, &ctx->ledger, &ctx->out, &ctx->mmax,
                     &ctx->pH, &ctx->pQX, &ctx->pQY, &ctx->pPK, &ctx->ppart, &ctx->pctl, &ctx->tH, &ctx->tQX, &ctx->tQY,
-                    &ctx->tpart, &ctx->tctl, &ctx->tRow, &ctx->tGw, &ctx->tSnapRow, &ctx->aTpk, &ctx->aRing, &ctx->aTape, &ctx->aTape2, &ctx->aLA, &ctx->aLB, &ctx->aGx, &ctx->aGy, &ctx->aGx2, &ctx->aGy2,
+                    &ctx->tpart, &ctx->tctl, &ctx->tArr, &ctx->tRow, &ctx->tGw, &ctx->tSnapRow, &ctx->aTpk, &ctx->aRing, &ctx->aTape, &ctx->aTape2, &ctx->aLA, &ctx->aLB, &ctx->aGx, &ctx->aGy, &ctx->aGx2, &ctx->aGy2,
                     &ctx->aSeg, &ctx->aNst, &ctx->aSeedC, &ctx->aSeedS, &ctx->aSeedW, &ctx->aSeedN, &ctx->aTmon,
                     &ctx->mDz, &ctx->mZe, &ctx->mAux, &ctx->mJp, &ctx->mJob, &ctx->mOut, &ctx->wsb, &ctx->rIn, &ctx->rOut,
                     &ctx->lDt, &ctx->lS4, &ctx->lSs, &ctx->lFb, &ctx->bG, &ctx->bJ, &ctx->bJ2, &ctx->bNever})
@@ -696,20 +698,19 @@ static void launch_update(const PlainArgs& A, dim3 grid, cudaStream_t st) {
   }
 }
 
-// One step's update of the tiled batched path: the row-band sweep (itr_band.cuh) over
-// (segment groups, bands, designs), or with option band = 0 the 16x16-tile kernel.
-static void launch_tiled_update(const itr_ctx* ctx, const PlainArgs& A, dim3 grid, cudaStream_t st) {
-  if (!ctx->band) { launch_update(A, grid, st); return; }
-  const bool bnd = A.bh != nullptr || A.P.inflow.n > 0;
+// One step of the tiled batched path: the row-band sweep (itr_band.cuh) over (segment groups, bands,
+// designs), which with `fin` also advances the integrators; or with option band = 0 the 16x16-tile
+// kernel's update alone. The dry-row instantiation only where a step can skip rows.
+template <bool TAPE>
+static void launch_band(const PlainArgs& A, dim3 grid, cudaStream_t st, int fin) {
+  const bool bnd = A.bh != nullptr || A.P.inflow.n > 0, skip = !TAPE && A.rowwet != nullptr;
   const BandGeom bg = band_geom(A.nx, A.ny, A.band_rows);
   const dim3 block((unsigned)(32 * bg.wpb));
-  if (A.mode == 1) {
-    if (bnd) k_band<true, true><<<grid, block, 0, st>>>(A);
-    else k_band<true, false><<<grid, block, 0, st>>>(A);
-  } else {
-    if (bnd) k_band<false, true><<<grid, block, 0, st>>>(A);
-    else k_band<false, false><<<grid, block, 0, st>>>(A);
-  }
+  auto go = [&](auto crest, auto b, auto s) { k_band<decltype(crest)::value, decltype(b)::value, TAPE, decltype(s)::value && !TAPE><<<grid, block, 0, st>>>(A, fin); };
+  using T = std::true_type;
+  using F = std::false_type;
+  if (A.mode == 1) { if (bnd) { if (skip) go(T(), T(), T()); else go(T(), T(), F()); } else { if (skip) go(T(), F(), T()); else go(T(), F(), F()); } }
+  else { if (bnd) { if (skip) go(F(), T(), T()); else go(F(), T(), F()); } else { if (skip) go(F(), F(), T()); else go(F(), F(), F()); } }
 }
 
 // Blocks per design of the tiled path's update (the finalize's partials).
@@ -720,8 +721,9 @@ static dim3 tiled_grid(const itr_ctx* ctx, int nx, int ny, int n) {
 }
 
 static int run_plain_design(itr_ctx* ctx, PlainArgs& A, int n_blocks, dim3 grid, int* launches) {
-  k_plain_init<<<1, 1024, 0, ctx->stream>>>(A);
-  k_plain_finalize<<<1, 32, 0, ctx->stream>>>(A, n_blocks, 1);
+  const int ib = plain_blocks(A.nx, A.ny, 1);
+  k_plain_init<<<dim3((unsigned)ib), 256, 0, ctx->stream>>>(A);
+  k_plain_finalize<<<1, kFinThreads, 0, ctx->stream>>>(A, ib, 1);
   *launches += 2;
   int done = 0;
   PlainCtl* hctl = ctx->hout.as<PlainCtl>();
@@ -766,20 +768,26 @@ static int run_tiled_batch(itr_ctx* ctx, PlainArgs& A, int n, dim3 tgrid, int* l
   // baseline-locked dt: the LOCKED finalize, each followed by the snapshot copy it may ask for
   const bool locked = A.locked_dt != nullptr;
   const dim3 cgrid(64, (unsigned)n);
-  k_plain_init<<<n, 1024, 0, st>>>(A);
+  const int ib = plain_blocks(A.nx, A.ny, n);
+  if (A.rowwet) CU(cudaMemsetAsync(A.rowwet, 0, (size_t)n * 2 * (A.ny + 2) * 4, st));
+  if (A.arrive) CU(cudaMemsetAsync(A.arrive, 0, (size_t)n * 4, st));
+  k_plain_init<<<dim3((unsigned)ib, (unsigned)n), 256, 0, st>>>(A);
   if (locked) {
-    k_plain_finalize_locked<<<n, 32, 0, st>>>(A, nb, 1);
+    k_plain_finalize_locked<<<n, kFinThreads, 0, st>>>(A, ib, 1);
     k_plain_locked_copy<<<cgrid, 256, 0, st>>>(A);
     *launches += 1;
   } else {
-    k_plain_finalize<<<n, 32, 0, st>>>(A, nb, 1);
+    k_plain_finalize<<<n, kFinThreads, 0, st>>>(A, ib, 1);
   }
   *launches += 2;
   const int K = tape ? tape->K : ctx->steps_per_submit;
   if (tape) { tape->dt.assign(n, std::vector<double>()); tape->blocks = 0; }
   auto block = [&]() {
     for (int s = 0; s < K; ++s) {
-      launch_tiled_update(ctx, A, grid, st);
+      const bool fin = ctx->band && !locked;   // the band kernel advances the integrators too
+      if (ctx->band) launch_band<false>(A, grid, st, fin ? 1 : 0);
+      else launch_update(A, grid, st);
+      if (fin) continue;
       if (locked) {
         k_plain_finalize_locked<<<n, kFinThreads, 0, st>>>(A, nb, 0);
         k_plain_locked_copy<<<cgrid, 256, 0, st>>>(A);
@@ -826,7 +834,7 @@ static int run_tiled_batch(itr_ctx* ctx, PlainArgs& A, int n, dim3 tgrid, int* l
     }
     if (ge) { const cudaError_t e = cudaGraphLaunch(ge, st); if (e != cudaSuccess) { rc = fail(ctx, ITR_DEVICE_ERROR, "cudaGraphLaunch: %s", cudaGetErrorString(e)); break; } }
     else block();
-    *launches += (locked ? 3 : 2) * K;
+    *launches += (locked ? 3 : ctx->band ? 1 : 2) * K;
     cudaError_t e = cudaMemcpyAsync(hc, A.ctl, (size_t)n * sizeof(PlainCtl), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) { rc = fail(ctx, ITR_DEVICE_ERROR, "tiled run: %s", cudaGetErrorString(e)); break; }
@@ -989,10 +997,11 @@ static int vjp_backward(itr_ctx* ctx, const PlainArgs& F, const itr_objective* o
   T.P = F.P; T.nx = nx; T.ny = ny; T.mode = F.mode; T.n_designs = n;
   T.wet = F.wet; T.gn2 = F.gn2; T.bc = F.bc; T.bh = F.bh;
   T.dzx = F.dzx; T.dzy = F.dzy; T.dzx2 = F.dzx2; T.dzy2 = F.dzy2;
+  T.G = F.G; T.J = F.J; T.J2 = F.J2;
   T.state_stride = 3 * N; T.plane_stride = S3;
   T.band_rows = band_rows_for(nx, ny, n, ctx->sm_count);
   const BandGeom tg = band_geom(nx, ny, T.band_rows);
-  const dim3 tgrid((unsigned)tg.gx, (unsigned)tg.gy, (unsigned)n), tblock((unsigned)(32 * tg.wpb));
+  const dim3 tgrid((unsigned)tg.gx, (unsigned)tg.gy, (unsigned)n);
   A.band_rows = adj_rows_for(nx, ny, n, ctx->sm_count);
   const AdjGeom ag = adj_geom(nx, ny, A.band_rows);
   const dim3 agrid((unsigned)ag.gx, (unsigned)ag.gy, (unsigned)n), ablock((unsigned)(32 * ag.wpb));
@@ -1013,13 +1022,7 @@ static int vjp_backward(itr_ctx* ctx, const PlainArgs& F, const itr_objective* o
         PlainArgs Tj = T;
         Tj.H = tapes[slot] + (size_t)j * S3; Tj.QX = Tj.H + N; Tj.QY = Tj.H + 2 * N;
         Tj.ctl = plan + (size_t)j * n;
-        if (crest) {
-          if (bnd) k_band<true, true, true><<<tgrid, tblock, 0, s2>>>(Tj);
-          else k_band<true, false, true><<<tgrid, tblock, 0, s2>>>(Tj);
-        } else {
-          if (bnd) k_band<false, true, true><<<tgrid, tblock, 0, s2>>>(Tj);
-          else k_band<false, false, true><<<tgrid, tblock, 0, s2>>>(Tj);
-        }
+        launch_band<true>(Tj, tgrid, s2, 0);
       }
       CU(cudaEventRecord(ctx->ev_rep[slot], s2));
       return ITR_OK;
@@ -1436,6 +1439,27 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
   int n_tiles = (int)(tgrid.x * tgrid.y);
   const int max_tiles = std::max((nx + kTile - 1) / kTile * ((ny + kTile - 1) / kTile), n_tiles);
   const bool bnd_grid = has_stage || P.inflow.n > 0;   // stage or inflow ghosts
+  auto pack_inputs = [&](PackArgs& K) -> cudaError_t {   // the cluster and row-band kernels' copy of the inputs
+    const size_t PJ = (size_t)pairs(nx) + 2, rec = (size_t)(ny + 1) * PJ;
+    cudaError_t e = ctx->bG.ensure(ny * PJ * 16);
+    if (e == cudaSuccess) e = ctx->bJ.ensure(n * rec * 16);
+    if (e == cudaSuccess && crest) e = ctx->bJ2.ensure(n * rec * 16);
+    if (e == cudaSuccess) e = ctx->bNever.ensure((size_t)n * 4);
+    if (e == cudaSuccess) e = cudaMemsetAsync(ctx->bNever.p, 0, (size_t)n * 4, ctx->stream);
+    memset(&K, 0, sizeof(K));
+    if (e != cudaSuccess) return e;
+    K.nx = nx; K.ny = ny; K.n = n;
+    K.wet = reinterpret_cast<const float*>(dv + o_wet); K.gn2 = reinterpret_cast<const float*>(dv + o_gn2);
+    K.dzx = reinterpret_cast<const float*>(dv + o_dzx); K.dzy = reinterpret_cast<const float*>(dv + o_dzy);
+    if (crest) { K.dzx2 = reinterpret_cast<const float*>(dv + o_dzx2); K.dzy2 = reinterpret_cast<const float*>(dv + o_dzy2); }
+    K.bc = reinterpret_cast<const uint8_t*>(dv + o_bc);
+    K.bh = has_stage ? reinterpret_cast<const float*>(dv + o_bh) : nullptr;
+    K.G = ctx->bG.as<float4>(); K.J = ctx->bJ.as<float4>(); K.J2 = crest ? ctx->bJ2.as<float4>() : nullptr;
+    K.never = ctx->bNever.as<unsigned>();
+    k_pack_inputs<<<dim3((unsigned)((rec + 255) / 256), (unsigned)n), 256, 0, ctx->stream>>>(K);
+    launches += 1;
+    return cudaGetLastError();
+  };
   auto tiled_args = [&](PlainArgs& A) -> cudaError_t {
     cudaError_t e = ctx->tH.ensure((size_t)n * 2 * N * 4);
     if (e == cudaSuccess) e = ctx->tQX.ensure((size_t)n * 2 * N * 4);
@@ -1481,7 +1505,14 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
       ctx->locked_run = true;
     }
     A.band_rows = band_rows_for(nx, ny, n, ctx->sm_count);
-    if (ctx->band && e == cudaSuccess) {   // dry-row skipping on the row-band path
+    if (ctx->band && e == cudaSuccess) {
+      PackArgs K;
+      e = pack_inputs(K);
+      A.G = K.G; A.J = K.J; A.J2 = K.J2;
+      if (e == cudaSuccess) e = ctx->tArr.ensure((size_t)n * 4);
+      A.arrive = ctx->tArr.as<unsigned>();
+    }
+    if (ctx->band && P.skip_dry && e == cudaSuccess) {   // dry-row skipping (the storm leaves a rain-free step)
       const size_t R = (size_t)ny + 2;
       e = ctx->tRow.ensure((size_t)n * 2 * R * 4);
       if (e == cudaSuccess && bnd_grid) e = ctx->tGw.ensure((size_t)n * R);
@@ -1516,27 +1547,11 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
     A.warm = warm_dev;
     // launch configuration
     LaunchCfg cfg;
-    auto pack = [&]() -> cudaError_t {   // the kernel's copy of the inputs
-      const size_t PJ = (size_t)pairs(nx) + 2, rec = (size_t)(ny + 1) * PJ;
-      cudaError_t e = ctx->bG.ensure(ny * PJ * 16);
-      if (e == cudaSuccess) e = ctx->bJ.ensure(n * rec * 16);
-      if (e == cudaSuccess && crest) e = ctx->bJ2.ensure(n * rec * 16);
-      if (e == cudaSuccess) e = ctx->bNever.ensure((size_t)n * 4);
-      if (e == cudaSuccess) e = cudaMemsetAsync(ctx->bNever.p, 0, (size_t)n * 4, ctx->stream);
-      if (e != cudaSuccess) return e;
+    auto pack = [&]() -> cudaError_t {
       PackArgs K;
-      memset(&K, 0, sizeof(K));
-      K.nx = nx; K.ny = ny; K.n = n;
-      K.wet = reinterpret_cast<const float*>(dv + o_wet); K.gn2 = reinterpret_cast<const float*>(dv + o_gn2);
-      K.dzx = reinterpret_cast<const float*>(dv + o_dzx); K.dzy = reinterpret_cast<const float*>(dv + o_dzy);
-      if (crest) { K.dzx2 = reinterpret_cast<const float*>(dv + o_dzx2); K.dzy2 = reinterpret_cast<const float*>(dv + o_dzy2); }
-      K.bc = A.bc; K.bh = A.bh;
-      K.G = ctx->bG.as<float4>(); K.J = ctx->bJ.as<float4>(); K.J2 = crest ? ctx->bJ2.as<float4>() : nullptr;
-      K.never = ctx->bNever.as<unsigned>();
-      k_pack_inputs<<<dim3((unsigned)((rec + 255) / 256), (unsigned)n), 256, 0, ctx->stream>>>(K);
-      launches += 1;
+      const cudaError_t e = pack_inputs(K);
       A.G = K.G; A.J = K.J; A.J2 = K.J2; A.never = K.never;
-      return cudaGetLastError();
+      return e;
     };
     auto key = std::make_tuple(nx, ny, n, (int)g->mode + (bnd ? 2 : 0));
     if (ctx->cluster > 0 || ctx->threads > 0) {
@@ -1595,7 +1610,6 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
     }
   }
   if (tiled) {
-    const int nb = n_tiles;
     PlainArgs A;
     CU(tiled_args(A));
     if (ctx->vjp) {
@@ -1611,7 +1625,7 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
     rc = run_tiled_batch(ctx, A, n, tgrid, &launches);
     ctx->last_band = ctx->band;
     if (rc != ITR_OK) return rc;
-    k_plain_outputs<<<n, 256, 0, ctx->stream>>>(A, nb, ctx->out.as<DesignOut>(), ctx->depth.as<float>());
+    k_plain_outputs<<<dim3((unsigned)plain_blocks(nx, ny, n), (unsigned)n), 256, 0, ctx->stream>>>(A, ctx->out.as<DesignOut>(), ctx->depth.as<float>());
     launches += 1;
     CU(cudaEventRecord(ctx->ev[2], ctx->stream));
     ctx->last_tiled = A;

@@ -248,47 +248,6 @@ ITR_DEV double rain_integral(const Rain& R, double a, double b) {
   return total;
 }
 
-// The same rate and integral, for sorted breakpoints, with a cursor that only moves
-// forward (simulated time is monotone): identical arithmetic on identical operands, so
-// identical bits, without rescanning the table every step.
-struct RainCursor {
-  int seg;   // first k with t[k+1] >= last query (rate) ...
-  int brk;   // first breakpoint index with t[k] > last lower limit
-};
-
-ITR_DEV double rain_rate_c(const Rain& R, double x, int& seg) {
-  if (R.n == 0) return 0.0;
-  if (x <= R.t[0]) return R.r[0];
-  while (seg + 1 < R.n && R.t[seg + 1] < x) ++seg;
-  if (seg + 1 < R.n) {
-    double t0 = R.t[seg], r0 = R.r[seg], t1 = R.t[seg + 1], r1 = R.r[seg + 1];
-    if (t1 == t0) return r1;
-    return r0 + (r1 - r0) * (x - t0) / (t1 - t0);
-  }
-  return R.r[R.n - 1];
-}
-
-ITR_DEV double rain_integral_c(const Rain& R, double a, double b, RainCursor& cu) {
-  if (b <= a) return 0.0;
-  if (R.n == 0) return 0.0;
-  int seg = cu.seg;
-  double total = 0.0, tt = a, rr = rain_rate_c(R, a, seg);
-  cu.seg = seg;
-  while (cu.brk < R.n && !(R.t[cu.brk] > a)) ++cu.brk;
-  for (int k = cu.brk; k < R.n && R.t[k] < b; ++k) {
-    double tk = R.t[k];
-    int s2 = seg;
-    double rk = rain_rate_c(R, tk, s2);
-    total += 0.5 * (rr + rk) * (tk - tt);
-    tt = tk;
-    rr = rk;
-    seg = s2;
-  }
-  double rb = rain_rate_c(R, b, seg);
-  total += 0.5 * (rr + rb) * (b - tt);
-  return total;
-}
-
 // Inflow boundaries (Ghost::Inflow, boundary.rs:26-31,45-50,66-71). The inflow cells of a
 // grid fall into groups, one per distinct (hydrograph, 1 / segment length) pair; a group's
 // discharge per unit width q = rate(t) * inv_len * inflow_scale and its critical depth
@@ -427,31 +386,8 @@ struct StepPlan {
   bool hits;
 };
 
-ITR_DEV StepPlan plan_step(const RunParams& P, double t, uint32_t sync_index, double dt_cfl) {
-  StepPlan s;
-  double t_sync = dmin_num((double)(sync_index + 1) * P.sync, P.duration);
-  double dt = dmin_num(dt_cfl, P.dt_max);
-  s.hits = t + dt >= t_sync - 1e-9 * P.sync;
-  if (s.hits) dt = t_sync - t;
-  s.rain = rain_integral(P.rain, t, t + dt);
-  s.t_new = s.hits ? t_sync : t + dt;
-  s.dt = dt;
-  return s;
-}
-
-ITR_DEV StepPlan plan_step_c(const RunParams& P, double t, uint32_t sync_index, double dt_cfl, RainCursor& cu) {
-  StepPlan s;
-  double t_sync = dmin_num((double)(sync_index + 1) * P.sync, P.duration);
-  double dt = dmin_num(dt_cfl, P.dt_max);
-  s.hits = t + dt >= t_sync - 1e-9 * P.sync;
-  if (s.hits) dt = t_sync - t;
-  s.rain = P.rain_sorted ? rain_integral_c(P.rain, t, t + dt, cu) : rain_integral(P.rain, t, t + dt);
-  s.t_new = s.hits ? t_sync : t + dt;
-  s.dt = dt;
-  return s;
-}
-
-// The same schedule split for a kernel that overlaps it with work that needs no dt. The rate at the
+// The step's schedule (solver.rs:449-489) as straight-line arithmetic. dt_pick: the dt before the clip to
+// the sync instant t_sync (t_hit: the start from which a step is clipped). The rate at the
 // step's start is known from the step before; while no breakpoint lies inside the step the integral is
 // one trapezoid of the piece `seg`, else (or for an unsorted storm) `rare` is set and the general
 // integral replaces s.rain.
@@ -465,31 +401,6 @@ ITR_DEV StepPlan plan_step_fast(const RunParams& P, double t, double t_sync, dou
   s.rain = 0.5 * (rate_t + rain_piece(P.rain.seg[seg], b)) * (b - t);
   rare = b > P.rain.seg[seg].end || !P.rain_sorted;
   s.t_new = s.hits ? t_sync : b;
-  return s;
-}
-
-// plan_step for a step whose dt before the sync clip is given (the baseline-locked dt).
-ITR_DEV StepPlan plan_step_dt(const RunParams& P, double t, uint32_t sync_index, double dt) {
-  StepPlan s;
-  double t_sync = dmin_num((double)(sync_index + 1) * P.sync, P.duration);
-  s.hits = t + dt >= t_sync - 1e-9 * P.sync;
-  if (s.hits) dt = t_sync - t;
-  s.rain = rain_integral(P.rain, t, t + dt);
-  s.t_new = s.hits ? t_sync : t + dt;
-  s.dt = dt;
-  return s;
-}
-
-// plan_step_c for a step whose dt before the sync clip is given: the baseline-locked dt
-// (solver.rs:452-456 sets dt from the schedule, then :484-487 clip it to the sync instant).
-ITR_DEV StepPlan plan_step_dt_c(const RunParams& P, double t, uint32_t sync_index, double dt, RainCursor& cu) {
-  StepPlan s;
-  double t_sync = dmin_num((double)(sync_index + 1) * P.sync, P.duration);
-  s.hits = t + dt >= t_sync - 1e-9 * P.sync;
-  if (s.hits) dt = t_sync - t;
-  s.rain = P.rain_sorted ? rain_integral_c(P.rain, t, t + dt, cu) : rain_integral(P.rain, t, t + dt);
-  s.t_new = s.hits ? t_sync : t + dt;
-  s.dt = dt;
   return s;
 }
 

@@ -55,6 +55,7 @@ struct PlainCtl {
   int locked_live;
   int copy_req;
   unsigned long long rows_skipped;   // dry rows skipped so far (kernel.rs:605-612)
+  int seg;           // the storm's piece at t (RainSeg)
   unsigned unsafe;   // bit 0: the state is not known to be bounded, bit 1: never will be (StepK::exact)
 };
 
@@ -82,6 +83,7 @@ struct PlainArgs {
   float* QY;
   float* PK;          // per design nx*ny
   double* part;       // per design, per tile: [kPart]
+  unsigned* arrive;   // per design: blocks of the step's update that are done (k_band's last block finalizes)
   PlainCtl* ctl;      // per design
   double* ledger;     // per design max_rows*8
   int max_rows;
@@ -112,6 +114,10 @@ struct PlainArgs {
   // stride 3 N, and plane 1 = the next step's slot.
   size_t state_stride;
   size_t plane_stride;
+  // row-band kernel: packed inputs (BatchArgs::G, J, J2)
+  const float4* G;
+  const float4* J;
+  const float4* J2;
 };
 
 // Padded row j is dry for the step about to run: no water in its state nor in its stage or
@@ -295,30 +301,73 @@ __global__ void __launch_bounds__(kTileThreads, 6) k_plain_update(const PlainArg
 
 // Threads per design of the step finalize (any multiple of 32 up to 1024 works).
 constexpr int kFinThreads = 256;
+static_assert(sizeof(PlainCtl) % 8 == 0, "the finalize copies the control block by 8-byte words");
 
-// Advance the integrator after a step (or plan the first step when `first`). Launched with
-// a block of warps per design: all of them sum the tile partials (one warp alone waits on
-// hundreds of dependent rounds of loads for a large grid), warp 0 does the rest.
+// Advance the integrator of design d after a step (or plan the first step when `first`), by one whole
+// block: its warps sum the partials (one component a warp, in block order per lane, then a
+// butterfly), warp 0 does the rest. It works on a copy of the control block in shared memory: the
+// chain of f64 operations then waits on no load from memory. What bounds it is that chain (the
+// block is alone on its design), so its divisions are the multiplications of div_rn.
 // LOCKED: the baseline-locked dt (solver.rs:436-483): each step takes the schedule's dt while
 // dt * smax of the current state stays within cfl_hard; at the first step where it would not
 // (or the schedule has run out) the control block goes back to the last sync snapshot, which
 // the next k_plain_locked_copy completes with the state planes, and the run continues with the
 // adaptive dt. Snapshots: at the start and after every sync's abort tests.
 template <bool LOCKED>
-ITR_DEV void plain_finalize_body(const PlainArgs& A, int n_blocks, int first) {
-  __shared__ double red[32][kPart];
-  const PlainDesign D = plain_design(A, blockIdx.x, n_blocks);
-  PlainCtl& c = *D.ctl;
+ITR_DEV void plain_finalize_steps(const PlainArgs& A, const PlainDesign& D, int d, int first, PlainCtl& c, const double* sums);
+
+template <bool LOCKED>
+ITR_DEV void plain_finalize_body(const PlainArgs& A, int d, int n_blocks, int first) {
+  __shared__ PlainCtl c;
+  __shared__ double sums[kPart];
+  __shared__ unsigned s_skip;
+  const PlainDesign D = plain_design(A, d, n_blocks);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const RunParams& P = A.P;
-  if constexpr (LOCKED) { if (threadIdx.x == 0) c.copy_req = 0; }   // the last request has been served
-  if (c.done) return;
+  constexpr int kWords = sizeof(PlainCtl) / 8;
+  const volatile unsigned long long* src = reinterpret_cast<const volatile unsigned long long*>(D.ctl);
+  for (int i = threadIdx.x; i < kWords; i += blockDim.x) reinterpret_cast<unsigned long long*>(&c)[i] = first ? 0ull : src[i];
+  if (threadIdx.x == 0) s_skip = 0u;
+  for (int j = wid; j < kPart; j += nw) {
+    const bool is_max = first && j > 0;   // (the start's partials: volume, then maxima)
+    double t = 0.0;
+    for (int b = lane; b < n_blocks; b += 32) {
+      const double v = first && j > 3 ? 0.0 : __ldcg(D.part + (size_t)b * kPart + j);
+      t = is_max ? (t > v ? t : v) : t + v;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double v = __shfl_xor_sync(0xffffffffu, t, o);
+      t = is_max ? (t > v ? t : v) : t + v;
+    }
+    if (lane == 0) sums[j] = t;
+  }
+  __syncthreads();
+  if (first && threadIdx.x == 0) {
+    const WarmStart* W = (A.warm && A.warm[d].state) ? &A.warm[d] : nullptr;
+    if (W) {
+      c.t = W->t; c.dt_cfl = W->dt_cfl; c.acc_rain = W->acc_rain; c.v0 = W->v0; c.volume = W->volume; c.rel_res = W->rel_res;
+      c.tot_infil = W->tot_infil; c.tot_fix = W->tot_fix; c.tot_in = W->tot_in; c.tot_out = W->tot_out;
+      c.step = W->step; c.sync_index = W->sync_index; c.n_rows = W->n_rows;
+      c.unsafe = P.cfl <= 0.99 * (double)P.s_safe * W->dt_cfl ? 0u : 1u;   // dt_cfl = cfl / largest wave rate
+    } else {
+      c.v0 = sums[0] * P.area; c.volume = c.v0;
+      c.dt_cfl = sums[1] > 0.0 ? dmin_num(P.cfl / sums[1], P.dt_max) : P.dt_max;
+      c.s_cur = sums[1];
+      c.unsafe = sums[2] > 0.0 ? 1u : 0u;
+    }
+    if (sums[3] > 0.0) c.unsafe |= 2u;
+  }
+  __syncthreads();
+  const bool was_done = c.done != 0;
+  __syncthreads();   // read by every warp before warp 0 goes on to change it
+  if (was_done) {
+    if constexpr (LOCKED) { if (threadIdx.x == 0) D.ctl->copy_req = 0; }   // the last request has been served
+    return;
+  }
   if (!first && D.rowwet) {
     // dry rows the step just skipped (k_band's predicate on the flags it read: the state of
     // parity c.par, not yet flipped), then clear those flags: the next step writes them
-    __shared__ unsigned s_skip;
-    if (threadIdx.x == 0) s_skip = 0u;
-    __syncthreads();
     const int R = A.ny + 2;
     unsigned* rw = D.rowwet + (size_t)c.par * R;
     if (P.skip_dry && !(c.k.rain > 0.0f)) {
@@ -331,23 +380,34 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int n_blocks, int first) {
     for (int j = threadIdx.x; j < R; j += blockDim.x) rw[j] = 0u;
     if (threadIdx.x == 0) c.rows_skipped += s_skip;
   }
-  double tot[kPart] = {0, 0, 0, 0, 0, 0, 0};
-  if (!first) {
-    for (int b = threadIdx.x; b < n_blocks; b += blockDim.x)
-      for (int j = 0; j < kPart; ++j) tot[j] += D.part[(size_t)b * kPart + j];
-    for (int j = 0; j < kPart; ++j)
-      for (int o = 16; o > 0; o >>= 1) tot[j] += __shfl_xor_sync(0xffffffffu, tot[j], o);
-    if (nw > 1) {
-      if (lane == 0)
-        for (int j = 0; j < kPart; ++j) red[wid][j] = tot[j];
-      __syncthreads();
-      for (int j = 0; j < kPart; ++j) {
-        tot[j] = lane < nw ? red[lane][j] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) tot[j] += __shfl_xor_sync(0xffffffffu, tot[j], o);
-      }
-    }
+  if (wid == 0) {
+    if constexpr (LOCKED) { if (lane == 0) c.copy_req = 0; __syncwarp(); }
+    plain_finalize_steps<LOCKED>(A, D, d, first, c, sums);
   }
-  if (wid != 0) return;
+  __syncthreads();
+  unsigned long long* dst = reinterpret_cast<unsigned long long*>(D.ctl);
+  for (int i = threadIdx.x; i < kWords; i += blockDim.x) dst[i] = reinterpret_cast<const unsigned long long*>(&c)[i];
+}
+
+// The dt before the sync clip, the step's plan and its constants, from the integrator in c (lane 0).
+ITR_DEV void plain_plan(const PlainArgs& A, PlainCtl& c, double dt_pick) {
+  const RunParams& P = A.P;
+  const double t_sync = dmin_num((double)(c.sync_index + 1) * P.sync, P.duration);
+  while (P.rain_sorted && c.t > P.rain.seg[c.seg].end) ++c.seg;
+  bool rare;
+  c.pl = plan_step_fast(P, c.t, t_sync, t_sync - 1e-9 * P.sync, dt_pick, rain_piece(P.rain.seg[c.seg], c.t), c.seg, rare);
+  if (rare) c.pl.rain = rain_integral(P.rain, c.t, c.t + c.pl.dt);
+  c.k = step_consts(P, c.pl.dt, c.pl.rain);
+  c.k.exact = c.unsafe ? 1u : 0u;
+}
+
+template <bool LOCKED>
+ITR_DEV void plain_finalize_steps(const PlainArgs& A, const PlainDesign& D, int d, int first, PlainCtl& c, const double* sums) {
+  const int lane = threadIdx.x & 31;
+  const RunParams& P = A.P;
+  double tot[kPart] = {0, 0, 0, 0, 0, 0, 0};
+  if (!first)
+    for (int j = 0; j < kPart; ++j) tot[j] = sums[j];
   if (!first) {
     {   // y_boundary (kernel.rs:452-472): the top edge is inflow when its net flux is > 0,
         // the bottom edge outflow
@@ -358,6 +418,7 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int n_blocks, int first) {
     }
     const double smax = (double)__uint_as_float(c.smax_bits);
     const unsigned badv = c.bad;
+    const bool hits = c.pl.hits;   // (read by every lane here: lane 0 may replace c below)
     __syncwarp();
     if (lane == 0) {
       c.tot_infil += tot[0]; c.tot_fix += tot[1]; c.tot_in += tot[2]; c.tot_out += tot[3];
@@ -371,10 +432,10 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int n_blocks, int first) {
     }
     __syncwarp();
     if (badv & 1u) { if (lane == 0) { c.status = 3; c.done = 1; } return; }
-    if (lane == 0) c.dt_cfl = smax > 0.0 ? P.cfl / smax : P.dt_max;
+    if (lane == 0) c.dt_cfl = smax > 0.0 ? (c.unsafe ? P.cfl / smax : div_by_f32(P.cfl, smax)) : P.dt_max;
     if constexpr (LOCKED) { if (lane == 0) c.s_cur = smax; }
     __syncwarp();
-    if (c.pl.hits) {
+    if (hits) {
       int decision = 0;
       if (lane == 0) {
         c.sync_index += 1;
@@ -394,7 +455,7 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int n_blocks, int first) {
             double best = 0.0; int bk = -1;
             for (int g = 0; g < ob.n_guard; ++g) {
               int mp = ob.guard_pos[g];
-              double w = (double)D.PK[A.mon_cells[mp]] - ob.baseline[mp] - ob.tol;
+              double w = (double)__ldcg(D.PK + A.mon_cells[mp]) - ob.baseline[mp] - ob.tol;
               if (w > 0.0 && (bk < 0 || w > best)) { best = w; bk = g; }
             }
             if (bk >= 0) {
@@ -407,7 +468,7 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int n_blocks, int first) {
             for (int a = 0; a < ob.n_assets; ++a) {
               double pk = 0.0;
               for (int m = ob.asset_off[a]; m < ob.asset_off[a + 1]; ++m) {
-                double x = (double)D.PK[A.mon_cells[ob.asset_pos[m]]];
+                double x = (double)__ldcg(D.PK + A.mon_cells[ob.asset_pos[m]]);
                 pk = pk > x ? pk : x;
               }
               jr += ob.asset_w[a] * ob.tau * itr_math::softplus((pk - ob.asset_thr[a]) / ob.tau);
@@ -421,7 +482,7 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int n_blocks, int first) {
       __syncwarp();
       if (c.done) return;
       if constexpr (LOCKED) {   // sync snapshot (solver.rs:611-614)
-        if (lane == 0 && c.locked_live) { A.snapctl[blockIdx.x] = c; c.copy_req = 1; }
+        if (lane == 0 && c.locked_live) { A.snapctl[d] = c; c.copy_req = 1; }
         __syncwarp();
       }
     }
@@ -430,8 +491,8 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int n_blocks, int first) {
     if (lane == 0) {
       if (first) {   // the snapshot at the start (solver.rs:444-447)
         c.locked_live = 1;
-        A.fallback_t[blockIdx.x] = -1.0;
-        A.snapctl[blockIdx.x] = c;
+        A.fallback_t[d] = -1.0;
+        A.snapctl[d] = c;
         c.copy_req = 1;
       }
       if (!(c.t < P.duration && c.sync_index < P.n_sync)) {
@@ -442,10 +503,10 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int n_blocks, int first) {
         // back to the last sync snapshot, adaptive from here on. A snapshot taken by this very
         // finalize (save still pending) is the current state: nothing to copy back.
         const int pending_save = c.copy_req;
-        c = A.snapctl[blockIdx.x];
+        c = A.snapctl[d];
         c.locked_live = 0;
         c.copy_req = pending_save == 1 ? 0 : 2;
-        A.fallback_t[blockIdx.x] = c.t;
+        A.fallback_t[d] = c.t;
       }
     }
     __syncwarp();
@@ -454,10 +515,7 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int n_blocks, int first) {
     __syncwarp();
     if (D.gwet) plain_ghost_wet(A, D.bh, c.inf, D.gwet, lane);
     if (lane == 0) {
-      const double dt = c.locked_live ? A.locked_dt[c.step] : dmin_num(c.dt_cfl, P.dt_max);
-      c.pl = plan_step_dt(P, c.t, c.sync_index, dt);
-      c.k = step_consts(P, c.pl.dt, c.pl.rain);
-      c.k.exact = c.unsafe ? 1u : 0u;
+      plain_plan(A, c, c.locked_live ? A.locked_dt[c.step] : dmin_num(c.dt_cfl, P.dt_max));
     }
     return;
   }
@@ -469,9 +527,7 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int n_blocks, int first) {
   if (lane == 0) {
     if (!(c.t < P.duration && c.sync_index < P.n_sync)) { c.done = 1; return; }
     if (c.step >= A.max_steps) { c.status = 4; c.done = 1; return; }
-    c.pl = plan_step(P, c.t, c.sync_index, c.dt_cfl);
-    c.k = step_consts(P, c.pl.dt, c.pl.rain);
-    c.k.exact = c.unsafe ? 1u : 0u;
+    plain_plan(A, c, dmin_num(c.dt_cfl, P.dt_max));
     if (D.dt_log) {   // ring of max_log entries, slot step mod max_log
       double* q = D.dt_log + (size_t)(c.step % (unsigned long long)A.max_log) * kLog;
       q[0] = c.pl.dt; q[1] = c.pl.rain; q[2] = c.t; q[3] = (double)c.k.exact;
@@ -479,9 +535,9 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int n_blocks, int first) {
   }
 }
 
-__global__ void k_plain_finalize(const PlainArgs A, int n_blocks, int first) { plain_finalize_body<false>(A, n_blocks, first); }
+__global__ void k_plain_finalize(const PlainArgs A, int n_blocks, int first) { plain_finalize_body<false>(A, blockIdx.x, n_blocks, first); }
 __global__ void k_plain_finalize_locked(const PlainArgs A, int n_blocks, int first) {
-  plain_finalize_body<true>(A, n_blocks, first);
+  plain_finalize_body<true>(A, blockIdx.x, n_blocks, first);
 }
 
 // Baseline-locked dt: after a finalize that asked for it, copy each design's current state
@@ -515,77 +571,68 @@ __global__ void k_plain_locked_copy(const PlainArgs A) {
   }
 }
 
-// Initial state and the first dt (solver.rs:381-390), or a warm start's checkpoint.
+// Initial state (solver.rs:381-390), or a warm start's checkpoint: blocks x designs, each block a share of
+// the cells. The blocks' volumes, wave rates and flags go to the partials, from which the first
+// finalize makes the control block. Row flags are zeroed before the launch.
 __global__ void k_plain_init(const PlainArgs A) {
-  const PlainDesign D = plain_design(A, blockIdx.x, 0);
-  const int nx = A.nx, ny = A.ny, n = nx * ny;
+  const int d = blockIdx.y;
+  const PlainDesign D = plain_design(A, d, gridDim.x);
+  const int nx = A.nx, ny = A.ny;
+  const size_t n = (size_t)nx * ny, stride = (size_t)gridDim.x * blockDim.x, first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const RunParams& P = A.P;
-  const WarmStart* W = (A.warm && A.warm[blockIdx.x].state) ? &A.warm[blockIdx.x] : nullptr;
-  // dry-row flags of the initial state (init_state: a row is dry when all its depths are 0)
-  if (D.rowwet) {
-    for (int j = threadIdx.x; j < 2 * (ny + 2); j += blockDim.x) D.rowwet[j] = 0u;
-    __syncthreads();
-  }
+  const WarmStart* W = (A.warm && A.warm[d].state) ? &A.warm[d] : nullptr;
   // a crest jump or stage depth out of the branch-free step's bounds keeps the run on the scalar path
-  bool neg = false;
+  bool neg = false, uns = false;
   if (A.mode == 1) {
-    for (size_t i = threadIdx.x; i < (size_t)ny * (nx + 1); i += blockDim.x) neg = neg || !jump_safe(D.dzx[i]) || !jump_safe(D.dzx2[i]);
-    for (size_t i = threadIdx.x; i < (size_t)(ny + 1) * nx; i += blockDim.x) neg = neg || !jump_safe(D.dzy[i]) || !jump_safe(D.dzy2[i]);
+    for (size_t i = first; i < (size_t)ny * (nx + 1); i += stride) neg = neg || !jump_safe(D.dzx[i]) || !jump_safe(D.dzx2[i]);
+    for (size_t i = first; i < (size_t)(ny + 1) * nx; i += stride) neg = neg || !jump_safe(D.dzy[i]) || !jump_safe(D.dzy2[i]);
   }
   if (D.bh)
-    for (int i = threadIdx.x; i < 2 * (nx + ny); i += blockDim.x) neg = neg || !stage_safe(A.bc[i], D.bh[i]);
-  const unsigned never = __syncthreads_or(neg ? 1 : 0) ? 2u : 0u;
-  if (W) {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      D.H[i] = W->state[i]; D.QX[i] = W->state[n + i]; D.QY[i] = W->state[2 * n + i]; D.PK[i] = W->state[3 * n + i];
-      if (D.tpk) D.tpk[i] = 0u;
-      if (D.rowwet && W->state[i] != 0.0f) D.rowwet[1 + i / nx] = 1u;
+    for (size_t i = first; i < 2 * (size_t)(nx + ny); i += stride) neg = neg || !stage_safe(A.bc[i], D.bh[i]);
+  double s0 = 0.0, v0 = 0.0;
+  for (size_t i = first; i < n; i += stride) {
+    float h;
+    if (W) {
+      h = W->state[i];
+      D.QX[i] = W->state[n + i]; D.QY[i] = W->state[2 * n + i]; D.PK[i] = W->state[3 * n + i];
+    } else {
+      h = D.h0[i];
+      D.QX[i] = 0.0f; D.QY[i] = 0.0f; D.PK[i] = 0.0f;
+      uns = uns || !depth_safe(P, h);
+      const double hd = (double)h;
+      v0 += hd;
+      if (hd > P.h_dry) {
+        const double cd = sqrt(P.g * hd);
+        const double r = (0.0 / hd + cd) / P.dx + (0.0 / hd + cd) / P.dy;
+        s0 = s0 > r ? s0 : r;
+      }
     }
-    if (threadIdx.x == 0) {
-      PlainCtl c;
-      memset(&c, 0, sizeof(c));
-      c.t = W->t; c.dt_cfl = W->dt_cfl; c.acc_rain = W->acc_rain; c.v0 = W->v0; c.volume = W->volume; c.rel_res = W->rel_res;
-      c.tot_infil = W->tot_infil; c.tot_fix = W->tot_fix; c.tot_in = W->tot_in; c.tot_out = W->tot_out;
-      c.step = W->step; c.sync_index = W->sync_index; c.n_rows = W->n_rows;
-      c.unsafe = never | (P.cfl <= 0.99 * (double)P.s_safe * W->dt_cfl ? 0u : 1u);   // dt_cfl = cfl / largest wave rate
-      *D.ctl = c;
-    }
-    return;
+    D.H[i] = h;
+    if (D.tpk) D.tpk[i] = 0u;
+    if (D.rowwet && h != 0.0f) D.rowwet[1 + i / nx] = 1u;   // (init_state: a row is dry when all its depths are 0)
   }
   __shared__ double ss[32], sv[32];
-  double s0 = 0.0, v0 = 0.0;
-  bool uns = false;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    float h = D.h0[i];
-    D.H[i] = h; D.QX[i] = 0.0f; D.QY[i] = 0.0f; D.PK[i] = 0.0f;
-    if (D.tpk) D.tpk[i] = 0u;
-    if (D.rowwet && h != 0.0f) D.rowwet[1 + i / nx] = 1u;
-    uns = uns || !depth_safe(P, h);
-    double hd = (double)h;
-    v0 += hd;
-    if (hd > P.h_dry) {
-      double cd = sqrt(P.g * hd);
-      double r = (0.0 / hd + cd) / P.dx + (0.0 / hd + cd) / P.dy;
-      s0 = s0 > r ? s0 : r;
-    }
-  }
   for (int o = 16; o > 0; o >>= 1) {
-    double a = __shfl_xor_sync(0xffffffffu, s0, o); s0 = s0 > a ? s0 : a;
+    const double a = __shfl_xor_sync(0xffffffffu, s0, o); s0 = s0 > a ? s0 : a;
     v0 += __shfl_xor_sync(0xffffffffu, v0, o);
   }
   if ((threadIdx.x & 31) == 0) { ss[threadIdx.x >> 5] = s0; sv[threadIdx.x >> 5] = v0; }
-  const unsigned unsafe = never | (__syncthreads_or(uns ? 1 : 0) ? 1u : 0u);
+  const bool any_neg = __syncthreads_or(neg ? 1 : 0) != 0, any_uns = __syncthreads_or(uns ? 1 : 0) != 0;
   if (threadIdx.x == 0) {
     double s = 0.0, v = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { s = s > ss[w] ? s : ss[w]; v += sv[w]; }
-    PlainCtl c;
-    memset(&c, 0, sizeof(c));
-    c.v0 = v * P.area; c.volume = c.v0;
-    c.dt_cfl = s > 0.0 ? dmin_num(P.cfl / s, P.dt_max) : P.dt_max;
-    c.s_cur = s;
-    c.unsafe = unsafe;
-    *D.ctl = c;
+    double* o = D.part + (size_t)blockIdx.x * kPart;
+    o[0] = v; o[1] = s; o[2] = any_uns ? 1.0 : 0.0; o[3] = any_neg ? 1.0 : 0.0;
   }
+}
+
+// Blocks per design of k_plain_init and k_plain_outputs, both bound by memory (one block of one SM cannot
+// draw more than about 1/148 of its rate): one per 1024 cells, enough to fill the device, and never
+// more than the partials have room for.
+inline int plain_blocks(int nx, int ny, int n_designs) {
+  const long long cells = (long long)nx * ny, want = (cells + 1023) / 1024, share = (2048 + n_designs - 1) / n_designs;
+  const long long b = want < share ? want : share;
+  return (int)(b < 1 ? 1 : b);
 }
 
 // Baseline record (one design): the current state plane and running peaks into dst [4][N].
@@ -615,20 +662,21 @@ __global__ void k_rec_rows(const PlainArgs A, const float* state, uint8_t* wet) 
 
 // Per-design results of a tiled batched run: the scalar outcome from the control block and
 // the final depth (the plane the last step wrote).
-__global__ void k_plain_outputs(const PlainArgs A, int n_tiles, DesignOut* out, float* depth) {
-  const PlainDesign D = plain_design(A, blockIdx.x, n_tiles);
+__global__ void k_plain_outputs(const PlainArgs A, DesignOut* out, float* depth) {
+  const int d = blockIdx.y;
+  const PlainDesign D = plain_design(A, d, 0);
   const PlainCtl& c = *D.ctl;
   const size_t N = (size_t)A.nx * A.ny;
   const float* H = D.H + (size_t)c.par * N;
-  for (size_t i = threadIdx.x; i < N; i += blockDim.x) depth[blockIdx.x * N + i] = H[i];
-  if (threadIdx.x == 0) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (size_t)gridDim.x * blockDim.x) depth[d * N + i] = H[i];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     DesignOut o;
     memset(&o, 0, sizeof(o));
     o.steps = c.step; o.t_end = c.t; o.sync_count = c.sync_index; o.status = c.status;
     o.breach_cell = c.breach_cell; o.breach_sync = c.breach_sync; o.violation = c.violation;
     o.lower_bound = c.lower_bound; o.v0 = c.v0; o.volume = c.volume; o.rel_residual = c.rel_res; o.n_rows = c.n_rows;
     o.rows_skipped = c.rows_skipped;
-    out[blockIdx.x] = o;
+    out[d] = o;
   }
 }
 

@@ -253,8 +253,9 @@ extern "C" int itr_gpu_run_plain_static(int device, const itr_params* p, const i
   A.ledger = max_rows > 0 ? ledger : nullptr;
   A.max_rows = max_rows;
   A.max_steps = kStaticMaxSteps;
-  k_plain_init<<<1, 1024, 0, st>>>(A);
-  k_plain_finalize<<<1, 32, 0, st>>>(A, nb, 1);
+  const int ib = plain_blocks(nx, ny, 1);
+  k_plain_init<<<dim3((unsigned)ib), 256, 0, st>>>(A);
+  k_plain_finalize<<<1, kFinThreads, 0, st>>>(A, ib, 1);
   constexpr int kStepsPerPoll = 64;
   PlainCtl hc;
   for (uint64_t polls = 0;; ++polls) {
