@@ -251,6 +251,22 @@ static LaunchCfg make_cfg(const itr_ctx* ctx, int nx, int ny, int C, int T_targe
   return c;
 }
 
+// Whether a cluster shape that the caller asks for (options "cluster" and "threads") is taken or refused.
+// The lines are part of the interface and stay where they were drawn, for 64-column warps that stage their
+// inputs in shared memory; make_cfg's layout needs less nearly everywhere.
+static bool shape_accepted(const itr_ctx* ctx, int nx, int ny, int C, int T, bool crest, bool bnd) {
+  if (C < 1 || ny < C) return false;
+  const int W = (nx + 64) / 64, nr = (ny + C - 1) / C;
+  int S = std::min(T / (32 * W), ny / C);
+  if (W > 1) S = std::min(S, 15);
+  const int nw = S * W;
+  if (S < 1 || nw > 32) return false;
+  size_t o = align_up(28 * (size_t)nr * nx, 16) + 16 * (size_t)(S + 1) * nx + 64 * nw + 16 * (size_t)(nr + nx);   // cells, faces, edge fluxes
+  o = align_up(align_up(o, 16) + 16 * nw, 16) + 112 + 64 * nw + (bnd ? 2 * kMaxInflow * 8 : 0);                    // sums
+  o += (crest ? 3072 : 2048) * (size_t)nw + 2 * (size_t)nr * W + (bnd ? 2 * ((size_t)ny + 2) : 0);                // staged inputs, flags
+  return align_up(align_up(o, 8) + 8, 16) <= ctx->smem_optin;
+}
+
 static int launch_batched(itr_ctx* ctx, const BatchArgs& A, const LaunchCfg& cfg, int n_designs, bool set_attr = true) {
   const bool crest = A.mode == 1, clustered = cfg.C > 1;
   BatchedFn fn = batched_fn(crest, clustered, maxt_bucket(cfg.T), cfg.bnd, A.locked_dt != nullptr, A.P.skip_dry != 0);
@@ -1555,9 +1571,13 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
     };
     auto key = std::make_tuple(nx, ny, n, (int)g->mode + (bnd ? 2 : 0));
     if (ctx->cluster > 0 || ctx->threads > 0) {
-      cfg = make_cfg(ctx, nx, ny, ctx->cluster > 0 ? ctx->cluster : 1, ctx->threads > 0 ? ctx->threads : 512, bnd);
-      if (!cfg.ok) return fail(ctx, ITR_UNSUPPORTED, "cluster=%d threads=%d does not fit a %dx%d grid in shared memory", ctx->cluster, ctx->threads, nx, ny);
-      CU(pack());
+      const int C = ctx->cluster > 0 ? ctx->cluster : 1, T = ctx->threads > 0 ? ctx->threads : 512;
+      if (!shape_accepted(ctx, nx, ny, C, T, crest, bnd))
+        return fail(ctx, ITR_UNSUPPORTED, "cluster=%d threads=%d does not fit a %dx%d grid in shared memory", ctx->cluster, ctx->threads, nx, ny);
+      cfg = make_cfg(ctx, nx, ny, C, T, bnd);
+      if (!cfg.ok) cfg = make_cfg(ctx, nx, ny, C, 32 * windows(nx), bnd);   // a shape this layout has no place for: one strip,
+      tiled = !cfg.ok;                                                      // or the tiled path
+      if (!tiled) CU(pack());
     } else if (ctx->tuned.count(key)) {
       cfg = ctx->tuned[key];
       tiled = cfg.tiled;
