@@ -180,7 +180,8 @@ __global__ void __launch_bounds__(kTileThreads, 6) k_adj_replay(const AdjArgs A,
 // adjoints. dz: the (first) jump's adjoint; dz2: the crest face's second jump's.
 struct FaceBwd { float hl, ul, vl, cl, hr, ur, vr, cr, dz, dz2; };
 
-template <bool NORMAL_X, bool CREST>
+// F: the special operations (Exact or Fast, itr_device.cuh).
+template <class F, bool NORMAL_X, bool CREST>
 ITR_DEV FaceBwd face_bwd(float hl, float ul, float vl, float cl, float hr, float ur, float vr, float cr, float dz,
                          float dz2, const StepK& k, float lm, float lnl, float lnr, float lt) {
   // forward, as face_signed / face_crest and hll compute it
@@ -188,9 +189,9 @@ ITR_DEV FaceBwd face_bwd(float hl, float ul, float vl, float cl, float hr, float
   const float a_l = CREST ? hl - dz : hl - rmax(dz, 0.0f), a_r = CREST ? hr - dz2 : hr - rmax(-dz, 0.0f);
   const float hsl = rmax(a_l, 0.0f), hsr = rmax(a_r, 0.0f);
   const float hred = pos ? hsl : hsr;
-  const float cred = CREST ? 0.0f : sqrt_rn(k.g * hred);
-  const float csl_c = (CREST && dz > 0.0f) ? sqrt_rn(k.g * hsl) : cl;
-  const float csr_c = (CREST && dz2 > 0.0f) ? sqrt_rn(k.g * hsr) : cr;
+  const float cred = CREST ? 0.0f : F::sqrt(k.g * hred);
+  const float csl_c = (CREST && dz > 0.0f) ? F::sqrt(k.g * hsl) : cl;
+  const float csr_c = (CREST && dz2 > 0.0f) ? F::sqrt(k.g * hsr) : cr;
   const float csl = CREST ? csl_c : (pos ? cred : cl), csr = CREST ? csr_c : (pos ? cr : cred);
   const float unl = NORMAL_X ? ul : vl, utl = NORMAL_X ? vl : ul;
   const float unr = NORMAL_X ? ur : vr, utr = NORMAL_X ? vr : ur;
@@ -206,7 +207,7 @@ ITR_DEV FaceBwd face_bwd(float hl, float ul, float vl, float cl, float hr, float
   const float pl = ml * unl + pl_, pr = mr * unr + pr_;
   const bool both = dry_l && dry_r, use_l = sl >= 0.0f, use_r = sr <= 0.0f;
   const float den = (both || use_l || use_r) ? 1.0f : sr - sl;
-  const float inv = rcp(den);
+  const float inv = F::rcp(den);
   const float F1 = sr * ml - sl * mr + sl * sr * (hsr - hsl);
   const float F2 = sr * pl - sl * pr + sl * sr * (mr - ml);
   const float fm = both ? 0.0f : (use_l ? ml : (use_r ? mr : F1 * inv));
@@ -252,12 +253,12 @@ ITR_DEV FaceBwd face_bwd(float hl, float ul, float vl, float cl, float hr, float
   FaceBwd b;
   b.cl = 0.0f; b.cr = 0.0f;
   if (CREST) {   // each side's celerity is its reduced depth's where its jump is positive
-    if (dz > 0.0f) { if (csl > 0.0f) lhsl += lcsl * k.g * 0.5f / csl; } else b.cl = lcsl;
-    if (dz2 > 0.0f) { if (csr > 0.0f) lhsr += lcsr * k.g * 0.5f / csr; } else b.cr = lcsr;
+    if (dz > 0.0f) { if (csl > 0.0f) lhsl += F::div(lcsl * k.g * 0.5f, csl); } else b.cl = lcsl;
+    if (dz2 > 0.0f) { if (csr > 0.0f) lhsr += F::div(lcsr * k.g * 0.5f, csr); } else b.cr = lcsr;
   } else {
     float lcred = 0.0f;
     if (pos) { lcred += lcsl; b.cr = lcsr; } else { b.cl = lcsl; lcred += lcsr; }
-    const float lhred = cred > 0.0f ? lcred * k.g * 0.5f / cred : 0.0f;
+    const float lhred = cred > 0.0f ? F::div(lcred * k.g * 0.5f, cred > 0.0f ? cred : 1.0f) : 0.0f;
     if (pos) lhsl += lhred; else lhsr += lhred;
   }
   const float la_l = a_l > 0.0f ? lhsl : 0.0f, la_r = a_r > 0.0f ? lhsr : 0.0f;
@@ -271,6 +272,7 @@ ITR_DEV FaceBwd face_bwd(float hl, float ul, float vl, float cl, float hr, float
 
 // Adjoint of the sources (numerics.rs:158-194): from the adjoint of the new (h, qx, qy) to
 // that of (h1, qx1, qy1) after the flux update, recomputing the forward as update_cell does.
+template <class F>
 ITR_DEV void sources_bwd(float h, float qx, float qy, const FaceF& w, const FaceF& e, const FaceF& n, const FaceF& s,
                          float wet, float gn2, const StepK& k, float lh, float lqx, float lqy,
                          float& l1h, float& l1qx, float& l1qy) {
@@ -285,9 +287,9 @@ ITR_DEV void sources_bwd(float h, float qx, float qy, const FaceF& w, const Face
   const float r = rcbrt(dry ? 1.0f : h3);
   const float r3 = r * r * r;
   const float r7 = r3 * r3 * r;
-  const float qm = sqrt_rn(qx1 * qx1 + qy1 * qy1);
+  const float qm = F::sqrt(qx1 * qx1 + qy1 * qy1);
   const float a = k.dt * gn2;
-  const float inv = rcp(1.0f + a * qm * r7);
+  const float inv = F::rcp(1.0f + a * qm * r7);
   float lh3 = lh;
   l1qx = 0.0f; l1qy = 0.0f;
   if (!dry) {
@@ -300,10 +302,22 @@ ITR_DEV void sources_bwd(float h, float qx, float qy, const FaceF& w, const Face
     const float lqm = lD * a * r7;
     const float lr7 = lD * a * qm;
     lh3 += lr7 * (-7.0f / 3.0f) * r7 * r3;                  // d h^(-7/3) / dh
-    if (qm > 0.0f) { l1qx += lqm * qx1 / qm; l1qy += lqm * qy1 / qm; }
+    if (qm > 0.0f) { l1qx += F::div(lqm * qx1, qm); l1qy += F::div(lqm * qy1, qm); }
   }
   const float lh2 = capw < h2 ? lh3 : 0.0f;                // infiltration capped at h2 -> h3 = 0
   l1h = h1 < 0.0f ? 0.0f : lh2;                            // positivity fix
+}
+
+// The velocity map u = qx t(h), v = qy t(h), c = sqrt(g h) (numerics.rs:38-45) taken back: t(h), dt/dh and
+// d(c)/dh times lc.
+template <class F>
+ITR_DEV void vel_bwd(float h, float c, float lc, const StepK& k, float& t, float& dtdh, float& lch) {
+  const float h2 = h * h, den = h2 + rmax(h2, k.heps2);
+  t = (h + h) * F::rcp(den);
+  const bool deep = h2 > k.heps2;
+  dtdh = F::div(deep ? -1.0f : 2.0f * (k.heps2 - h2), deep ? h2 : den * den);
+  const bool wet = c > 0.0f;
+  lch = wet ? F::div(lc * k.g * 0.5f, wet ? c : 1.0f) : 0.0f;
 }
 
 // ---- the backward step ----
@@ -313,15 +327,27 @@ ITR_DEV void sources_bwd(float h, float qx, float qy, const FaceF& w, const Face
 // four faces' input adjoints (ghost sides folded back onto the interior cell).
 constexpr int kR = 20, kQ = 18;
 
-template <bool BND, bool CREST>
-__global__ void __launch_bounds__(kTileThreads) k_adj_step(const AdjArgs A, int j) {
-  __shared__ float sh[kR * kR], sqx[kR * kR], sqy[kR * kR], su[kR * kR], sv[kR * kR], sc[kR * kR];
-  __shared__ FaceF fx[kQ * 19], fy[19 * kQ];           // forward faces of the 18x18 cells
-  __shared__ float jx[kQ * 19], jy[19 * kQ];            // their jumps
-  __shared__ float jx2[CREST ? kQ * 19 : 1], jy2[CREST ? 19 * kQ : 1];   // crest: second jumps
-  __shared__ float l1[3][kQ * kQ];                      // adjoint of (h1, qx1, qy1)
-  __shared__ float bx[16 * 17][8], by[17 * 16][8];      // face input adjoints: L (h,u,v,c), R (h,u,v,c)
-  __shared__ float2 sinf[kMaxInflow];                   // the step's inflow group values
+// Shared memory of one tile.
+template <bool CREST>
+struct AdjTile {
+  float sh[kR * kR], sqx[kR * kR], sqy[kR * kR], su[kR * kR], sv[kR * kR], sc[kR * kR];
+  FaceF fx[kQ * 19], fy[19 * kQ];           // forward faces of the 18x18 cells
+  float jx[kQ * 19], jy[19 * kQ];            // their jumps
+  float jx2[CREST ? kQ * 19 : 1], jy2[CREST ? 19 * kQ : 1];   // crest: second jumps
+  float l1[3][kQ * kQ];                      // adjoint of (h1, qx1, qy1)
+  float bx[16 * 17][8], by[17 * 16][8];      // face input adjoints: L (h,u,v,c), R (h,u,v,c)
+  float2 sinf[kMaxInflow];                   // the step's inflow group values
+};
+
+template <class F, bool BND, bool CREST>
+ITR_DEV void adj_step_tile(const AdjArgs& A, int j, AdjTile<CREST>& sm) {
+  auto &sh = sm.sh, &sqx = sm.sqx, &sqy = sm.sqy, &su = sm.su, &sv = sm.sv, &sc = sm.sc;
+  auto &fx = sm.fx, &fy = sm.fy;
+  auto &jx = sm.jx, &jy = sm.jy;
+  auto &jx2 = sm.jx2, &jy2 = sm.jy2;
+  auto &l1 = sm.l1;
+  auto &bx = sm.bx, &by = sm.by;
+  auto &sinf = sm.sinf;
   const int d = blockIdx.z;
   const int nx = A.nx, ny = A.ny;
   const size_t N = (size_t)nx * ny, SX = (size_t)ny * (nx + 1), SY = (size_t)(ny + 1) * nx;
@@ -381,7 +407,7 @@ __global__ void __launch_bounds__(kTileThreads) k_adj_step(const AdjArgs A, int 
     const int ix = e % kR, iy = e / kR;
     float h, qx, qy, u, v, c;
     adj_load<BND>(A, X, gx0 - 2 + ix, gy0 - 2 + iy, h, qx, qy, bh, sinf);
-    cell_vel(h, qx, qy, k.g, k.heps2, u, v, c);
+    cell_vel<F>(h, qx, qy, k.g, k.heps2, u, v, c);
     sh[e] = h; sqx[e] = qx; sqy[e] = qy; su[e] = u; sv[e] = v; sc[e] = c;
   }
   jx[li] = jxa; jy[li] = jya;
@@ -400,7 +426,7 @@ __global__ void __launch_bounds__(kTileThreads) k_adj_step(const AdjArgs A, int 
       FaceF o{};
       if (row >= 0 && row < ny && f >= 0 && f <= nx) {
         const int a = (jr + 1) * kR + fi;
-        o = face<true, CREST>(sh[a], su[a], sv[a], sc[a], sh[a + 1], su[a + 1], sv[a + 1], sc[a + 1], jx[e],
+        o = face<true, CREST, F>(sh[a], su[a], sv[a], sc[a], sh[a + 1], su[a + 1], sv[a + 1], sc[a + 1], jx[e],
                               CREST ? jx2[e] : 0.0f, k);
       }
       fx[e] = o;
@@ -411,7 +437,7 @@ __global__ void __launch_bounds__(kTileThreads) k_adj_step(const AdjArgs A, int 
       FaceF o{};
       if (col >= 0 && col < nx && f >= 0 && f <= ny) {
         const int a = fr * kR + ic + 1, b = a + kR;
-        o = face<false, CREST>(sh[a], su[a], sv[a], sc[a], sh[b], su[b], sv[b], sc[b], jy[e], CREST ? jy2[e] : 0.0f, k);
+        o = face<false, CREST, F>(sh[a], su[a], sv[a], sc[a], sh[b], su[b], sv[b], sc[b], jy[e], CREST ? jy2[e] : 0.0f, k);
       }
       fy[e] = o;
     }
@@ -432,7 +458,7 @@ __global__ void __launch_bounds__(kTileThreads) k_adj_step(const AdjArgs A, int 
         if (A.seed_cell[si] == gi && A.seed_state[si] == n + 1) lh += A.seed_w[si];
       }
       const int a = (jr + 1) * kR + ic + 1;
-      sources_bwd(sh[a], sqx[a], sqy[a], fx[jr * 19 + ic], fx[jr * 19 + ic + 1], fy[jr * kQ + ic], fy[(jr + 1) * kQ + ic],
+      sources_bwd<F>(sh[a], sqx[a], sqy[a], fx[jr * 19 + ic], fx[jr * 19 + ic + 1], fy[jr * kQ + ic], fy[(jr + 1) * kQ + ic],
                   A.wet[gi], A.gn2[gi], k, lh, lqx, lqy, a0, a1, a2);
     }
     l1[0][e] = a0; l1[1][e] = a1; l1[2][e] = a2;
@@ -452,7 +478,7 @@ __global__ void __launch_bounds__(kTileThreads) k_adj_step(const AdjArgs A, int 
         const float lt = -k.dtdx * l1[2][L] + k.dtdx * l1[2][R];
         const int a = (yr + 1) * kR + xl;   // region cell of L
         const float dz = jx[yr * 19 + xl], dz2 = CREST ? jx2[yr * 19 + xl] : 0.0f;
-        const FaceBwd b = face_bwd<true, CREST>(sh[a], su[a], sv[a], sc[a], sh[a + 1], su[a + 1], sv[a + 1], sc[a + 1], dz, dz2, k,
+        const FaceBwd b = face_bwd<F, true, CREST>(sh[a], su[a], sv[a], sc[a], sh[a + 1], su[a + 1], sv[a + 1], sc[a + 1], dz, dz2, k,
                                          lm, lnl, lnr, lt);
         o[0] = b.hl; o[1] = b.ul; o[2] = b.vl; o[3] = b.cl; o[4] = b.hr; o[5] = b.ur; o[6] = b.vr; o[7] = b.cr;
         if (xown) *gxp = gx_old + (double)b.dz;
@@ -471,7 +497,7 @@ __global__ void __launch_bounds__(kTileThreads) k_adj_step(const AdjArgs A, int 
         const float lnl = -k.dtdy * l1[2][T], lnr = k.dtdy * l1[2][B];
         const int a = yt * kR + xc + 1;      // region cell of T
         const float dz = jy[yt * kQ + xc], dz2 = CREST ? jy2[yt * kQ + xc] : 0.0f;
-        const FaceBwd b = face_bwd<false, CREST>(sh[a], su[a], sv[a], sc[a], sh[a + kR], su[a + kR], sv[a + kR], sc[a + kR], dz, dz2,
+        const FaceBwd b = face_bwd<F, false, CREST>(sh[a], su[a], sv[a], sc[a], sh[a + kR], su[a + kR], sv[a + kR], sc[a + kR], dz, dz2,
                                           k, lm, lnl, lnr, lt);
         o[0] = b.hl; o[1] = b.ul; o[2] = b.vl; o[3] = b.cl; o[4] = b.hr; o[5] = b.ur; o[6] = b.vr; o[7] = b.cr;
         if (yown) *gyp = gy_old + (double)b.dz;
@@ -521,14 +547,12 @@ __global__ void __launch_bounds__(kTileThreads) k_adj_step(const AdjArgs A, int 
         if (BND && code >= 2) fold(code, Sf + 4, a + kR);
         else { const float s = code == 0 ? -1.0f : 1.0f; lh += Sf[4]; lu += Sf[5]; lv += s * Sf[6]; lc += Sf[7]; }
       }
-      // velocity map (numerics.rs:38-45): u = qx t(h), v = qy t(h), c = sqrt(g h)
-      const float h = sh[a], qx = sqx[a], qy = sqy[a], c = sc[a];
-      const float h2 = h * h, den = h2 + rmax(h2, k.heps2);
-      const float t = (h + h) * rcp(den);
-      const float dtdh = h2 > k.heps2 ? -1.0f / h2 : 2.0f * (k.heps2 - h2) / (den * den);
+      const float h = sh[a], qx = sqx[a], qy = sqy[a];
+      float t, dtdh, lch;
+      vel_bwd<F>(h, sc[a], lc, k, t, dtdh, lch);
       const int q = (ly + 1) * kQ + lx + 1;
       const size_t gi = (size_t)gy * nx + gx;
-      float oh = lh + (lu * qx + lv * qy) * dtdh + (c > 0.0f ? lc * k.g * 0.5f / c : 0.0f) + l1[0][q];
+      float oh = lh + (lu * qx + lv * qy) * dtdh + lch + l1[0][q];
       float oqx = lu * t + l1[1][q], oqy = lv * t + l1[2][q];
       if (BND) { oh += gh; oqx += gqx; oqy += gqy; }
       LO[gi] = oh;
@@ -536,6 +560,13 @@ __global__ void __launch_bounds__(kTileThreads) k_adj_step(const AdjArgs A, int 
       LO[2 * N + gi] = oqy;
     }
   }
+}
+
+template <bool BND, bool CREST>
+__global__ void __launch_bounds__(kTileThreads) k_adj_step(const AdjArgs A, int j) {
+  __shared__ AdjTile<CREST> sm;
+  if (A.seg[((size_t)blockIdx.z * A.K + j) * kLog + 3] == 0.0) adj_step_tile<Fast, BND, CREST>(A, j, sm);
+  else adj_step_tile<Exact, BND, CREST>(A, j, sm);
 }
 
 // Checkpoint: the current state plane of every design into dst (per design [3][N]).

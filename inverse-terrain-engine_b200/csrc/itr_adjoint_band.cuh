@@ -20,6 +20,11 @@
 //     one face-adjoint pair, against 1.27 of each for the tile;
 //   * lane 0's west x-face needs the cell two columns west: computed for every row of the band
 //     before the sweep (one face per lane) and kept in shared memory.
+// What bounds it: instruction issue and latency of the long dependent chains of a face's adjoint at 24
+// warps an SM. In a step from a bounded state (the recorded flag of the forward step) the square
+// roots, reciprocals and divisions run without branches (Fast), so that a row's chains overlap, and
+// divisions by 1 on dry sides are selected instead of branched over: the backward pass of 4 designs of
+// 600 x 512, 454 steps, 68.6 -> 54.4 ms (replay included), of 8 of 240 x 192, 592 steps, 8.0 -> 7.3 ms.
 #pragma once
 #include <cmath>
 #include "itr_adjoint.cuh"
@@ -31,8 +36,9 @@ constexpr int kAdjOwn = 29;     // columns a warp owns (lanes 1 .. 29)
 constexpr int kAdjWarps = 4;    // most warps (segments) per block
 constexpr int kAdjRows = 32;    // most rows per band
 #ifndef ITR_ADJ_MIN_BLOCKS
-#define ITR_ADJ_MIN_BLOCKS 6    // resident blocks per SM the register budget is cut for (85
-                                // registers, a few spilled: measured faster than 4 and 8)
+#define ITR_ADJ_MIN_BLOCKS 6    // resident blocks per SM the register budget is cut for (80
+                                // registers, some spilled: the 600 x 512 pass above takes 54.4 ms,
+                                // 57.2 ms with 5 and 57.0 ms with 4 blocks)
 #endif
 
 struct AdjGeom {
@@ -125,10 +131,9 @@ ITR_DEV FaceBwd facebwd_shfl_down(const FaceBwd& b) {
   return r;
 }
 
-template <bool BND, bool CREST>
-__global__ void __launch_bounds__(kAdjWarps * 32, ITR_ADJ_MIN_BLOCKS) k_adj_band(const AdjArgs A, int j) {
-  __shared__ FaceF edge[kAdjWarps][2 * 32];   // lane 0's west x-face, rows r0 - 1 .. r1
-  __shared__ float2 sinf[kMaxInflow];
+// edge: lane 0's west x-face, rows r0 - 1 .. r1. F: the special operations (Exact or Fast).
+template <class F, bool BND, bool CREST>
+ITR_DEV void adj_band_sweep(const AdjArgs& A, int j, FaceF (*edge)[2 * 32], float2* sinf) {
   const int d = blockIdx.z;
   const int nx = A.nx, ny = A.ny, nxp1 = nx + 1;
   const size_t N = (size_t)nx * ny, SX = (size_t)ny * (nx + 1), SY = (size_t)(ny + 1) * nx;
@@ -172,7 +177,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, ITR_ADJ_MIN_BLOCKS) k_adj_band
     a.u = a.v = a.c = 0.0f;
     return a;
   };
-  auto vel = [&](ACell a) -> ACell { cell_vel(a.h, a.qx, a.qy, k.g, k.heps2, a.u, a.v, a.c); return a; };
+  auto vel = [&](ACell a) -> ACell { cell_vel<F>(a.h, a.qx, a.qy, k.g, k.heps2, a.u, a.v, a.c); return a; };
   auto cell = [&](int gx, int gy) -> ACell { return vel(raw(gx, gy)); };
   const bool xcol = col >= 0 && col <= nx;    // x-face `col` exists
   const bool ycol = col >= 0 && col < nx;     // y-faces of column `col` exist
@@ -180,13 +185,13 @@ __global__ void __launch_bounds__(kAdjWarps * 32, ITR_ADJ_MIN_BLOCKS) k_adj_band
   // (computed on every lane, then zeroed where the face does not exist: one straight-line body
   //  lets the compiler interleave a row's independent chains)
   auto xfwd = [&](const ACell& L, const ACell& C, int r, float dz, float dz2) -> FaceF {
-    FaceF o = face<true, CREST>(L.h, L.u, L.v, L.c, C.h, C.u, C.v, C.c, dz, dz2, k);
+    FaceF o = face<true, CREST, F>(L.h, L.u, L.v, L.c, C.h, C.u, C.v, C.c, dz, dz2, k);
     if (!(xcol && r >= 0 && r < ny)) o = FaceF{};
     return o;
   };
   // forward y-face f between (f - 1, col) and (f, col)
   auto yfwd = [&](const ACell& T, const ACell& B, int f, float dz, float dz2) -> FaceF {
-    FaceF o = face<false, CREST>(T.h, T.u, T.v, T.c, B.h, B.u, B.v, B.c, dz, dz2, k);
+    FaceF o = face<false, CREST, F>(T.h, T.u, T.v, T.c, B.h, B.u, B.v, B.c, dz, dz2, k);
     if (!(ycol && f >= 0 && f <= ny)) o = FaceF{};
     return o;
   };
@@ -200,7 +205,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, ITR_ADJ_MIN_BLOCKS) k_adj_band
     if (f >= 0 && f <= nx && r >= 0 && r < ny) {
       const ACell a = cell(f - 1, r), b = cell(f, r);
       const size_t xo = (size_t)r * nxp1 + f;
-      o = face<true, CREST>(a.h, a.u, a.v, a.c, b.h, b.u, b.v, b.c, dzx[xo], CREST ? dzx2[xo] : 0.0f, k);
+      o = face<true, CREST, F>(a.h, a.u, a.v, a.c, b.h, b.u, b.v, b.c, dzx[xo], CREST ? dzx2[xo] : 0.0f, k);
     }
     edge[wid][e] = o;
   }
@@ -231,7 +236,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, ITR_ADJ_MIN_BLOCKS) k_adj_band
         if (A.seed_cell[si] == gi && A.seed_state[si] == n + 1) lh += A.seed_w[si];
       }
     }
-    sources_bwd(C.h, C.qx, C.qy, W, E, Nf, Sf, wet, gn2, k, lh, lqx, lqy, o.h, o.qx, o.qy);
+    sources_bwd<F>(C.h, C.qx, C.qy, W, E, Nf, Sf, wet, gn2, k, lh, lqx, lqy, o.h, o.qx, o.qy);
     if (!in) o = L1{0.0f, 0.0f, 0.0f};
     return o;
   };
@@ -278,7 +283,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, ITR_ADJ_MIN_BLOCKS) k_adj_band
     const float lm = -k.dtdy * lb.h + k.dtdy * lc.h;
     const float lt = -k.dtdy * lb.qx + k.dtdy * lc.qx;
     const float lnl = -k.dtdy * lb.qy, lnr = k.dtdy * lc.qy;
-    nb = face_bwd<false, CREST>(Sb.h, Sb.u, Sb.v, Sb.c, Sc.h, Sc.u, Sc.v, Sc.c, jyb, jyb2, k, lm, lnl, lnr, lt);
+    nb = face_bwd<F, false, CREST>(Sb.h, Sb.u, Sb.v, Sb.c, Sc.h, Sc.u, Sc.v, Sc.c, jyb, jyb2, k, lm, lnl, lnr, lt);
     if (own) {
       double* gp = A.gdzy + d * SY + (size_t)r0 * nx + col;
       *gp = *gp + (double)nb.dz;
@@ -321,7 +326,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, ITR_ADJ_MIN_BLOCKS) k_adj_band
       const float lm = -k.dtdy * lc.h + k.dtdy * ld.h;
       const float lt = -k.dtdy * lc.qx + k.dtdy * ld.qx;
       const float lnl = -k.dtdy * lc.qy, lnr = k.dtdy * ld.qy;
-      sb = face_bwd<false, CREST>(Sc.h, Sc.u, Sc.v, Sc.c, Sd.h, Sd.u, Sd.v, Sd.c, jyc, jyc2, k, lm, lnl, lnr, lt);
+      sb = face_bwd<F, false, CREST>(Sc.h, Sc.u, Sc.v, Sc.c, Sd.h, Sd.u, Sd.v, Sd.c, jyc, jyc2, k, lm, lnl, lnr, lt);
     }
     // adjoint of the west x-face of (r, col), lanes 1 .. 30 (lane 30's is the east face of 29)
     const ACell Wc = acell_shfl_up(Sc);
@@ -332,7 +337,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32, ITR_ADJ_MIN_BLOCKS) k_adj_band
       const float lm = -k.dtdx * lwh + k.dtdx * lc.h;
       const float lnl = -k.dtdx * lwqx, lnr = k.dtdx * lc.qx;
       const float lt = -k.dtdx * lwqy + k.dtdx * lc.qy;
-      xb = face_bwd<true, CREST>(Wc.h, Wc.u, Wc.v, Wc.c, Sc.h, Sc.u, Sc.v, Sc.c, jxc, jxc2, k, lm, lnl, lnr, lt);
+      xb = face_bwd<F, true, CREST>(Wc.h, Wc.u, Wc.v, Wc.c, Sc.h, Sc.u, Sc.v, Sc.c, jxc, jxc2, k, lm, lnl, lnr, lt);
     }
     if (!(xcol && lane >= 1)) xb = FaceBwd{};   // (lane 0 and columns past the east face)
     if (yown_r) {
@@ -381,13 +386,11 @@ __global__ void __launch_bounds__(kAdjWarps * 32, ITR_ADJ_MIN_BLOCKS) k_adj_band
         if (BND && code >= 2) fold(code, Sf + 4, Sd);
         else { const float sg_ = code == 0 ? -1.0f : 1.0f; lh += Sf[4]; lu += Sf[5]; lv += sg_ * Sf[6]; lcc += Sf[7]; }
       }
-      // velocity map (numerics.rs:38-45): u = qx t(h), v = qy t(h), c = sqrt(g h)
-      const float h = Sc.h, qx = Sc.qx, qy = Sc.qy, c = Sc.c;
-      const float h2 = h * h, den = h2 + rmax(h2, k.heps2);
-      const float t = (h + h) * rcp(den);
-      const float dtdh = h2 > k.heps2 ? -1.0f / h2 : 2.0f * (k.heps2 - h2) / (den * den);
+      const float h = Sc.h, qx = Sc.qx, qy = Sc.qy;
+      float t, dtdh, lch;
+      vel_bwd<F>(h, Sc.c, lcc, k, t, dtdh, lch);
       const size_t gi = (size_t)r * nx + col;
-      float oh = lh + (lu * qx + lv * qy) * dtdh + (c > 0.0f ? lcc * k.g * 0.5f / c : 0.0f) + lc.h;
+      float oh = lh + (lu * qx + lv * qy) * dtdh + lch + lc.h;
       float oqx = lu * t + lc.qx, oqy = lv * t + lc.qy;
       if (BND) { oh += gh; oqx += gqx; oqy += gqy; }
       LO[gi] = oh;
@@ -401,6 +404,14 @@ __global__ void __launch_bounds__(kAdjWarps * 32, ITR_ADJ_MIN_BLOCKS) k_adj_band
     lc = ld;
     nb = sb;
   }
+}
+
+template <bool BND, bool CREST>
+__global__ void __launch_bounds__(kAdjWarps * 32, ITR_ADJ_MIN_BLOCKS) k_adj_band(const AdjArgs A, int j) {
+  __shared__ FaceF edge[kAdjWarps][2 * 32];
+  __shared__ float2 sinf[kMaxInflow];
+  if (A.seg[((size_t)blockIdx.z * A.K + j) * kLog + 3] == 0.0) adj_band_sweep<Fast, BND, CREST>(A, j, edge, sinf);
+  else adj_band_sweep<Exact, BND, CREST>(A, j, edge, sinf);
 }
 
 }  // namespace itr

@@ -64,16 +64,49 @@ ITR_DEV float sqrt_rn(float x) {
   return z ? x : r;
 }
 
+// The special operations of the scalar path: Exact for every operand; Fast without branches, the same
+// bits for operands in the ranges that rcp2 and sqrt2 (below) state, which hold in a step from a
+// bounded state (StepK::exact == 0). Fast::div: a y with y = 1 / b rounded, corrected twice by the
+// exact residual (as div_rn), b in rcp2's range; a small |a| (adjoints at the fringe of their domain
+// of dependence) is scaled by 2^64 and back, which keeps the residual a normal number.
+struct Exact {
+  static ITR_DEV float rcp(float x) { return itr::rcp(x); }
+  static ITR_DEV float sqrt(float x) { return sqrt_rn(x); }
+  static ITR_DEV float div(float a, float b) { return a / b; }
+};
+ITR_DEV float rcp_est(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+ITR_DEV float rsqrt_est(float x) { float r; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+struct Fast {
+  static ITR_DEV float rcp(float x) {
+    const float y = rcp_est(x);
+    return __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
+  }
+  static ITR_DEV float sqrt(float x) {
+    const float xs = 0x1p48f * x, y = rsqrt_est(xs + 0x1p-126f);
+    const float s = xs * y;
+    return __fmaf_rn(__fmaf_rn(-s, s, xs), 0x1p-25f * y, 0x1p-24f * s);
+  }
+  static ITR_DEV float div(float a, float b) {
+    const bool tiny = fabsf(a) < 0x1p-60f;
+    const float y = rcp(b), as = a * (tiny ? 0x1p64f : 1.0f);
+    float q = as * y;
+    q = __fmaf_rn(__fmaf_rn(-b, q, as), y, q);
+    return __fmaf_rn(__fmaf_rn(-b, q, as), y, q) * (tiny ? 0x1p-64f : 1.0f);
+  }
+};
+
+template <class F = Exact>
 ITR_DEV void cell_vel(float h, float qx, float qy, float g, float heps2, float& u, float& v, float& c) {
   float h2 = h * h;
-  float inv = rcp(h2 + rmax(h2, heps2));
+  float inv = F::rcp(h2 + rmax(h2, heps2));
   float t = (h + h) * inv;
   u = qx * t;
   v = qy * t;
-  c = sqrt_rn(g * h);
+  c = F::sqrt(g * h);
 }
 
 // HLL flux with two-rarefaction wave speeds; dry-dry faces give exactly zero.
+template <class F = Exact>
 ITR_DEV FaceF hll(float hl, float ul, float tl, float cl, float hr, float ur, float tr, float cr, float g_half) {
   const bool dry_l = !(hl > 0.0f);
   const bool dry_r = !(hr > 0.0f);
@@ -93,7 +126,7 @@ ITR_DEV FaceF hll(float hl, float ul, float tl, float cl, float hr, float ur, fl
   const bool use_l = sl >= 0.0f;
   const bool use_r = sr <= 0.0f;
   float den = (both_dry || use_l || use_r) ? 1.0f : sr - sl;
-  float inv = rcp(den);
+  float inv = F::rcp(den);
   float slsr = sl * sr;
   float fm_star = (sr * ml - sl * mr + slsr * (hr - hl)) * inv;
   float fn_star = (sr * pl - sl * pr + slsr * (mr - ml)) * inv;
@@ -107,37 +140,37 @@ ITR_DEV FaceF hll(float hl, float ul, float tl, float cl, float hr, float ur, fl
 
 // Signed-jump face (dz = z_R - z_L): one reduced side, one square root. `normal_x` picks
 // which velocity component is normal. (ul,vl,cl) are the left/top cell's velocity.
-template <bool NORMAL_X>
+template <bool NORMAL_X, class F>
 ITR_DEV FaceF face_signed(float hl, float ul, float vl, float cl, float hr, float ur, float vr, float cr,
                           float dz, float g, float g_half) {
   const bool pos = dz > 0.0f;
   float hsl = rmax(hl - rmax(dz, 0.0f), 0.0f);
   float hsr = rmax(hr - rmax(-dz, 0.0f), 0.0f);
   float hred = pos ? hsl : hsr;
-  float cred = sqrt_rn(g * hred);
+  float cred = F::sqrt(g * hred);
   float csl = pos ? cred : cl;
   float csr = pos ? cr : cred;
-  if (NORMAL_X) return hll(hsl, ul, vl, csl, hsr, ur, vr, csr, g_half);
-  return hll(hsl, vl, ul, csl, hsr, vr, ur, csr, g_half);
+  if (NORMAL_X) return hll<F>(hsl, ul, vl, csl, hsr, ur, vr, csr, g_half);
+  return hll<F>(hsl, vl, ul, csl, hsr, vr, ur, csr, g_half);
 }
 
 // Crest face: two non-negative jumps d_l = z_f - z_L, d_r = z_f - z_R.
-template <bool NORMAL_X>
+template <bool NORMAL_X, class F>
 ITR_DEV FaceF face_crest(float hl, float ul, float vl, float cl, float hr, float ur, float vr, float cr,
                          float d_l, float d_r, float g, float g_half) {
   float hsl = rmax(hl - d_l, 0.0f);
   float hsr = rmax(hr - d_r, 0.0f);
-  float csl = d_l > 0.0f ? sqrt_rn(g * hsl) : cl;
-  float csr = d_r > 0.0f ? sqrt_rn(g * hsr) : cr;
-  if (NORMAL_X) return hll(hsl, ul, vl, csl, hsr, ur, vr, csr, g_half);
-  return hll(hsl, vl, ul, csl, hsr, vr, ur, csr, g_half);
+  float csl = d_l > 0.0f ? F::sqrt(g * hsl) : cl;
+  float csr = d_r > 0.0f ? F::sqrt(g * hsr) : cr;
+  if (NORMAL_X) return hll<F>(hsl, ul, vl, csl, hsr, ur, vr, csr, g_half);
+  return hll<F>(hsl, vl, ul, csl, hsr, vr, ur, csr, g_half);
 }
 
-template <bool NORMAL_X, bool CREST>
+template <bool NORMAL_X, bool CREST, class F = Exact>
 ITR_DEV FaceF face(float hl, float ul, float vl, float cl, float hr, float ur, float vr, float cr,
                    float d0, float d1, const StepK& k) {
-  if (CREST) return face_crest<NORMAL_X>(hl, ul, vl, cl, hr, ur, vr, cr, d0, d1, k.g, k.g_half);
-  return face_signed<NORMAL_X>(hl, ul, vl, cl, hr, ur, vr, cr, d0, k.g, k.g_half);
+  if (CREST) return face_crest<NORMAL_X, F>(hl, ul, vl, cl, hr, ur, vr, cr, d0, d1, k.g, k.g_half);
+  return face_signed<NORMAL_X, F>(hl, ul, vl, cl, hr, ur, vr, cr, d0, k.g, k.g_half);
 }
 
 // Result of one cell update. c is sqrt(g*h) of the new depth, which is also the next
@@ -542,7 +575,6 @@ ITR_DEV B2 gt2(float2 a, float b) { return B2{a.x > b, a.y > b}; }
 // refinement: P. Markstein, IBM J. Res. Dev. 34(1), 1990; J.-M. Muller et al., Handbook of
 // Floating-Point Arithmetic, 2nd ed., 2018, ch. 4): y = est(1/x); e = fma(-x, y, 1); y + y e.
 // Equal to CUDA's IEEE reciprocal on every 32-bit input of that range (checked on the B200).
-ITR_DEV float rcp_est(float x) { float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 ITR_DEV float2 rcp2(float2 x) {
   const float2 y = make_float2(rcp_est(x.x), rcp_est(x.y));
   const float2 e = make_float2(__fmaf_rn(-x.x, y.x, 1.0f), __fmaf_rn(-x.y, y.y, 1.0f));
@@ -554,7 +586,6 @@ ITR_DEV float2 rcp2(float2 x) {
 // The 2^-126 added for the estimate alone keeps it finite at 0 and vanishes in rounding
 // elsewhere. Equal to CUDA's IEEE square root on every 32-bit input of that range (checked on the
 // B200); about half its time, and without the branch that would end the basic block.
-ITR_DEV float rsqrt_est(float x) { float r; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 ITR_DEV float2 sqrt2(float2 x) {
   const float2 xs = mulc2(0x1p48f, x);
   const float2 xt = addc2(xs, 0x1p-126f);
