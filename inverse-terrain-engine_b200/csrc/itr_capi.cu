@@ -1396,7 +1396,7 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
     const size_t items = faces > NB ? faces : NB;
     k_materialize<<<dim3((unsigned)((N + 255) / 256), (unsigned)n), 256, 0, ctx->stream>>>(MA);
     k_mat_jumps<<<dim3((unsigned)((items + 255) / 256), (unsigned)n), 256, 0, ctx->stream>>>(MA);
-    k_mat_volumes<<<(n + 3) / 4, 128, 0, ctx->stream>>>(MA);   // a warp per design
+    k_mat_volumes<<<n, kVolThreads, 0, ctx->stream>>>(MA);
     launches += 3;
     double* hv = ctx->mVol.as<double>();
     CU(cudaMemcpyAsync(hv, dv + o_cut, (size_t)n * 8, cudaMemcpyDeviceToHost, ctx->stream));
@@ -2124,7 +2124,8 @@ extern "C" int itr_gpu_vjp_primitives(itr_ctx* ctx, const itr_params* p, const i
   CU(ctx->mAux.ensure(2 * N));
   CU(ctx->mJp.ensure((jp.size() > 0 ? jp.size() : 1) * sizeof(MatPrim)));
   CU(ctx->mJob.ensure((jobs.size() > 0 ? jobs.size() : 1) * sizeof(MatJob)));
-  CU(ctx->mOut.ensure((size_t)(3 * (jobs.size() > 0 ? jobs.size() : 1)) * 8));
+  const int slices = mat_dgrad_slices((int)jobs.size(), ctx->sm_count), n_out = 3 * (int)jobs.size();
+  CU(ctx->mOut.ensure((size_t)(slices + 1) * (n_out > 0 ? n_out : 1) * 8));
   CU(ctx->mZe.ensure((size_t)n * N * 8));
   CU(cudaMemcpyAsync(ctx->mAux.p, sp->editable, N, cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync(ctx->mAux.as<uint8_t>() + N, sp->wall, N, cudaMemcpyHostToDevice, st));
@@ -2142,9 +2143,12 @@ extern "C" int itr_gpu_vjp_primitives(itr_ctx* ctx, const itr_params* p, const i
     MA.ox = sp->origin_x; MA.oy = sp->origin_y; MA.dx = g->dx; MA.dy = g->dy;
     MA.z_wall = sp->z_wall; MA.max_abs_dz = sp->max_abs_dz;
     MA.editable = ctx->mAux.as<uint8_t>();
-    k_mat_dgrad<<<(unsigned)jobs.size(), 256, 0, st>>>(MA, ctx->mJp.as<MatPrim>(), ctx->mJob.as<MatJob>(), ctx->mDz.as<double>(),
-                                                       gdz, ob->earth_weight, ob->cut_cost, ob->fill_cost, ctx->mOut.as<double>());
-    CU(cudaMemcpyAsync(dj_dprim, ctx->mOut.p, 3 * jobs.size() * 8, cudaMemcpyDeviceToHost, st));
+    double* const out = ctx->mOut.as<double>();
+    k_mat_dgrad<<<dim3((unsigned)jobs.size(), (unsigned)slices), 256, 0, st>>>(MA, ctx->mJp.as<MatPrim>(), ctx->mJob.as<MatJob>(),
+                                                                               ctx->mDz.as<double>(), gdz, ob->earth_weight,
+                                                                               ob->cut_cost, ob->fill_cost, out + n_out, n_out);
+    k_mat_dgrad_sum<<<(unsigned)((n_out + 255) / 256), 256, 0, st>>>(out + n_out, slices, n_out, out);
+    CU(cudaMemcpyAsync(dj_dprim, out, (size_t)n_out * 8, cudaMemcpyDeviceToHost, st));
   }
   CU(cudaStreamSynchronize(st));
   return ITR_OK;

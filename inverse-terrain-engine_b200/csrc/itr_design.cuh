@@ -56,8 +56,8 @@ struct MatArgs {
   float* bh;               // n * (2nx+2ny) stage-ghost depths
 };
 
-// Primitive::profile (design.rs:107-134).
-__device__ __forceinline__ double mat_profile(const MatPrim& p, double x, double y) {
+// Distance of (x, y) from the primitive's segment.
+__device__ __forceinline__ double mat_distance(const MatPrim& p, double x, double y) {
   const double vx = p.x1 - p.x0, vy = p.y1 - p.y0;
   const double l2 = vx * vx + vy * vy;
   double t = 0.0;
@@ -66,7 +66,12 @@ __device__ __forceinline__ double mat_profile(const MatPrim& p, double x, double
     t = t < 0.0 ? 0.0 : (t > 1.0 ? 1.0 : t);
   }
   const double px = p.x0 + t * vx - x, py = p.y0 + t * vy - y;
-  const double d = sqrt(px * px + py * py);
+  return sqrt(px * px + py * py);
+}
+
+// Primitive::profile (design.rs:107-134).
+__device__ __forceinline__ double mat_profile(const MatPrim& p, double x, double y) {
+  const double d = mat_distance(p, x, y);
   const double s = d / (0.5 * p.width);
   if (s >= 1.0) return 0.0;
   if (p.kind == 2) {   // cut: flat bottom, then a (1 - u^2)^2 bank
@@ -79,7 +84,18 @@ __device__ __forceinline__ double mat_profile(const MatPrim& p, double x, double
   return w * w;
 }
 
-// dz and the edited level of every cell of every design (grid: cells / 256 x designs).
+// Every sub-sample of the cell centred on (x, y) lies outside the primitive, where its profile is 0: the
+// samples are within 0.375 (dx + dy) of the centre, and 1e-9 of the coordinates' size covers the
+// rounding. False for anything not a number, a negative width or an infinite height (0 times that).
+__device__ __forceinline__ bool mat_outside(const MatPrim& p, double x, double y, double dx, double dy) {
+  const double reach = 0.5 * p.width + 0.4 * (dx + dy) +
+                       1e-9 * (fabs(x) + fabs(y) + fabs(p.x0) + fabs(p.y0) + fabs(p.x1) + fabs(p.y1));
+  return p.width >= 0.0 && fabs(p.height) < 1e300 && mat_distance(p, x, y) > reach;
+}
+
+// dz and the edited level of every cell of every design (grid: cells / 256 x designs). Bound by f64
+// divisions and square roots, 16 profiles per cell and primitive; the union box of a design is mostly
+// outside any one primitive, and there one distance says that its sum is 0.
 __global__ void k_materialize(const MatArgs M) {
   const int d = blockIdx.y;
   const size_t N = (size_t)M.nx * M.ny;
@@ -92,7 +108,7 @@ __global__ void k_materialize(const MatArgs M) {
     double acc = 0.0;
     for (int q = D.p0; q < D.p1; ++q) {
       const MatPrim p = M.prims[q];
-      if (p.height == 0.0) continue;
+      if (p.height == 0.0 || mat_outside(p, M.ox + ((double)c + 0.5) * M.dx, M.oy - ((double)r + 0.5) * M.dy, M.dx, M.dy)) continue;
       double s = 0.0;
       for (int sy = 0; sy < 4; ++sy)
         for (int sx = 0; sx < 4; ++sx) {
@@ -144,30 +160,64 @@ __global__ void k_mat_jumps(const MatArgs M) {
 }
 
 // Cut and fill volumes of each design's edit (design.rs:376-383), summed over its bounding
-// box in row-major order as the reference does. One warp per design: the lanes load 32
-// consecutive cells of a row at once, and every lane runs the sum over them in column order
-// (values broadcast by shuffle), so the f64 sums are the sequential ones, bit for bit.
-__global__ void k_mat_volumes(const MatArgs M) {
-  const int lane = threadIdx.x & 31;
-  const int d = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (d >= M.n) return;   // (whole warps)
+// box in row-major order as the reference does: a chain of f64 additions per volume, bit for bit. What
+// bounds it is that chain, so only it is serial. One block per design takes the box in chunks of
+// kVolChunk cells: every thread loads its cells and forms the products, the ones that are not 0
+// (adding 0 changes nothing) are listed in order by ballots and counts, raised cells from the front and
+// lowered ones from the back, and two threads of different warps add up the two lists while
+// the other warps load the next chunk. With one warp per design walking the
+// whole box, and every sample of every primitive evaluated, the materialisation of 16 designs of
+// 1024 x 1024 took 18.9 ms; now 1.1 ms.
+constexpr int kVolThreads = 512, kVolChunk = 8 * kVolThreads;
+
+__global__ void __launch_bounds__(kVolThreads) k_mat_volumes(const MatArgs M) {
+  __shared__ double list[kVolChunk];
+  __shared__ int count[2][kVolThreads / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, d = blockIdx.x;
   const MatDesign D = M.des[d];
-  const size_t N = (size_t)M.nx * M.ny;
+  const double* dz = M.dz + (size_t)d * M.nx * M.ny;
   const double a = M.dx * M.dy;
-  double cut = 0.0, fill = 0.0;
-  for (int r = D.r0; r < D.r1; ++r)
-    for (int c0 = D.c0; c0 < D.c1; c0 += 32) {
-      const int c = c0 + lane, m = D.c1 - c0 < 32 ? D.c1 - c0 : 32;
-      const double mine = c < D.c1 ? M.dz[(size_t)d * N + (size_t)r * M.nx + c] : 0.0;
-      for (int k = 0; k < m; ++k) {
-        const double v = __shfl_sync(0xffffffffu, mine, k);
-        if (v > 0.0) fill += v * a; else cut -= v * a;
-      }
+  const int w = D.c1 > D.c0 ? D.c1 - D.c0 : 0, h = D.r1 > D.r0 ? D.r1 - D.r0 : 0, total = w * h;   // (at most 2^30 cells)
+  const unsigned below = (1u << lane) - 1u;
+  double sum = 0.0;   // thread 0: fill, thread 32: cut
+  for (int base = 0; base < total; base += kVolChunk) {
+    double p[8];
+    unsigned up[8], dn[8];
+    int nu = 0, nd = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int i = base + 256 * wid + 32 * k + lane;
+      const double v = i < total ? dz[(size_t)(D.r0 + i / w) * M.nx + D.c0 + i % w] : 0.0;
+      p[k] = v * a;
+      up[k] = __ballot_sync(0xffffffffu, p[k] != 0.0 && v > 0.0);
+      dn[k] = __ballot_sync(0xffffffffu, p[k] != 0.0 && !(v > 0.0));
+      nu += __popc(up[k]); nd += __popc(dn[k]);
     }
-  if (lane == 0) {
-    M.cut[d] = cut;
-    M.fill[d] = fill;
+    if (lane == 0) { count[0][wid] = nu; count[1][wid] = nd; }
+    __syncthreads();   // (and the lists of the last chunk are summed)
+    int ou = 0, od = 0, tu = 0, td = 0;
+    for (int q = 0; q < kVolThreads / 32; ++q) {
+      const int cu = count[0][q], cd = count[1][q];
+      if (q < wid) { ou += cu; od += cd; }
+      tu += cu; td += cd;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (up[k] >> lane & 1u) list[ou + __popc(up[k] & below)] = p[k];
+      if (dn[k] >> lane & 1u) list[kVolChunk - 1 - (od + __popc(dn[k] & below))] = p[k];
+      ou += __popc(up[k]); od += __popc(dn[k]);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll 8
+      for (int i = 0; i < tu; ++i) sum += list[i];
+    } else if (threadIdx.x == 32) {
+#pragma unroll 8
+      for (int i = 0; i < td; ++i) sum -= list[kVolChunk - 1 - i];
+    }
   }
+  if (threadIdx.x == 0) M.fill[d] = sum;
+  else if (threadIdx.x == 32) M.cut[d] = sum;
 }
 
 // ---- the design chain of the adjoint: dJ/d(height, width, length) per primitive ----
@@ -237,22 +287,42 @@ struct MatJob {
   int pad;
 };
 
-// One block per primitive: over its box, d(dz)/d(height, width, length) of every editable cell
+// Over a primitive's box, d(dz)/d(height, width, length) of every editable cell
 // whose dz is not clamped, contracted with dJ/d(dz) plus the earthwork weight (the side of 0
-// the cell's dz lies on; the mean of both sides at 0, as a central difference would see it).
+// the cell's dz lies on; the mean of both sides at 0, as a central difference would see it). Bound by
+// f64 divisions and square roots, as k_materialize, and like there most of a slanted box is outside the
+// primitive. Blocks: primitives x slices of the box's cells (few primitives would leave the device
+// idle: mat_dgrad_slices), each slice's sums at part + slice * stride; k_mat_dgrad_sum adds
+// them in order.
+inline int mat_dgrad_slices(int jobs, int sm_count) {
+  const int s = 4 * (sm_count > 0 ? sm_count : 148) / (jobs > 0 ? jobs : 1);
+  return s < 1 ? 1 : s > 64 ? 64 : s;
+}
+__global__ void k_mat_dgrad_sum(const double* part, int slices, int n, double* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double t = 0.0;
+  for (int s = 0; s < slices; ++s) t += part[(size_t)s * n + i];
+  out[i] = t;
+}
+
 __global__ void k_mat_dgrad(const MatArgs M, const MatPrim* jp, const MatJob* jobs, const double* dz, const double* gdz,
-                            double earth_w, double cut_cost, double fill_cost, double* out) {
+                            double earth_w, double cut_cost, double fill_cost, double* part, int stride) {
   const MatJob J = jobs[blockIdx.x];
   const MatPrim p = jp[J.prim];
   const int w = J.c1 - J.c0, h = J.r1 - J.r0;
   const size_t N = (size_t)M.nx * M.ny;
   const double area = M.dx * M.dy;
   double s[3] = {0, 0, 0};
-  for (int k = threadIdx.x; w > 0 && h > 0 && k < w * h; k += blockDim.x) {
-    const int r = J.r0 + k / w, c = J.c0 + k % w;
+  for (long long k = (long long)blockIdx.y * blockDim.x + threadIdx.x; w > 0 && h > 0 && k < (long long)w * h;
+       k += (long long)gridDim.y * blockDim.x) {
+    const int r = J.r0 + (int)(k / w), c = J.c0 + (int)(k % w);
     const size_t i = (size_t)r * M.nx + c;
     const double z = dz[(size_t)J.design * N + i];
     if (!M.editable[i] || !(z > -M.max_abs_dz && z < M.max_abs_dz)) continue;
+    const double we = area * (z > 0.0 ? fill_cost : (z < 0.0 ? -cut_cost : 0.5 * (fill_cost - cut_cost)));
+    const double g = gdz[(size_t)J.design * N + i] + earth_w * we;
+    if (fabs(g) < 1e300 && mat_outside(p, M.ox + ((double)c + 0.5) * M.dx, M.oy - ((double)r + 0.5) * M.dy, M.dx, M.dy)) continue;
     double a0 = 0.0, a1 = 0.0, a2 = 0.0;
     for (int sy = 0; sy < 4; ++sy)
       for (int sx = 0; sx < 4; ++sx) {
@@ -262,8 +332,6 @@ __global__ void k_mat_dgrad(const MatArgs M, const MatPrim* jp, const MatJob* jo
         mat_profile_d(p, x, y, P, dw, dl);
         a0 += P; a1 += dw; a2 += dl;
       }
-    const double we = area * (z > 0.0 ? fill_cost : (z < 0.0 ? -cut_cost : 0.5 * (fill_cost - cut_cost)));
-    const double g = gdz[(size_t)J.design * N + i] + earth_w * we;
     s[0] += g * a0 * (1.0 / 16.0);
     s[1] += g * p.height * a1 * (1.0 / 16.0);
     s[2] += g * p.height * a2 * (1.0 / 16.0);
@@ -278,7 +346,7 @@ __global__ void k_mat_dgrad(const MatArgs M, const MatPrim* jp, const MatJob* jo
     double t[3] = {0, 0, 0};
     for (int q = 0; q < (int)(blockDim.x >> 5); ++q)
       for (int j = 0; j < 3; ++j) t[j] += red[q][j];
-    for (int j = 0; j < 3; ++j) out[J.out + j] = t[j];
+    for (int j = 0; j < 3; ++j) part[(size_t)blockIdx.y * stride + J.out + j] = t[j];
   }
 }
 
