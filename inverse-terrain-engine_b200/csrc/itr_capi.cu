@@ -175,6 +175,8 @@ struct itr_ctx {
   cudaEvent_t ev_fork = nullptr;
   double vjp_fwd_ms = 0, vjp_bwd_ms = 0;
   HostBuf stage, hout;
+  HostBuf ring;                 // fetch_all: two slots
+  cudaEvent_t ev_ring[2] = {nullptr, nullptr};
   // last run
   double kernel_ms = 0, total_ms = 0;
   uint64_t cell_updates = 0;
@@ -485,14 +487,20 @@ static float safe_rate_limit(const RunParams& P, const float* wet, const float* 
   for (int i = 0; i < P.rain.n; ++i) ok = ok && in(P.rain.r[i], -1.0, 1.0);
   for (int g = 0; g < P.inflow.n; ++g)
     for (int i = P.inflow.off[g]; i < P.inflow.off[g + 1]; ++i) ok = ok && in(P.inflow.q[i] * P.inflow.inv_len[g] * P.inflow.scale, -256.0, 256.0);
-  float wl = 0.0f, wh = 0.0f, gl = 0.0f, gh = 0.0f;
-  bool num = true;
+  // (compared as integers, which orders numbers that are not negative, puts NaN above them and vectorises)
+  int wmax = 0, gmax = 0, sign = 0;
   for (size_t i = 0; i < N; ++i) {
-    wl = std::min(wl, wet[i]); wh = std::max(wh, wet[i]);
-    gl = std::min(gl, gn2[i]); gh = std::max(gh, gn2[i]);
-    num = num & (wet[i] == wet[i]) & (gn2[i] == gn2[i]);
+    int w, g;
+    memcpy(&w, wet + i, 4);
+    memcpy(&g, gn2 + i, 4);
+    sign |= w | g;
+    wmax = w > wmax ? w : wmax;
+    gmax = g > gmax ? g : gmax;
   }
-  ok = ok && num && wl >= 0.0f && wh <= 1.0f && gl >= 0.0f && gh <= 1024.0f;
+  float wh, gh;
+  memcpy(&wh, &wmax, 4);
+  memcpy(&gh, &gmax, 4);
+  ok = ok && sign >= 0 && wh <= 1.0f && gh <= 1024.0f;
   if (!ok) return -1.0f;
   const double r = (dt_most + 1e-9 * P.sync) / std::min(P.dx, P.dy);
   if (!(dt_most * gh * 0x1p40 * std::pow(P.h_dry, -7.0 / 3.0) < 0x1p120) || !(r <= 4096.0)) return -1.0f;
@@ -634,6 +642,8 @@ void itr_gpu_destroy(itr_ctx* ctx) {
   ctx->mVol.release();
   ctx->stage.release();
   ctx->hout.release();
+  ctx->ring.release();
+  for (cudaEvent_t e : ctx->ev_ring) if (e) cudaEventDestroy(e);
   for (int i = 0; i < 4; ++i) if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
@@ -874,6 +884,58 @@ static int run_tiled_batch(itr_ctx* ctx, PlainArgs& A, int n, dim3 tgrid, int* l
   return rc;
 }
 
+// One copy from device memory to the caller's: `bytes` at `off` of the allocation `dev`.
+struct Fetch { const char* dev; size_t off; char* host; size_t bytes; };
+
+// Copies device arrays to the caller's (pageable) memory. Straight into it, each array is a synchronous
+// copy of its own through the driver's staging (about 10 us each). Here they stream through two slots of
+// pinned memory: arrays that lie one after the other on the device share a transfer, and a slot's contents are
+// copied out while the other slot fills (32 depths of 45 x 35: 0.75 ms -> 0.1 ms; more threads for the
+// copying out gained nothing below 64 MB). Ends with the stream drained.
+static int fetch_all(itr_ctx* ctx, const std::vector<Fetch>& list) {
+  constexpr size_t kSlotMax = 4u << 20;
+  size_t total = 0;
+  for (const Fetch& f : list) total += f.bytes;
+  const size_t slot = std::min(kSlotMax, align_up(total + 1, 64 << 10));
+  CU(ctx->ring.ensure(2 * slot));
+  for (cudaEvent_t& e : ctx->ev_ring) if (!e) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  struct Piece { char* host; const char* src; size_t bytes; };
+  std::vector<Piece> pieces[2];
+  auto copy_out = [&](int k) -> cudaError_t {
+    const cudaError_t e = cudaEventSynchronize(ctx->ev_ring[k]);
+    if (e != cudaSuccess) return e;
+    for (const Piece& q : pieces[k]) memcpy(q.host, q.src, q.bytes);
+    pieces[k].clear();
+    return cudaSuccess;
+  };
+  size_t i = 0, done = 0;   // next byte to fetch: list[i] from `done`
+  int k = 0;
+  while (i < list.size()) {
+    if (!pieces[k].empty()) CU(copy_out(k));
+    char* base = ctx->ring.as<char>() + (size_t)k * slot;
+    size_t used = 0, run_off = 0, run = 0, src = 0;   // the transfer being collected: run bytes at src of run_dev into run_off
+    const char* run_dev = nullptr;                    // (one allocation: two may be neighbours, and no copy spans them)
+    while (i < list.size() && used < slot) {
+      const Fetch& f = list[i];
+      const size_t b = std::min(f.bytes - done, slot - used);
+      if (!(run > 0 && run_dev == f.dev && src + run == f.off + done)) {
+        if (run > 0) CU(cudaMemcpyAsync(base + run_off, run_dev + src, run, cudaMemcpyDeviceToHost, ctx->stream));
+        run_dev = f.dev; src = f.off + done; run_off = used; run = 0;
+      }
+      if (b > 0) pieces[k].push_back({f.host + done, base + used, b});
+      run += b; used += b; done += b;
+      if (done == f.bytes) { ++i; done = 0; }
+    }
+    if (run > 0) CU(cudaMemcpyAsync(base + run_off, run_dev + src, run, cudaMemcpyDeviceToHost, ctx->stream));
+    CU(cudaEventRecord(ctx->ev_ring[k], ctx->stream));
+    k ^= 1;
+  }
+  for (int q = 0; q < 2; ++q, k ^= 1)
+    if (!pieces[k].empty()) CU(copy_out(k));
+  CU(cudaStreamSynchronize(ctx->stream));
+  return ITR_OK;
+}
+
 // ------------------------------------------------------------------ adjoint ----------
 // Backward sweep after a taped tiled forward (itr_adjoint.cuh): seeds from the monitor
 // maxima and their argmax states, then segment by segment (last first) replay K steps from
@@ -1088,12 +1150,11 @@ static int vjp_backward(itr_ctx* ctx, const PlainArgs& F, const itr_objective* o
     if (b > 0) { rc_ = replay(b - 1); if (rc_ != ITR_OK) return rc_; }
     CU(cudaGetLastError());
   }
-  CU(cudaMemcpyAsync(V->gx, ctx->aGx.p, (size_t)n * SX * 8, cudaMemcpyDeviceToHost, st));
-  CU(cudaMemcpyAsync(V->gy, ctx->aGy.p, (size_t)n * SY * 8, cudaMemcpyDeviceToHost, st));
-  if (crest && V->gx2) CU(cudaMemcpyAsync(V->gx2, ctx->aGx2.p, (size_t)n * SX * 8, cudaMemcpyDeviceToHost, st));
-  if (crest && V->gy2) CU(cudaMemcpyAsync(V->gy2, ctx->aGy2.p, (size_t)n * SY * 8, cudaMemcpyDeviceToHost, st));
-  CU(cudaStreamSynchronize(st));
-  return ITR_OK;
+  std::vector<Fetch> want = {{ctx->aGx.as<char>(), 0, reinterpret_cast<char*>(V->gx), (size_t)n * SX * 8},
+                             {ctx->aGy.as<char>(), 0, reinterpret_cast<char*>(V->gy), (size_t)n * SY * 8}};
+  if (crest && V->gx2) want.push_back({ctx->aGx2.as<char>(), 0, reinterpret_cast<char*>(V->gx2), (size_t)n * SX * 8});
+  if (crest && V->gy2) want.push_back({ctx->aGy2.as<char>(), 0, reinterpret_cast<char*>(V->gy2), (size_t)n * SY * 8});
+  return fetch_all(ctx, want);
 }
 
 // Results of a finished batch: per-design outcomes, monitor maxima, ledgers, J (host), and
@@ -1127,10 +1188,12 @@ static int collect_results(itr_ctx* ctx, const Collect& c) {
   if (max_rows > 0) CU(cudaMemcpyAsync(hled, ctx->ledger.p, (size_t)n * max_rows * 64, cudaMemcpyDeviceToHost, ctx->stream));
   ctx->fallback.assign((size_t)n, -1.0);
   if (ctx->locked_run) CU(cudaMemcpyAsync(ctx->fallback.data(), ctx->lFb.p, (size_t)n * 8, cudaMemcpyDeviceToHost, ctx->stream));
-  for (int d = 0; d < n; ++d) {
-    if (res[d].peak) CU(cudaMemcpyAsync(res[d].peak, ctx->peak.as<float>() + d * N, N * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    if (res[d].depth) CU(cudaMemcpyAsync(res[d].depth, ctx->depth.as<float>() + d * N, N * 4, cudaMemcpyDeviceToHost, ctx->stream));
-  }
+  std::vector<Fetch> want;
+  for (int d = 0; d < n; ++d)
+    if (res[d].peak) want.push_back({ctx->peak.as<char>(), d * N * 4, reinterpret_cast<char*>(res[d].peak), N * 4});
+  for (int d = 0; d < n; ++d)
+    if (res[d].depth) want.push_back({ctx->depth.as<char>(), d * N * 4, reinterpret_cast<char*>(res[d].depth), N * 4});
+  if (!want.empty()) { rc = fetch_all(ctx, want); if (rc != ITR_OK) return rc; }
   CU(cudaEventRecord(ctx->ev[3], ctx->stream));
   CU(cudaStreamSynchronize(ctx->stream));
 #ifdef ITR_CHECKED
@@ -1308,7 +1371,13 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
     if (!M->prims.empty()) memcpy(st + o_mp, M->prims.data(), M->prims.size() * sizeof(MatPrim));
     memcpy(st + o_md, M->des.data(), (size_t)n * sizeof(MatDesign));
   }
-  const float hinit = (float)(p->initial_depth > 0.0 ? p->initial_depth : 0.0);
+  // start depths that no design gives: filled on the device where that is the shorter way (a launch against
+  // writing and uploading n N floats)
+  float hinit = (float)(p->initial_depth > 0.0 ? p->initial_depth : 0.0);
+  if (hinit == 0.0f) hinit = 0.0f;   // (no -0)
+  bool given = false;
+  for (int d = 0; d < n; ++d) given = given || ds[d].h0 != nullptr;
+  const bool fill_h0 = !given && (size_t)n * N >= (64u << 10);
   for (int d = 0; d < n; ++d) {
     if (!M) {
       memcpy(st + o_dzx + d * SX * 4, ds[d].dzx, SX * 4);
@@ -1317,7 +1386,7 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
     if (crest) { memcpy(st + o_dzx2 + d * SX * 4, ds[d].dzx2, SX * 4); memcpy(st + o_dzy2 + d * SY * 4, ds[d].dzy2, SY * 4); }
     float* h0 = reinterpret_cast<float*>(st + o_h0) + d * N;
     if (ds[d].h0) memcpy(h0, ds[d].h0, N * 4);
-    else for (size_t i = 0; i < N; ++i) h0[i] = g->wet[i] != 0.0f ? (hinit == 0.0f ? 0.0f : hinit) : 0.0f;  // init_state
+    else if (!fill_h0) for (size_t i = 0; i < N; ++i) h0[i] = g->wet[i] != 0.0f ? hinit : 0.0f;  // init_state
     reinterpret_cast<double*>(st + o_cut)[d] = ds[d].cut_m3;
     reinterpret_cast<double*>(st + o_fill)[d] = ds[d].fill_m3;
   }
@@ -1341,7 +1410,7 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
   CU(ctx->out.ensure((size_t)n * sizeof(DesignOut)));
   CU(ctx->mmax.ensure((size_t)n * (n_mon > 0 ? n_mon : 1) * 4));
   const size_t out_bytes = (size_t)n * sizeof(DesignOut) + (size_t)n * (n_mon > 0 ? n_mon : 1) * 4 +
-                           (size_t)n * (max_rows > 0 ? max_rows : 1) * 64 + 2 * n * N * 4 + 1024;
+                           (size_t)n * (max_rows > 0 ? max_rows : 1) * 64 + 1024;
   const size_t ctl_bytes = (size_t)n * sizeof(PlainCtl);
   CU(ctx->hout.ensure(out_bytes > ctl_bytes ? out_bytes : ctl_bytes));
 
@@ -1369,8 +1438,22 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
     CU(cudaMemcpyToSymbolAsync(g_itr_err, z, sizeof(z), 0, cudaMemcpyHostToDevice, ctx->stream));
   }
 #endif
-  CU(cudaMemcpyAsync(dv, st, in_bytes, cudaMemcpyHostToDevice, ctx->stream));
   int launches = 0;
+  {   // the parts of the slab that the host filled: not the jumps of designs given as primitives, nor a filled start
+    const size_t cuts[4][2] = {{0, o_dzx}, {o_dzx, M ? o_dzx : o_h0}, {o_h0, fill_h0 ? o_h0 : o_cut}, {o_cut, in_bytes}};
+    size_t lo = 0, hi = 0;
+    for (const auto& c : cuts) {
+      if (c[0] == c[1]) continue;
+      if (c[0] != hi) { if (hi > lo) CU(cudaMemcpyAsync(dv + lo, st + lo, hi - lo, cudaMemcpyHostToDevice, ctx->stream)); lo = c[0]; }
+      hi = c[1];
+    }
+    CU(cudaMemcpyAsync(dv + lo, st + lo, hi - lo, cudaMemcpyHostToDevice, ctx->stream));
+    if (fill_h0) {
+      k_fill_start<<<dim3((unsigned)((N + 255) / 256), (unsigned)std::min(n, 65535)), 256, 0, ctx->stream>>>(
+          reinterpret_cast<const float*>(dv + o_wet), N, n, hinit, reinterpret_cast<float*>(dv + o_h0));
+      launches += 1;
+    }
+  }
   if (M) {   // materialise every design on the device; the volumes come back for J
     CU(ctx->mDz.ensure((size_t)n * N * 8));
     CU(ctx->mZe.ensure((size_t)n * N * 8));
@@ -1472,7 +1555,7 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
     K.bh = has_stage ? reinterpret_cast<const float*>(dv + o_bh) : nullptr;
     K.G = ctx->bG.as<float4>(); K.J = ctx->bJ.as<float4>(); K.J2 = crest ? ctx->bJ2.as<float4>() : nullptr;
     K.never = ctx->bNever.as<unsigned>();
-    k_pack_inputs<<<dim3((unsigned)((rec + 255) / 256), (unsigned)n), 256, 0, ctx->stream>>>(K);
+    k_pack_inputs<<<dim3((unsigned)((rec + 255) / 256), (unsigned)std::min(n, 65535)), 256, 0, ctx->stream>>>(K);
     launches += 1;
     return cudaGetLastError();
   };

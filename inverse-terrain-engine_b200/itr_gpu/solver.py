@@ -211,6 +211,12 @@ def _ptr(a, t):
     return a.ctypes.data_as(C.POINTER(t)) if a is not None else None
 
 
+def _records(struct, n):
+    """n zeroed ctypes records (at least one) and their memory as 8-byte words: (records, uint64, float64)."""
+    w = np.zeros((max(n, 1), C.sizeof(struct) // 8), dtype=np.uint64)
+    return (struct * max(n, 1)).from_buffer(w), w, w.view(np.float64)
+
+
 def _z_edges(base, terrains):
     """Per-design z levels behind the boundary cells, needed when the grid has stage cells."""
     return [t.z_edge() for t in terrains] if getattr(base, "has_stage", False) else None
@@ -335,17 +341,26 @@ class GpuSolver:
             return a
 
         Gd = self._grid(base, arr)
-        D = (_lib.Design * max(n, 1))()
-        for i in range(n):
-            a = arr(dzx[i], np.float32) if dzx[i] is not None else None
-            b = arr(dzy[i], np.float32) if dzy[i] is not None else None
-            a2 = arr(dzx2[i], np.float32) if dzx2 and dzx2[i] is not None else None
-            b2 = arr(dzy2[i], np.float32) if dzy2 and dzy2[i] is not None else None
-            hh = arr(h0[i], np.float32) if h0 and h0[i] is not None else None
-            cut, fill = vols[i] if vols else (0.0, 0.0)
-            ze = arr(z_edge[i], np.float64) if z_edge and z_edge[i] is not None else None
-            D[i] = _lib.Design(_ptr(a, C.c_float), _ptr(b, C.c_float), _ptr(a2, C.c_float), _ptr(b2, C.c_float),
-                               _ptr(hh, C.c_float), cut, fill, _ptr(ze, C.c_double))
+        # the designs' and results' records, filled by column: one ctypes pointer object per field and design
+        # took as long as a small batch's kernel
+        D, Dw, Dv = _records(_lib.Design, n)
+
+        def put(field, arrays, dt):
+            if arrays is not None:
+                col = getattr(_lib.Design, field).offset // 8
+                for i, a in enumerate(arrays):
+                    if a is not None:
+                        Dw[i, col] = arr(a, dt).__array_interface__["data"][0]
+
+        put("dzx", dzx, np.float32)
+        put("dzy", dzy, np.float32)
+        put("dzx2", dzx2, np.float32)
+        put("dzy2", dzy2, np.float32)
+        put("h0", h0, np.float32)
+        put("z_edge", z_edge, np.float64)
+        if vols and n:
+            Dv[:n, _lib.Design.cut_m3.offset // 8] = [v[0] for v in vols]
+            Dv[:n, _lib.Design.fill_m3.offset // 8] = [v[1] for v in vols]
         mon = arr(monitors.cells, np.uint32)
         nm = len(mon)
         O = None
@@ -363,18 +378,19 @@ class GpuSolver:
                                1 if d.require_no_offsite_worsening else 0, 1 if guard_abort else 0,
                                1 if incumbent is not None else 0, float(incumbent or 0.0))
             keep.append(O)
-        R = (_lib.Result * max(n, 1))()
+        R, Rw, _ = _records(_lib.Result, n)
         outs = []
+        mms = np.zeros((max(n, 1), max(nm, 1)), dtype=np.float64)
+        at = {f: getattr(_lib.Result, f).offset // 8 for f in ("monitor_max", "peak", "depth", "ledger", "max_rows")}
+        Rw[:, at["monitor_max"]] = mms.__array_interface__["data"][0] + np.arange(max(n, 1), dtype=np.uint64) * np.uint64(mms.strides[0])
         for i in range(n):
-            mm = np.zeros(max(nm, 1), dtype=np.float64)
             pk = np.zeros(nx * ny, dtype=np.float32) if want_peak else None
             dp = np.zeros(nx * ny, dtype=np.float32) if want_depth else None
             lg = np.zeros((max(ledger_rows, 1), 8), dtype=np.float64) if ledger_rows else None
-            outs.append((mm, pk, dp, lg))
-            R[i].monitor_max = _ptr(mm, C.c_double)
-            R[i].peak = _ptr(pk, C.c_float)
-            R[i].depth = _ptr(dp, C.c_float)
-            R[i].ledger = _ptr(lg, C.c_double)
+            outs.append((mms[i], pk, dp, lg))
+            for f, a in (("peak", pk), ("depth", dp), ("ledger", lg)):
+                if a is not None:
+                    Rw[i, at[f]] = a.__array_interface__["data"][0]
             R[i].max_rows = ledger_rows
         keep += [Gd, D, R]
         return dict(n=n, nx=nx, ny=ny, base=base, Gd=Gd, D=D, mon=mon, nm=nm, O=O, R=R, outs=outs)

@@ -127,3 +127,13 @@ def test_scalar_operations_outside_the_bounds(gpu, name, impl):
     base, p, t = form(name)
     for exact in (0, 1):
         with_options(gpu, {"impl": impl, "exact_special": exact}, lambda: check(gpu, base, p, [t], f"{name} impl {impl} exact {exact}"))
+
+
+def test_more_designs_than_a_grid_extent(gpu):
+    """65535 is the extent of a launch's y and z: the cluster path takes more designs than that."""
+    base, p = scene(3, 2, False)
+    t, n = PreparedTerrain(base), 65535 + 3
+    runs = gpu.run_batch(p, [t] * n, MonitorSet(np.arange(2)))
+    o = orc.flat_run(base_arrays(base), design_dict(t, p), p, MonitorSet(np.arange(2)))
+    for i in (0, 1, 65534, 65535, n - 1):
+        compare_run(runs[i], o, f"design {i}")
