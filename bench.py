@@ -238,9 +238,9 @@ def plain_comparison(g, sc, terrs, n_sample=2):
 
 def adjoint_summary(g, K=128, duration=None, which=4, sweep=()):
     """Config 4 (rolling hills 240x192 @2.5 m, 60 min storm, 32 designs x 4 primitives), or
-    config 5 (fractal 1024x1024 @2 m, 90 min storm, 16 designs x 6 primitives): the autotuned
+    config 5 (fractal 1024x1024 @2 m, 90 min storm, 16 designs x 6 primitives): the default
     forward against itr_gpu_vjp (taped forward + checkpointed backward), device time, both on
-    the second call (the first autotunes and sizes the buffers)."""
+    the second call (the first sizes the buffers)."""
     from itr_gpu.scenes import config
     sc = config(which)
     if duration is not None:
@@ -257,7 +257,7 @@ def adjoint_summary(g, K=128, duration=None, which=4, sweep=()):
         terrs = [t for _, _, t in sc.designs(n)]
         fwd_call = lambda: g.run_batch(sc.params, terrs, sc.monitors, objective=sc.objective, want_depth=False)  # noqa: E731
         vjp_call = lambda k: g.vjp(sc.params, terrs, sc.monitors, sc.objective, checkpoint_interval=k)  # noqa: E731
-    fwd_call()   # autotune
+    fwd_call()   # sizes the buffers
     fwd_call()
     fwd = g.last_timing()["kernel_ms"]
 
@@ -325,7 +325,7 @@ def ladder_summary(g):
         inc = min(r.j for r in g.run_batch(p, prev, sc.monitors, objective=sc.objective, want_depth=False))
         spec.append(dict(terrains=ts, monitors=sc.monitors, objective=sc.objective, baseline_max=base.monitor_max,
                          guard_abort=True, incumbent=inc))
-    g.run_ladder(p, spec)                                        # autotunes each group's shape
+    g.run_ladder(p, spec)                                        # sizes each group's buffers
     out = g.run_ladder(p, spec)
     t = g.last_timing()
     cs = sum(r.cell_updates for o in out for r in o)
@@ -341,7 +341,7 @@ def boundary_summary(g):
     inflow-driven valley at 5 m (90x70; inflow hydrographs on the west and south edges,
     stage on the east and north), 40 min storm, 64 designs on the batched path, beside the
     same designs on the valley with its plain transmissive outlet. Both run twice; the
-    second run (autotuned shape) is timed."""
+    second run is timed."""
     from itr_gpu.scenes import inflow_valley_scene, valley_scene
     out = {}
     for name, sc in (("stage_inflow", inflow_valley_scene(5.0)), ("transmissive_only", valley_scene(5.0))):
@@ -567,15 +567,15 @@ def main():
     ap.add_argument("--designs", type=int, default=64)
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-plain", action="store_true", help="skip the plain one-design-per-launch comparison")
-    ap.add_argument("--cluster", type=int, default=0, help="pin the cluster size (profiling; 0 = autotune)")
-    ap.add_argument("--threads", type=int, default=0, help="pin the threads per CTA (profiling; 0 = autotune)")
+    ap.add_argument("--cluster", type=int, default=0, help="pin the cluster size (profiling; 0 = by the sizes)")
+    ap.add_argument("--threads", type=int, default=0, help="pin the threads per CTA (profiling; 0 = by the sizes)")
     ap.add_argument("--no-adjoint", action="store_true", help="skip the config-4 adjoint summary")
     ap.add_argument("--no-ladder", action="store_true", help="skip the config-3 uneven-batch and stage/inflow summaries")
     ap.add_argument("--workload", type=int, default=2, choices=[2, 4, 5],
                     help="2: the bench workload; 4: the 240x192 scene (32 designs); 5: the 1024x1024 scene (16 designs) "
                          "(4 and 5: measurement / profiling only)")
     ap.add_argument("--impl-path", default="auto", choices=["auto", "tiled", "plain"],
-                    help="profiling: run the main workload on the tiled or plain path instead of the autotuned one")
+                    help="profiling: run the main workload on the tiled or plain path instead of the default one")
     ap.add_argument("--adjoint-only", action="store_true",
                     help="profiling: only the config-4 adjoint (forward + VJP) for --duration seconds of storm; prints its summary")
     ap.add_argument("--set", action="append", default=[], metavar="KEY=VALUE",
@@ -623,7 +623,7 @@ def main():
     N = sc.base.nx * sc.base.ny
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.float32, device="cuda")
 
-    # warm-up through the public call (also autotunes the launch shape)
+    # warm-up through the public call (also sizes the buffers)
     for _ in range(max(args.warmup, 3)):
         runs = g.run_batch(sc.params, terrs, sc.monitors, want_depth=False)
     steps_per_design = [r.steps for r in runs]
