@@ -344,6 +344,15 @@ static LaunchCfg batched_shape(itr_ctx* ctx, int nx, int ny, int n, bool crest, 
   return best;
 }
 
+// Predicted time per step of the tiled path: a launch and the integrator's chain, then a round of the resident
+// blocks (3 per SM) per row of a band and the row computed twice. Fitted to grids of 200x150 .. 300x180 and
+// 1 .. 32 designs, 16 .. 40 us a step, within 8 %.
+static double tiled_step_us(const itr_ctx* ctx, int nx, int ny, int n) {
+  const BandGeom b = band_geom(nx, ny, band_rows_for(nx, ny, n, ctx->sm_count));
+  const double blocks = (double)n * b.gx * b.gy, per_sm = std::min(3.0, std::ceil(blocks / ctx->sm_count));
+  return 8.0 + std::ceil(blocks / (3.0 * ctx->sm_count)) * (b.rows + 1) * (1.1 + 0.23 * per_sm);
+}
+
 // ------------------------------------------------------------------ input checks ------
 constexpr float kMaxInitialDepth = 1e4f;   // m
 
@@ -1667,7 +1676,12 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
       if (!tiled) CU(pack());
     } else {
       cfg = batched_shape(ctx, nx, ny, n, crest, bnd);
-      if (!cfg.ok) cfg.tiled = true;   // a design needs more shared memory than 8 CTAs hold
+      // A design needs more shared memory than 8 CTAs hold, or its strips are so tall (a band of five windows has
+      // one strip) that the whole device sweeping each step is the shorter way: by a margin above both models'
+      // errors. Kernel ms, cluster against tiled, about 600 steps: 250x230 x1 17.0 / 10.1, x16 33.5 / 15.8 (tiled);
+      // 240x192 x1 7.8 / 9.7, x32 22.9 / 22.0, 300x180 x1 10.8 / 9.8, x8 10.9 / 17.9 (cluster). A ladder's groups
+      // are branches of one graph and stay on the cluster kernel.
+      if (!cfg.ok || (!ctx->defer && ctx->band && n <= 65535 && tiled_step_us(ctx, nx, ny, n) < 0.85 * cfg.us)) cfg.tiled = true;
       ctx->tuned[key] = cfg;
       tiled = cfg.tiled;
       if (!tiled) CU(pack());

@@ -79,6 +79,14 @@ def test_cluster_kernel_edges(gpu, nx, ny, bnd):
                          lambda: check(gpu, base, p, terrs[:1], f"{nx}x{ny} {cluster} x {threads}"))
 
 
+@pytest.mark.parametrize("nx,ny,n", [(250, 230, 1), (250, 230, 3), (249, 221, 2), (240, 192, 2)])
+def test_either_side_of_the_path_rule(gpu, nx, ny, n):
+    """Grids whose strips are too tall for the cluster kernel take the tiled path, shorter ones do not: the same bits."""
+    base, p = scene(nx, ny, n == 3)
+    p.duration_s, p.sync_interval_s = 4.0, 2.0
+    check(gpu, base, p, [PreparedTerrain(base)] * n, f"{nx}x{ny} x{n}")
+
+
 def test_refused_shapes(gpu):
     """Cluster shapes are taken and refused by the same lines, whatever layout the kernel has: fewer rows
     than CTAs, fewer threads than one strip, more cells than the shared memory."""
