@@ -129,7 +129,7 @@ __host__ __device__ inline SmemPlan smem_plan(int nr_max, int nx, int S, int W, 
   p.sg = o;  o += (size_t)2 * nr_max * 4;          // west/east wall signs (-1 wall, 1 copy) [2][nr]
   o = align_up(o, 16);
   p.led = o;  o += 4 * 8;                          // f64 totals up to the last sync: infil, fix, in, out
-  p.slot = o; o += 2 * 8;                          // (smax bits, flags) [2 parity]
+  p.slot = o; o += 3 * 8;                          // (smax bits, flags) of a step [3 in turn]
   p.red = o;  o += (size_t)nwarps * 8 * 8;         // f64 reductions at sync points
   p.mbar = o; o += 16;
   p.inf = o;  o += bnd ? (size_t)2 * kMaxInflow * 8 : 0;   // float2 inflow values [2 parity][groups]
@@ -191,7 +191,7 @@ struct Smem {
   float* BY;       // [2 parity][2 side][2 P2]
   float* SG;       // [2 side][nr_max]
   double* LED;     // [4]
-  uint2* slot;     // [2 parity]
+  uint2* slot;     // [3], step n's in slot n mod 3
   double* red;     // [nwarps][8]
   unsigned long long* mbar;
   float2* INF;     // inflow group values [2 parity][kMaxInflow] (stage/inflow grids only)
@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
     sm.SG[i] = A.bc[bc_w + ra + i] == 0 ? -1.0f : 1.0f;
     sm.SG[nr_max + i] = A.bc[bc_e + ra + i] == 0 ? -1.0f : 1.0f;
   }
-  if (tid < 2) sm.slot[tid] = make_uint2(0u, 0u);
+  if (tid < 3) sm.slot[tid] = make_uint2(0u, 0u);
   if (tid < 4) {
     const bool w = WS && q == 0;   // a warm start's totals so far
     sm.LED[tid] = !w ? 0.0 : tid == 0 ? WS->tot_infil : tid == 1 ? WS->tot_fix : tid == 2 ? WS->tot_in : WS->tot_out;
@@ -485,6 +485,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
   const bool always_exact = A.exact != 0u || A.never[d] != 0u;
   bool unsafe = WS ? !(P.cfl <= 0.99 * (double)P.s_safe * dt_cfl) : uns_0;
   int status = 0;
+  int sc = 0;            // the step's slot of the CFL reduction
   unsigned phase = 0u;   // single-CTA designs: phase of the step's closing barrier
   unsigned breach_cell = 0, breach_sync = 0;
   double violation = 0.0, lower_bound = 0.0, volume = WS ? WS->volume : v0, rel_res = WS ? WS->rel_res : 0.0;
@@ -604,7 +605,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
           t = o.t; dt_cfl = o.dt_cfl; s_cur = o.s_cur; acc_rain = o.acc_rain; volume = o.volume; rel_res = o.rel_res;
           step = o.step; sync_index = o.sync_index; n_rows = o.n_rows;
           if (tid < 4) sm.LED[tid] = o.led[tid];
-          if (tid < 2) sm.slot[tid] = make_uint2(0u, 0u);
+          if (tid < 3) sm.slot[tid] = make_uint2(0u, 0u);
           sum_infil = sum_fix = sum_in = sum_out = 0.0;
           seg = 0; have_smax = false;
           next_sync(); rain_at_t(t);
@@ -929,8 +930,8 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
       const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(smax_l));
       const unsigned b = (__any_sync(0xffffffffu, bad_l) ? 1u : 0u) | (__any_sync(0xffffffffu, uns_l) ? 2u : 0u);
       if (lane == 0) {
-        atomicMax(&sm.slot[sp].x, m);
-        if (b) atomicOr(&sm.slot[sp].y, b);
+        atomicMax(&sm.slot[sc].x, m);
+        if (b) atomicOr(&sm.slot[sc].y, b);
       }
       // this strip's edge fluxes of the step (written by this warp)
       const double dt_dy = pl.dt * P.dy;
@@ -961,7 +962,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
     }
     // every CTA's slot, one per lane
     uint2 sl = make_uint2(0u, 0u);
-    if (lane < C) sl = (CLUSTERED ? remote(sm.slot, lane) : sm.slot)[sp];
+    if (lane < C) sl = (CLUSTERED ? remote(sm.slot, lane) : sm.slot)[sc];
     const unsigned smax_bits = __reduce_max_sync(0xffffffffu, sl.x), badv = __reduce_or_sync(0xffffffffu, sl.y);
     if (wid == 0) {
       const double dt_dx = pl.dt * P.dx;
@@ -987,7 +988,11 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
         }
       }
     }
-    if (tid == 0) sm.slot[sp ^ 1] = make_uint2(0u, 0u);
+    // Slots in turn: the one cleared here, step n + 2's, was read after step n - 1's barrier by threads that
+    // have since arrived at step n's, and is next written after step n + 1's, which this thread arrives at
+    // with the clear behind it. (Of two slots, the next step's would be cleared beside its writers.)
+    if (tid == 0) sm.slot[sc == 0 ? 2 : sc - 1] = make_uint2(0u, 0u);
+    sc = sc == 2 ? 0 : sc + 1;
     smax = (double)__uint_as_float(smax_bits);
     have_smax = true;
     step += 1;
