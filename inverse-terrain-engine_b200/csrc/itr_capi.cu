@@ -783,6 +783,9 @@ static int run_plain_design(itr_ctx* ctx, PlainArgs& A, int n_blocks, dim3 grid,
 // per step, driven entirely by the control blocks on the device, so a block of
 // steps_per_submit steps is captured once in a CUDA graph and replayed until every design
 // is done (the host reads the control blocks between replays).
+// The adjoint's kernels on row bands: bit 0 the replay, bit 1 the backward step (option adj_band).
+static int adj_band_bits(const itr_ctx* ctx, size_t N) { return ctx->adj_band >= 0 ? ctx->adj_band : (N >= (size_t(1) << 18) ? 3 : 1); }
+
 // Adjoint request: while set, run_batch takes the tiled path and records a tape.
 struct Vjp {
   int K;                                  // checkpoint interval (steps)
@@ -1077,8 +1080,9 @@ static int vjp_backward(itr_ctx* ctx, const PlainArgs& F, const itr_objective* o
   // blocks k_adj_plan writes for the segment (one buffer per tape).
   // (measured: the band backward step is faster than the tile's on 1024^2 grids, slower on
   //  240 x 192; the band replay is faster on both)
-  const int ab = ctx->adj_band >= 0 ? ctx->adj_band : (N >= (size_t(1) << 18) ? 3 : 1);
+  const int ab = adj_band_bits(ctx, N);
   const bool adj_band = (ab & 1) != 0, adj_step_band = (ab & 2) != 0;
+  if (adj_band && (!F.G || !F.J || (crest && !F.J2))) return fail(ctx, ITR_DEVICE_ERROR, "adjoint: the replay's packed inputs are missing");
   PlainArgs T;
   memset(&T, 0, sizeof(T));
   T.P = F.P; T.nx = nx; T.ny = ny; T.mode = F.mode; T.n_designs = n;
@@ -1613,11 +1617,13 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
       ctx->locked_run = true;
     }
     A.band_rows = band_rows_for(nx, ny, n, ctx->sm_count);
-    if (ctx->band && e == cudaSuccess) {
+    if ((ctx->band || (ctx->vjp && (adj_band_bits(ctx, N) & 1))) && e == cudaSuccess) {   // k_band runs the steps or their replay
       PackArgs K;
       e = pack_inputs(K);
       A.G = K.G; A.J = K.J; A.J2 = K.J2;
-      if (e == cudaSuccess) e = ctx->tArr.ensure((size_t)n * 4);
+    }
+    if (ctx->band && e == cudaSuccess) {
+      e = ctx->tArr.ensure((size_t)n * 4);
       A.arrive = ctx->tArr.as<unsigned>();
     }
     if (ctx->band && P.skip_dry && e == cudaSuccess) {   // dry-row skipping (the storm leaves a rain-free step)

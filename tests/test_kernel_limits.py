@@ -56,3 +56,22 @@ def test_low_wide_grids_with_flowing_edges(gpu, nx, ny, cluster):
     p = SolverParams(40.0, 20.0, rain=Hyetograph.from_mm_h([(0, 300), (20, 100)]), initial_depth=0.12)
     terrs = [PreparedTerrain(base)] * 2
     with_options(gpu, {"cluster": cluster, "threads": 512 if cluster else 0}, lambda: check(gpu, base, p, terrs, f"{nx}x{ny} cluster {cluster}"))
+
+
+@pytest.mark.parametrize("name", ["smooth", "stage_inflow", "crest"])
+def test_gradients_after_a_tiled_forward_on_16x16_tiles(gpu, name):
+    """Option band = 0 (the forward on 16x16 tiles) with the replay and the backward step on row bands or tiles:
+    the row-band replay needs its packed inputs whatever kernel ran the forward."""
+    from test_adjoint_band import CASES
+    p, terrains, obj, K = CASES[name](gpu)
+    grad = lambda: gpu.vjp(p, terrains, obj.monitors, obj, checkpoint_interval=K)
+    want = grad()
+    for ab in (-1, 3, 1, 0):
+        got = with_options(gpu, {"band": 0, "adj_band": ab}, grad, {"band": 1, "adj_band": -1})
+        for i, (a, b) in enumerate(zip(got, want)):
+            assert a.steps == b.steps and a.j == b.j, (name, ab, i)
+            for f in ("dj_ddzx", "dj_ddzy", "dj_ddzx2", "dj_ddzy2"):
+                ga, gb = getattr(a, f, None), getattr(b, f, None)
+                assert (ga is None) == (gb is None)
+                if ga is not None:
+                    assert np.array_equal(np.asarray(ga).view(np.uint64), np.asarray(gb).view(np.uint64)), (name, ab, i, f)
