@@ -93,7 +93,7 @@ __global__ void k_adj_plan(const AdjArgs A, PlainCtl* ctl) {
     c->par = 0;
     c->step = A.step0 + j;
     c->k = step_consts(A.P, sg[0], sg[1]);
-    c->k.exact = sg[3] != 0.0 ? 1u : 0u;
+    c->k.exact = (unsigned)sg[3] & 1u;
     c->pl.dt = sg[0]; c->pl.rain = sg[1]; c->pl.t_new = sg[2] + sg[0]; c->pl.hits = false;
   }
 }

@@ -472,6 +472,7 @@ static RunParams make_run_params(const itr_params* p, const itr_grid* g) {
   P.inv_dx_f = (float)(1.0 / g->dx); P.inv_dy_f = (float)(1.0 / g->dy);
   P.h_dry_f = (float)p->h_dry; P.heps2_f = (float)(p->h_eps * p->h_eps); P.q_min_f = (float)1e-30;
   P.nz = -0.0f;
+  P.adj_scalar = P.h_eps >= 0x1p-31 && P.h_eps <= 1024.0 ? 0u : 1u;   // h_eps^4 in 2^-124 .. 2^40
   P.s_safe = -1.0f;   // safe_rate_limit, where the kernels have a branch-free step
   P.inflow.n = 0;   // build_boundaries fills the groups
   P.inflow.scale = p->inflow_scale;

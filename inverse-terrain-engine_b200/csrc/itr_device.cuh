@@ -67,8 +67,12 @@ ITR_DEV float sqrt_rn(float x) {
 // The special operations of the scalar path: Exact for every operand; Fast without branches, the same
 // bits for operands in the ranges that rcp2 and sqrt2 (below) state, which hold in a step from a
 // bounded state (StepK::exact == 0). Fast::div: a y with y = 1 / b rounded, corrected twice by the
-// exact residual (as div_rn), b in rcp2's range; a small |a| (adjoints at the fringe of their domain
-// of dependence) is scaled by 2^64 and back, which keeps the residual a normal number.
+// exact residual (as div_rn), b in rcp2's range and not above 2^62; a small |a| (adjoints at the fringe of their domain
+// of dependence) is scaled by 2^64 and back, which keeps the residual a normal number. A quotient
+// that overflows, or of an infinity or NaN, is returned before the correction (infinity - infinity); one
+// below 2^-126 is rounded a second time on its way back, and may then lie one 2^-149 beside the IEEE
+// result. The adjoint's divisors: celerities and |q|, 2^-76 .. 2^40; h^2 above h_eps^2; and h_eps^4 up
+// to 4 h_eps^4, which asks for h_eps of 2^-31 or more (RunParams::adj_scalar).
 struct Exact {
   static ITR_DEV float rcp(float x) { return itr::rcp(x); }
   static ITR_DEV float sqrt(float x) { return sqrt_rn(x); }
@@ -89,9 +93,11 @@ struct Fast {
   static ITR_DEV float div(float a, float b) {
     const bool tiny = fabsf(a) < 0x1p-60f;
     const float y = rcp(b), as = a * (tiny ? 0x1p64f : 1.0f);
-    float q = as * y;
-    q = __fmaf_rn(__fmaf_rn(-b, q, as), y, q);
-    return __fmaf_rn(__fmaf_rn(-b, q, as), y, q) * (tiny ? 0x1p-64f : 1.0f);
+    const float q = as * y;
+    const bool finite = fabsf(q) <= 0x1.fffffep127f;
+    float r = __fmaf_rn(__fmaf_rn(-b, q, as), y, q);
+    r = __fmaf_rn(__fmaf_rn(-b, r, as), y, r);
+    return (finite ? r : q) * (tiny ? 0x1p-64f : 1.0f);
   }
 };
 
@@ -397,6 +403,7 @@ struct RunParams {
   float g_f, g_half_f, inv_dx_f, inv_dy_f, h_dry_f, heps2_f, q_min_f;
   double rdx, rdy;   // 1 / dx, 1 / dy rounded (div_rn)
   float nz;   // -0.0f, supplied at run time (see mul2)
+  unsigned adj_scalar;   // 1: the adjoint's divisors leave the range of Fast::div (its backward steps take Exact)
   float s_safe;   // largest wave rate of a state whose step may take the branch-free roots (safe_rate_limit)
 };
 

@@ -28,7 +28,8 @@ static_assert(kTileThreads >= 17 * 16, "one x-face and one y-face per thread");
 // mass fluxes (signed: the reference nets a y-edge over its whole row before splitting it
 // into inflow and outflow, kernel.rs:452-472).
 constexpr int kPart = 7;
-// A step's record for the adjoint: dt, rain, start time, StepK::exact.
+// A step's record for the adjoint: dt, rain, start time, and 1 for StepK::exact + 2 for RunParams::adj_scalar: the
+// replay takes the scalar path where the forward did, the backward step in either case.
 constexpr int kLog = 4;
 // The update kernels ask for 6 resident blocks per SM (32 registers a thread): with the
 // 18x18 halo loads waiting on HBM, more resident warps beat fewer registers (measured +10%).
@@ -530,7 +531,7 @@ ITR_DEV void plain_finalize_steps(const PlainArgs& A, const PlainDesign& D, int 
     plain_plan(A, c, dmin_num(c.dt_cfl, P.dt_max));
     if (D.dt_log) {   // ring of max_log entries, slot step mod max_log
       double* q = D.dt_log + (size_t)(c.step % (unsigned long long)A.max_log) * kLog;
-      q[0] = c.pl.dt; q[1] = c.pl.rain; q[2] = c.t; q[3] = (double)c.k.exact;
+      q[0] = c.pl.dt; q[1] = c.pl.rain; q[2] = c.t; q[3] = (double)(c.k.exact + 2u * P.adj_scalar);
     }
   }
 }

@@ -75,3 +75,50 @@ def test_gradients_after_a_tiled_forward_on_16x16_tiles(gpu, name):
                 assert (ga is None) == (gb is None)
                 if ga is not None:
                     assert np.array_equal(np.asarray(ga).view(np.uint64), np.asarray(gb).view(np.uint64)), (name, ab, i, f)
+
+
+def gradients_agree(a, b, what):
+    """Bit for bit but for quotients below the normal range (2^-149 each, through the sweep's linear factors)."""
+    nonzero = 0
+    for i, (x, y) in enumerate(zip(a, b)):
+        for f in ("dj_ddzx", "dj_ddzy", "dj_ddzx2", "dj_ddzy2"):
+            gx, gy = getattr(x, f, None), getattr(y, f, None)
+            assert (gx is None) == (gy is None)
+            if gx is None:
+                continue
+            gx, gy = np.asarray(gx), np.asarray(gy)
+            assert np.all(np.isfinite(gx)) and np.all(np.isfinite(gy)), (what, i, f, int(np.count_nonzero(~np.isfinite(gx))))
+            assert np.all(np.abs(gx - gy) <= 1e-30), (what, i, f, float(np.max(np.abs(gx - gy))))
+            nonzero += int(np.count_nonzero(gx))
+    assert nonzero > 0, what
+
+
+def half_dry(level):
+    """A slope that a stage covers in part: beyond the shore lies a film far below h_eps (a drizzle of 1e-13 m/s; the
+    adjoint of a cell without any water ends at the infiltration's minimum). Water runs in, so that the
+    assets' peaks come late and the backward sweep covers most steps."""
+    from itr_gpu import Asset, Objective, ObjectiveDef
+    nx, ny = 70 * level, 45 * level
+    base = synthetic_terrain(nx, ny, 5.0 / level, lambda x, y: 2.0 - 0.004 * x + 0.2 * math.sin(y / 15.0) + 0.1 * math.cos(x / 20.0), n=0.03,
+                             segments=[Segment("inflow", "north", (200.0, 320.0), hydrograph=[(0.0, 0.1), (40.0, 0.5)])], level=level)
+    p = SolverParams(40.0, 10.0, rain=Hyetograph([(0.0, 1e-13), (40.0, 1e-13)]), initial_depth=0.0, initial_stage=1.6)
+    t = PreparedTerrain(base)
+    h0 = t.initial_depth(0.0, 1.6).ravel()
+    assert 0.2 < np.mean(h0 == 0.0) < 0.8
+    wet = np.flatnonzero(h0 > 0.05)
+    cells = [int(wet[len(wet) // 4]), int(wet[len(wet) // 2]), int(wet[3 * len(wet) // 4])]
+    return p, [t], Objective(ObjectiveDef([Asset(f"a{i}", [c], float(h0[c]), 1.0 + i) for i, c in enumerate(cells)], []))
+
+
+@pytest.mark.parametrize("h_eps", [1e-5, 1e-9, 1e-10, 1e-11, 1e-14])
+@pytest.mark.parametrize("level", [1, 2])
+def test_backward_step_over_small_h_eps(gpu, level, h_eps):
+    """The velocity map's derivative divides by h_eps^4 and more in shallow and dry cells, below the range of the
+    branch-free reciprocal from h_eps = 2^-31 down: the gradients are those of the scalar operations."""
+    p, terrains, obj = half_dry(level)
+    p.h_eps = h_eps
+    grad = lambda: gpu.vjp(p, terrains, obj.monitors, obj, checkpoint_interval=24)
+    for ab in (0, 1, 3):
+        want = with_options(gpu, {"adj_band": ab, "exact_special": 1}, grad, {"adj_band": -1})
+        got = with_options(gpu, {"adj_band": ab}, grad, {"adj_band": -1})
+        gradients_agree(got, want, f"level {level} h_eps {h_eps} adj_band {ab}")
