@@ -251,7 +251,8 @@ ITR_DEV void adj_band_sweep(const AdjArgs& A, int j, FaceF (*edge)[2 * 32], floa
     }
     return q;
   };
-  const bool xown = (own && col <= nx) || (lane == kAdjOwn + 1 && col == nx);   // owns x-face `col`
+  // owns x-face `col`: its own columns' west faces, and the domain's east face beside the last of them
+  const bool xown = own || (lane >= 2 && lane <= kAdjOwn + 1 && col == nx);
 
   // ---- prologue: rows r0 - 2 .. r0 + 1, the source adjoints of rows r0 - 1 and r0, and the
   //      adjoint of the band's top y-face (r0 - 1 | r0), whose gradient this band owns ----

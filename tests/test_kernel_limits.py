@@ -122,3 +122,29 @@ def test_backward_step_over_small_h_eps(gpu, level, h_eps):
         want = with_options(gpu, {"adj_band": ab, "exact_special": 1}, grad, {"adj_band": -1})
         got = with_options(gpu, {"adj_band": ab}, grad, {"adj_band": -1})
         gradients_agree(got, want, f"level {level} h_eps {h_eps} adj_band {ab}")
+
+
+@pytest.mark.parametrize("nx", [24, 29, 30, 57])
+@pytest.mark.parametrize("level", [1, 2])
+def test_gradient_of_the_east_edge(gpu, level, nx):
+    """The jumps of the domain's east face, whichever lane of the row-band backward step comes upon it (a warp owns
+    29 columns): the same as the 16x16 tiles'."""
+    from itr_gpu import Asset, Objective, ObjectiveDef
+    ny = 16
+    base = synthetic_terrain(nx * level, ny * level, 5.0 / level, lambda x, y: 2.0 - 0.004 * x + 0.1 * math.sin(y / 15.0), n=0.03,
+                             segments=[Segment("transmissive", "east")], level=level)
+    t = PreparedTerrain(base)
+    t.dzx = t.dzx.copy()
+    t.dzx.reshape(ny, nx + 1)[:, nx] = 0.02   # a step up at the outlet
+    p = SolverParams(60.0, 20.0, rain=Hyetograph.from_mm_h([(0, 50), (60, 200)]), initial_depth=0.3)
+    cells = [3 * nx + nx - 2, 9 * nx + nx // 2, 12 * nx + nx - 1]
+    obj = Objective(ObjectiveDef([Asset(f"a{i}", [c], 0.3, 1.0 + i) for i, c in enumerate(cells)], []))
+    grad = lambda: gpu.vjp(p, [t], obj.monitors, obj, checkpoint_interval=16)
+    want = with_options(gpu, {"adj_band": 0}, grad, {"adj_band": -1})[0]
+    assert np.count_nonzero(np.asarray(want.dj_ddzx).reshape(ny, nx + 1)[:, nx]) > 0
+    got = with_options(gpu, {"adj_band": 3}, grad, {"adj_band": -1})[0]
+    for f in ("dj_ddzx", "dj_ddzy", "dj_ddzx2", "dj_ddzy2"):
+        ga, gb = getattr(got, f, None), getattr(want, f, None)
+        assert (ga is None) == (gb is None)
+        if ga is not None:
+            assert np.array_equal(np.asarray(ga).view(np.uint64), np.asarray(gb).view(np.uint64)), (f, float(np.max(np.abs(ga - gb))))
