@@ -27,6 +27,7 @@
 // Crest faces (coarse fidelity levels): two jumps per face, d_l and d_r, each side reduced by
 // its own jump; the gradient comes in both jump arrays.
 #pragma once
+#include <type_traits>
 #include "itr_plain.cuh"
 
 namespace itr {
@@ -366,7 +367,7 @@ ITR_DEV void adj_step_tile(const AdjArgs& A, int j, AdjTile<CREST>& sm) {
   }
   const float* X = A.tape + ((size_t)j * A.n_designs + d) * 3 * N;
   const double* sg = A.seg + ((size_t)d * A.K + j) * kLog;
-  const StepK k = step_consts(A.P, sg[0], sg[1]);
+  const StepK k = step_consts<std::is_same<F, Fast>::value>(A.P, sg[0], sg[1]);
   const float* dzx = A.dzx + d * SX;
   const float* dzy = A.dzy + d * SY;
   const float* dzx2 = CREST ? A.dzx2 + d * SX : nullptr;

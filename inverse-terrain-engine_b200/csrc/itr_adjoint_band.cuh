@@ -162,7 +162,7 @@ ITR_DEV void adj_band_sweep(const AdjArgs& A, int j, FaceF (*edge)[2 * 32], floa
   }
   const float* X = A.tape + ((size_t)j * A.n_designs + d) * 3 * N;
   const double* sg = A.seg + ((size_t)d * A.K + j) * kLog;
-  const StepK k = step_consts(A.P, sg[0], sg[1]);
+  const StepK k = step_consts<std::is_same<F, Fast>::value>(A.P, sg[0], sg[1]);
   const float* dzx = A.dzx + d * SX;
   const float* dzy = A.dzy + d * SY;
   const float* dzx2 = CREST ? A.dzx2 + d * SX : nullptr;

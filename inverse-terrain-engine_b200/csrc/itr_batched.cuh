@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
     t_hit = t_sync - 1e-9 * P.sync;
   };
   auto rain_at_t = [&](double x) {   // (t only grows, but for a locked run's return to its snapshot)
-    while (P.rain_sorted && x > P.rain.seg[seg].end) ++seg;
+    while (P.rain_pieces && x > P.rain.seg[seg].end) ++seg;
     rate_t = rain_piece(P.rain.seg[seg], x);
   };
   next_sync();
@@ -657,7 +657,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
         if (have_smax) dt_cfl = smax > 0.0 ? q_cfl : P.dt_max;
         const double dt_pick = use_lock ? dt_lock : dmin_num(dt_cfl, P.dt_max);
         pl = plan_step_fast(P, t, t_sync, t_hit, dt_pick, rate_t, seg, rare);
-        k = step_consts(P, pl.dt, pl.rain);
+        k = step_consts<true>(P, pl.dt, pl.rain);
         fW = face2<true, CREST>(lh, lu, lv, lc, cur.h, cur.u, cur.v, cur.c, hi2(jc), hi2(jc2), k);
         fN = face2<false, CREST>(above.h, above.u, above.v, above.c, cur.h, cur.u, cur.v, cur.c, lo2(jc), lo2(jc2), k);
       } else {

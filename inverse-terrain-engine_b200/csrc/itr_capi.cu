@@ -464,6 +464,14 @@ static RunParams make_run_params(const itr_params* p, const itr_grid* g) {
     s.rden = 1.0 / s.den;
     s.end = last ? HUGE_VAL : p->rain_t[i];
   }
+  // div_rn needs quotients and residuals in the normal range: the storm's times and rates and the steps' lengths
+  // (cfl over an f32 wave rate, dt_max, what is left to a sync instant) far from its ends
+  auto mid = [](double v, double lo) { v = std::fabs(v); return v >= lo && v <= 1.0 / lo; };   // false for NaN
+  P.rain_pieces = P.rain_sorted && mid(p->cfl, 0x1p-200) && mid(p->dt_max_s, 0x1p-200) && mid(p->sync_interval_s, 0x1p-200) &&
+                  p->duration_s <= 0x1p200;
+  for (int i = 0; i < p->n_rain; ++i)
+    P.rain_pieces = P.rain_pieces && (p->rain_t[i] == 0.0 || mid(p->rain_t[i], 0x1p-200)) &&
+                    (p->rain_rate[i] == 0.0 || mid(p->rain_rate[i], 0x1p-250)) && (P.rain.seg[i].dr == 0.0 || mid(P.rain.seg[i].dr, 0x1p-300));
   // Dry-row skipping can act only on a step without rain: keep it on only when the storm has
   // a rain-free stretch inside the run (no skipping is possible otherwise, and the kernels
   // then leave out its bookkeeping; the results are the same either way).
@@ -492,7 +500,7 @@ static RunParams make_run_params(const itr_params* p, const itr_grid* g) {
 // h_eps^2 and at most 2^81. dt_most: the longest step (dt_max or the locked schedule's longest).
 static float safe_rate_limit(const RunParams& P, const float* wet, const float* gn2, size_t N, bool bnd, double dt_most) {
   auto in = [](double v, double lo, double hi) { return v >= lo && v <= hi; };   // false for NaN
-  bool ok = in(P.g, 0.25, 64.0) && in(P.dx, 1e-3, 1e6) && in(P.dy, 1e-3, 1e6) && in(dt_most, 0.0, 4096.0) && in(P.sync, 0.0, 1e9) &&
+  bool ok = in(P.cfl, 0x1p-200, 0x1p200) && in(P.g, 0.25, 64.0) && in(P.dx, 1e-3, 1e6) && in(P.dy, 1e-3, 1e6) && in(dt_most, 0.0, 4096.0) && in(P.sync, 0.0, 1e9) &&
             in(P.h_dry, 0x1p-24, 1024.0) && in(P.h_eps, 0x1p-48, 1024.0) && in(P.infil, 0.0, 1.0);
   for (int i = 0; i < P.rain.n; ++i) ok = ok && in(P.rain.r[i], -1.0, 1.0);
   for (int g = 0; g < P.inflow.n; ++g)

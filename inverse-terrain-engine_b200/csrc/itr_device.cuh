@@ -396,7 +396,8 @@ struct RunParams {
   double dx, dy, g, area, wet_count;
   uint32_t n_sync;
   int skip_dry;
-  int rain_sorted;   // breakpoints non-decreasing in time: the cursor path is exact
+  int rain_sorted;   // breakpoints non-decreasing in time
+  int rain_pieces;   // ... and all numbers within div_rn's range: one piece at a time is the general integral's bits
   Rain rain;
   Inflow inflow;
   // step-invariant f32 constants (solver.rs:269-285), rounded once on the host
@@ -429,8 +430,8 @@ struct StepPlan {
 // The step's schedule (solver.rs:449-489) as straight-line arithmetic. dt_pick: the dt before the clip to
 // the sync instant t_sync (t_hit: the start from which a step is clipped). The rate at the
 // step's start is known from the step before; while no breakpoint lies inside the step the integral is
-// one trapezoid of the piece `seg`, else (or for an unsorted storm) `rare` is set and the general
-// integral replaces s.rain.
+// one trapezoid of the piece `seg`, else (or for a storm that is not sorted, or whose numbers leave div_rn's
+// range: RunParams::rain_pieces) `rare` is set and the general integral replaces s.rain.
 ITR_DEV double rain_piece(const RainSeg& g, double x) { return g.r0 + div_rn(g.dr * (x - g.t0), g.den, g.rden); }
 ITR_DEV StepPlan plan_step_fast(const RunParams& P, double t, double t_sync, double t_hit, double dt_pick, double rate_t, int seg,
                                 bool& rare) {
@@ -439,19 +440,22 @@ ITR_DEV StepPlan plan_step_fast(const RunParams& P, double t, double t_sync, dou
   s.dt = s.hits ? t_sync - t : dt_pick;
   const double b = t + s.dt;
   s.rain = 0.5 * (rate_t + rain_piece(P.rain.seg[seg], b)) * (b - t);
-  rare = b > P.rain.seg[seg].end || !P.rain_sorted;
+  rare = b > P.rain.seg[seg].end || !P.rain_pieces;
   s.t_new = s.hits ? t_sync : b;
   return s;
 }
 
 // Per-step constants from the host-rounded invariants and this step's dt and rain.
+// BOUNDED: a step whose state and parameters are known to be bounded (StepK::exact 0), and with them dt, dx and dy.
+template <bool BOUNDED = false>
 ITR_DEV StepK step_consts(const RunParams& P, double dt, double rain) {
   StepK k;
   k.g = P.g_f; k.g_half = P.g_half_f; k.inv_dx = P.inv_dx_f; k.inv_dy = P.inv_dy_f;
   k.h_dry = P.h_dry_f; k.heps2 = P.heps2_f; k.q_min = P.q_min_f;
   k.dt = (float)dt;
-  k.dtdx = (float)div_rn(dt, P.dx, P.rdx);
-  k.dtdy = (float)div_rn(dt, P.dy, P.rdy);
+  const bool bounded = BOUNDED || P.s_safe >= 0.0f;   // (div_rn's range)
+  k.dtdx = (float)(bounded ? div_rn(dt, P.dx, P.rdx) : dt / P.dx);
+  k.dtdy = (float)(bounded ? div_rn(dt, P.dy, P.rdy) : dt / P.dy);
   k.rain = (float)rain;
   k.cap = (float)(P.infil * dt);
   k.nz = P.nz;

@@ -394,7 +394,7 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int d, int n_blocks, int fi
 ITR_DEV void plain_plan(const PlainArgs& A, PlainCtl& c, double dt_pick) {
   const RunParams& P = A.P;
   const double t_sync = dmin_num((double)(c.sync_index + 1) * P.sync, P.duration);
-  while (P.rain_sorted && c.t > P.rain.seg[c.seg].end) ++c.seg;
+  while (P.rain_pieces && c.t > P.rain.seg[c.seg].end) ++c.seg;
   bool rare;
   c.pl = plan_step_fast(P, c.t, t_sync, t_sync - 1e-9 * P.sync, dt_pick, rain_piece(P.rain.seg[c.seg], c.t), c.seg, rare);
   if (rare) c.pl.rain = rain_integral(P.rain, c.t, c.t + c.pl.dt);

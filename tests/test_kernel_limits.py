@@ -148,3 +148,17 @@ def test_gradient_of_the_east_edge(gpu, level, nx):
         assert (ga is None) == (gb is None)
         if ga is not None:
             assert np.array_equal(np.asarray(ga).view(np.uint64), np.asarray(gb).view(np.uint64)), (f, float(np.max(np.abs(ga - gb))))
+
+
+RAIN = {"to infinity": [(0.0, 5e-5), (math.inf, 5e-5)], "steps": [(2.0, 0.0), (2.0, 4e-5), (9.0, 4e-5), (9.0, 1e-5)],
+        "vanishing": [(0.0, 0.0), (8.0, 1e-310), (16.0, 1e-310)], "far off": [(-1e300, 3e-5), (0.0, 3e-5), (1e300, 3e-5)]}
+
+
+@pytest.mark.parametrize("impl", [0, 1, 2])
+@pytest.mark.parametrize("name", list(RAIN))
+def test_storms_at_the_ends_of_the_number_range(gpu, name, impl):
+    """Breakpoints at infinity or at one instant, vanishing rates: the storm by its general integral where the
+    piecewise one leaves its range, bit for bit the oracle's."""
+    base = synthetic_terrain(26, 22, 2.0, lambda x, y: 3.0 - 0.01 * x + 0.02 * math.sin(y / 5.0), n=0.03, segments=[Segment("transmissive", "east")])
+    p = SolverParams(16.0, 4.0, rain=Hyetograph(RAIN[name]), initial_depth=0.05)
+    with_options(gpu, {"impl": impl}, lambda: check(gpu, base, p, [PreparedTerrain(base)], f"{name} impl {impl}"))
