@@ -192,7 +192,7 @@ struct itr_ctx {
   PlainArgs last_tiled;
   dim3 last_tgrid;
   int last_band = 1;   // the tiled update kernel of the last tiled batch (option band)
-  // launch shapes by (nx, ny, n_designs, mode)
+  // launch shapes by (nx, ny, n_designs, mode and options that the rule reads)
   std::map<std::tuple<int, int, int, int>, LaunchCfg> tuned;
   cudaGraphExec_t gexec = nullptr;
 };
@@ -680,7 +680,7 @@ int itr_gpu_info(itr_ctx* ctx, char* buf, size_t len) {
     snprintf(buf + k, len - (size_t)k, "; last batch: cluster kernel, %d CTAs x %d threads (%d strips of %d warps)",
              ctx->last_cfg.C, ctx->last_cfg.T, ctx->last_cfg.S, ctx->last_cfg.W);
   else if (k > 0 && (size_t)k < len && ctx->have_last && ctx->last_was_tiled)
-    snprintf(buf + k, len - (size_t)k, "; last batch: tiled path (%s)", ctx->band ? "row bands" : "16x16 tiles");
+    snprintf(buf + k, len - (size_t)k, "; last batch: tiled path (%s)", ctx->last_band ? "row bands" : "16x16 tiles");
   return ITR_OK;
 }
 
@@ -1676,7 +1676,8 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
       A.G = K.G; A.J = K.J; A.J2 = K.J2; A.never = K.never;
       return e;
     };
-    auto key = std::make_tuple(nx, ny, n, (int)g->mode + (bnd ? 2 : 0));
+    // (a kept shape holds for all that its rule reads: the grid, the population, the kernels open to the batch)
+    auto key = std::make_tuple(nx, ny, n, (int)g->mode + (bnd ? 2 : 0) + (ctx->band ? 4 : 0) + (ctx->defer ? 8 : 0));
     if (ctx->cluster > 0 || ctx->threads > 0) {
       const int C = ctx->cluster > 0 ? ctx->cluster : 1, T = ctx->threads > 0 ? ctx->threads : 512;
       if (!shape_accepted(ctx, nx, ny, C, T, crest, bnd))

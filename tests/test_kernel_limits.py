@@ -162,3 +162,29 @@ def test_storms_at_the_ends_of_the_number_range(gpu, name, impl):
     base = synthetic_terrain(26, 22, 2.0, lambda x, y: 3.0 - 0.01 * x + 0.02 * math.sin(y / 5.0), n=0.03, segments=[Segment("transmissive", "east")])
     p = SolverParams(16.0, 4.0, rain=Hyetograph(RAIN[name]), initial_depth=0.05)
     with_options(gpu, {"impl": impl}, lambda: check(gpu, base, p, [PreparedTerrain(base)], f"{name} impl {impl}"))
+
+
+def test_launch_shape_follows_option_band(gpu):
+    """The kernel of a batch follows from its sizes and the options, not from the calls before it: a grid that takes the
+    row bands runs elsewhere once option band is 0, as on a solver that never had it at 1."""
+    base = synthetic_terrain(250, 230, 5.0, lambda x, y: 5.0 + 0.01 * x + 0.1 * math.sin(y / 9.0), n=0.03, segments=[Segment("transmissive", "west")])
+    p = SolverParams(20.0, 10.0, rain=Hyetograph.from_mm_h([(0, 100)]), initial_depth=0.05)
+    terrs, mon = [PreparedTerrain(base)], MonitorSet(np.arange(0, 250 * 230, 991))
+    last = lambda g: g.adapter_info().split("last batch:")[1]
+
+    def run(g):
+        r = g.run_batch(p, terrs, mon, ledger_rows=4)[0]
+        return last(g), r
+
+    fresh = GpuSolver()
+    try:
+        fresh.set_option("band", 0)
+        want, a = run(fresh)
+    finally:
+        fresh.close()
+    first, _ = run(gpu)
+    assert "row bands" in first
+    got, b = with_options(gpu, {"band": 0}, lambda: run(gpu), {"band": 1})
+    assert got == want
+    np.testing.assert_array_equal(a.ledger, b.ledger)
+    assert run(gpu)[0] == first
