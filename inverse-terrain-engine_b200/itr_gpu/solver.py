@@ -345,22 +345,21 @@ class GpuSolver:
         # took as long as a small batch's kernel
         D, Dw, Dv = _records(_lib.Design, n)
 
-        def put(field, arrays, dt):
-            if arrays is not None:
-                col = getattr(_lib.Design, field).offset // 8
-                for i, a in enumerate(arrays):
-                    if a is not None:
-                        Dw[i, col] = arr(a, dt).__array_interface__["data"][0]
+        def put(field, arrays, dt):   # (one array per design: entries past them are not read)
+            col = getattr(_lib.Design, field).offset // 8
+            for i in range(n):
+                if arrays[i] is not None:
+                    Dw[i, col] = arr(arrays[i], dt).__array_interface__["data"][0]
 
         put("dzx", dzx, np.float32)
         put("dzy", dzy, np.float32)
-        put("dzx2", dzx2, np.float32)
-        put("dzy2", dzy2, np.float32)
-        put("h0", h0, np.float32)
-        put("z_edge", z_edge, np.float64)
+        for field, arrays, dt in (("dzx2", dzx2, np.float32), ("dzy2", dzy2, np.float32), ("h0", h0, np.float32),
+                                  ("z_edge", z_edge, np.float64)):
+            if arrays is not None and len(arrays):
+                put(field, arrays, dt)
         if vols and n:
-            Dv[:n, _lib.Design.cut_m3.offset // 8] = [v[0] for v in vols]
-            Dv[:n, _lib.Design.fill_m3.offset // 8] = [v[1] for v in vols]
+            Dv[:n, _lib.Design.cut_m3.offset // 8] = [vols[i][0] for i in range(n)]
+            Dv[:n, _lib.Design.fill_m3.offset // 8] = [vols[i][1] for i in range(n)]
         mon = arr(monitors.cells, np.uint32)
         nm = len(mon)
         O = None
