@@ -188,3 +188,22 @@ def test_launch_shape_follows_option_band(gpu):
     assert got == want
     np.testing.assert_array_equal(a.ledger, b.ledger)
     assert run(gpu)[0] == first
+
+
+@pytest.mark.parametrize("nx,ny", [(161, 133), (40, 300), (1, 40)])
+def test_dry_rows_beside_edges_that_come_alive(gpu, nx, ny):
+    """The row bands' dry-row test on grids with more edge cells than a block has threads, an inflow that starts
+    late and a stage on every side but one: the oracle's rows skipped, and its bits."""
+    dx = 2.0
+    segs = [Segment("inflow", "north", (0.3 * nx * dx, 0.8 * nx * dx), hydrograph=[(0.0, 0.0), (6.0, 0.0), (7.0, 1.5)]),
+            Segment("stage", "south", (0.0, 0.5 * nx * dx), stage_m=0.6), Segment("stage", "east", (0.6 * ny * dx, 0.9 * ny * dx), stage_m=0.02 * ny + 0.2),
+            Segment("inflow", "west", (0.1 * ny * dx, 0.3 * ny * dx), hydrograph=[(0.0, 0.0), (12.0, 0.0), (13.0, 0.5)])]
+    base = synthetic_terrain(nx, ny, dx, lambda x, y: 0.02 * y + 0.1 * math.sin(x / 7.0) + 0.1, n=0.03, segments=segs)
+    p = SolverParams(20.0, 5.0, dt_max_s=0.1, rain=Hyetograph([]), initial_depth=0.0)
+    t, mon = PreparedTerrain(base), MonitorSet(np.arange(0, nx * ny, 5))
+    o = orc.flat_run(base_arrays(base), design_dict(t, p), p, mon, want_peak=True, bnd=orc.bnd_dict(base, t))
+    assert o["rows_skipped"] > 0
+    r = with_options(gpu, {"impl": 2}, lambda: gpu.run_batch(p, [t, t], mon, want_peak=True))
+    for i in range(2):
+        compare_run(r[i], o, f"{nx}x{ny} design {i}")
+        assert r[i].rows_skipped == o["rows_skipped"]
