@@ -336,6 +336,10 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int d, int n_blocks, int fi
   const PlainDesign D = plain_design(A, d, n_blocks);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const RunParams& P = A.P;
+  if (!first && *(const volatile int*)&D.ctl->done) {   // a finished design (the steps left of a submitted block)
+    if constexpr (LOCKED) { if (threadIdx.x == 0) D.ctl->copy_req = 0; }   // the last request has been served
+    return;
+  }
   constexpr int kWords = sizeof(PlainCtl) / 8;
   const volatile unsigned long long* src = reinterpret_cast<const volatile unsigned long long*>(D.ctl);
   for (int i = threadIdx.x; i < kWords; i += blockDim.x) reinterpret_cast<unsigned long long*>(&c)[i] = first ? 0ull : src[i];
@@ -343,9 +347,16 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int d, int n_blocks, int fi
   for (int j = wid; j < kPart; j += nw) {
     const bool is_max = first && j > 0;   // (the start's partials: volume, then maxima)
     double t = 0.0;
-    for (int b = lane; b < n_blocks; b += 32) {
-      const double v = first && j > 3 ? 0.0 : __ldcg(D.part + (size_t)b * kPart + j);
-      t = is_max ? (t > v ? t : v) : t + v;
+    for (int b0 = lane; b0 < n_blocks; b0 += 32 * 8) {   // eight loads in flight, added in block order
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int b = b0 + 32 * u;
+        v[u] = b < n_blocks && !(first && j > 3) ? __ldcg(D.part + (size_t)b * kPart + j) : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (b0 + 32 * u < n_blocks) t = is_max ? (t > v[u] ? t : v[u]) : t + v[u];
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -371,12 +382,6 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int d, int n_blocks, int fi
     if (sums[3] > 0.0) c.unsafe |= 2u;
   }
   __syncthreads();
-  const bool was_done = c.done != 0;
-  __syncthreads();   // read by every warp before warp 0 goes on to change it
-  if (was_done) {
-    if constexpr (LOCKED) { if (threadIdx.x == 0) D.ctl->copy_req = 0; }   // the last request has been served
-    return;
-  }
   if (!first && D.rowwet) {
     // dry rows the step just skipped (k_band's predicate on the flags it read: the state of
     // parity c.par, not yet flipped), then clear those flags: the next step writes them

@@ -207,3 +207,20 @@ def test_dry_rows_beside_edges_that_come_alive(gpu, nx, ny):
     for i in range(2):
         compare_run(r[i], o, f"{nx}x{ny} design {i}")
         assert r[i].rows_skipped == o["rows_skipped"]
+
+
+@pytest.mark.parametrize("nx,ny", [(16, 16), (512, 16), (528, 16), (256, 256), (4112, 16), (500, 400)])
+def test_tile_partials_of_many_blocks(gpu, nx, ny):
+    """The step's sums over the 16x16 tiles' partials, block counts around 32 and 256: the oracle's bits, and the
+    ledgers of the row bands (f64 sums of the same terms in another order)."""
+    base = synthetic_terrain(nx, ny, 2.0, lambda x, y: 3.0 + 0.02 * math.sin(x / 5.0) - 0.001 * y, n=0.035,
+                             segments=[Segment("transmissive", "south"), Segment("inflow", "north", (0.0, nx), hydrograph=[(0.0, 0.5), (4.0, 1.0)])])
+    p = SolverParams(4.0, 2.0, rain=Hyetograph.from_mm_h([(0, 300), (4, 100)]), initial_depth=0.12, infil_capacity=1e-5)
+    t, mon = PreparedTerrain(base), MonitorSet(np.arange(0, nx * ny, 5))
+    o = orc.flat_run(base_arrays(base), design_dict(t, p), p, mon, want_peak=True, bnd=orc.bnd_dict(base, t))
+    go = lambda: gpu.run_batch(p, [t], mon, want_peak=True, ledger_rows=4)
+    ref = with_options(gpu, {"impl": 2}, go)[0]
+    for opts in ({"impl": 1}, {"impl": 2, "band": 0}):
+        r = with_options(gpu, opts, go, {"band": 1})[0]
+        compare_run(r, o, f"{nx}x{ny} {opts}")
+        np.testing.assert_allclose(r.ledger, ref.ledger, rtol=1e-12, atol=1e-9)
