@@ -759,10 +759,12 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
       if (lane == 0 && wis == 0) atomicAdd(sm.NSK, 1ull);   // once per skipped row (rain-free steps only)
     };
     // x_boundary (kernel.rs:435-450): mass flux of the west and east domain faces
-    const bool bx_w = wis == 0 && lane == 1, bx_e = east_g || east_y;
+    // (one lane has both of a single column's)
+    const bool bx_w = wis == 0 && lane == 1, bx_e = east_g || east_y, bx_2 = bx_w && bx_e, sec = east_y && !bx_w;
     float* const bx = sm.BX + (bx_w ? 0 : nr_max);
     auto put_edges = [&](int lr, const Face2& f) {
-      if (bx_w || bx_e) bx[lr] = east_y ? f.m.y : f.m.x;
+      if (bx_w || bx_e) bx[lr] = sec ? f.m.y : f.m.x;
+      if (bx_2) bx[nr_max + lr] = f.m.y;
     };
     // The update of one row on the scalar path: lanes' idle columns are left out one by one (in an
     // unbounded state their values need not be finite).

@@ -240,7 +240,7 @@ static LaunchCfg make_cfg(const itr_ctx* ctx, int nx, int ny, int C, int T_targe
   c.C = C;
   c.bnd = bnd;
   c.W = windows(nx);   // warps per strip row
-  if (C < 1 || ny < C || nx < 2) return c;   // (one column: its west and east faces share a lane; the tiled path takes it)
+  if (C < 1 || ny < C) return c;
   const int nr_min = ny / C, nr_max = (ny + C - 1) / C;
   int S = std::min(T_target, 512) / (32 * c.W);   // (more threads leave too few registers each: below)
   if (S > nr_min) S = nr_min;

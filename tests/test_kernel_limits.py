@@ -224,3 +224,31 @@ def test_tile_partials_of_many_blocks(gpu, nx, ny):
         r = with_options(gpu, opts, go, {"band": 1})[0]
         compare_run(r, o, f"{nx}x{ny} {opts}")
         np.testing.assert_allclose(r.ledger, ref.ledger, rtol=1e-12, atol=1e-9)
+
+
+@pytest.mark.parametrize("rain", [True, False])
+@pytest.mark.parametrize("level", [1, 2])
+@pytest.mark.parametrize("ny,cluster", [(1, 1), (9, 0), (9, 8), (40, 2), (300, 0), (301, 8)])
+def test_single_column_on_the_cluster_kernel(gpu, ny, cluster, level, rain):
+    """One column: its west and east faces, both flowing, belong to one lane. The oracle's bits, and the ledger's
+    inflow and outflow as on the tiled path."""
+    dx = 2.0
+    segs = [Segment("inflow", "west", hydrograph=[(0.0, 0.02), (30.0, 0.1)]), Segment("transmissive", "east"), Segment("transmissive", "south")]
+    base = synthetic_terrain(level, ny * level, dx / level, lambda x, y: 3.0 + 0.02 * math.cos(y / 7.0) - 0.01 * x, n=0.035, segments=segs, level=level)
+    assert base.nx == 1
+    p = SolverParams(24.0, 8.0, rain=Hyetograph.from_mm_h([(0, 0), (5, 300), (15, 0)] if rain else []), infil_capacity=2e-6, initial_depth=0.12 if rain else 0.0)
+    terrs, mon = [PreparedTerrain(base)] * 3, MonitorSet(np.arange(0, ny, 2))
+    ref = with_options(gpu, {"impl": 2}, lambda: gpu.run_batch(p, terrs, mon, ledger_rows=4))
+    o = orc.flat_run(base_arrays(base), design_dict(terrs[0], p), p, mon, want_peak=True, bnd=orc.bnd_dict(base, terrs[0]))
+
+    def run():
+        r = gpu.run_batch(p, terrs, mon, want_peak=True, ledger_rows=4)
+        assert "cluster kernel" in gpu.adapter_info()
+        return r
+
+    for r, a in zip(with_options(gpu, {"cluster": cluster, "threads": 128 if cluster else 0}, run), ref):
+        compare_run(r, o, f"1x{ny} cluster {cluster}")
+        assert r.rows_skipped == a.rows_skipped
+        # (time, volume, rain, inflow, outflow: f64 sums; the infiltration of a step is summed in f32, in another order)
+        np.testing.assert_allclose(r.ledger[:, :5], a.ledger[:, :5], rtol=1e-12, atol=1e-12)
+        assert np.all(r.ledger[:, 3:5] > 0.0)
