@@ -73,6 +73,7 @@ struct LaunchCfg {
   size_t smem = 0;
   bool ok = false;
   bool tiled = false;   // the tiled HBM path instead
+  bool tiles = false;   // ... on 16x16 tiles, not on row bands
   bool bnd = false;     // the grid has stage or inflow cells (k_batched<..., BND>)
   double us = 0.0;      // predicted time of a step
 };
@@ -344,13 +345,36 @@ static LaunchCfg batched_shape(itr_ctx* ctx, int nx, int ny, int n, bool crest, 
   return best;
 }
 
-// Predicted time per step of the tiled path: a launch and the integrator's chain, then a round of the resident
-// blocks (3 per SM) per row of a band and the row computed twice. Fitted to grids of 200x150 .. 300x180 and
-// 1 .. 32 designs, 16 .. 40 us a step, within 8 %.
-static double tiled_step_us(const itr_ctx* ctx, int nx, int ny, int n) {
+// Predicted time per step of the chosen cluster shape, for the comparison with the tiled path: as batched_shape, but
+// with whole warps per scheduler (9 warps take the time of 12) and 1.28 of a row's time for blocks above 384 threads.
+// Within 5 % on grids of 60x50 .. 900x40 and 1 .. 32 designs.
+static double cluster_step_us(const itr_ctx* ctx, const LaunchCfg& c, int ny, int n, int act) {
+  const int ctas = std::min(n, act) * c.C, per_sm = (ctas + ctx->sm_count - 1) / ctx->sm_count;
+  const double w = std::max(1.0, std::ceil(per_sm * c.T / 128.0)), rows = std::ceil(std::ceil((double)ny / c.C) / c.S);
+  const double r = c.T <= 256 ? 0.75 * (1.0 + 0.25 * (w - 1.0)) : (c.T <= 384 ? 0.8625 : 1.104) * (1.0 + 0.3 * (w - 1.0));
+  return std::ceil((double)n / act) * ((c.C > 1 ? 1.5 : 0.9) + (rows + 0.5) * r);
+}
+
+// Predicted time per step of the row bands: a launch and the integrator's chain (longer where a block has one warp),
+// then a round of the resident warps (12 per SM) per row of a band and the row computed twice. Within 12 % on grids of
+// 60x900 .. 1980x8 and 1 .. 100 designs, 14 .. 45 us a step. Locked dt takes two more launches.
+static double tiled_step_us(const itr_ctx* ctx, int nx, int ny, int n, bool locked) {
   const BandGeom b = band_geom(nx, ny, band_rows_for(nx, ny, n, ctx->sm_count));
-  const double blocks = (double)n * b.gx * b.gy, per_sm = std::min(3.0, std::ceil(blocks / ctx->sm_count));
-  return 8.0 + std::ceil(blocks / (3.0 * ctx->sm_count)) * (b.rows + 1) * (1.1 + 0.23 * per_sm);
+  const double blocks = (double)n * b.gx * b.gy, warps = blocks * b.wpb / ctx->sm_count, sched = std::min(3.0, std::ceil(warps / 4.0));
+  const double rounds = std::ceil(blocks / (12 / b.wpb * ctx->sm_count));
+  return (locked ? 11.5 : 8.0) + (b.wpb == 1 ? 3.5 : 0.0) + rounds * (std::min(b.rows, ny) + 1) * (1.1 + 0.23 * sched);
+}
+
+// A step of 16x16 tiles as one launch, whose last block advances the integrator, where its larger blocks (3 an SM)
+// run in one round: above, the update alone at 6 blocks an SM and a finalize are faster (us a step, one launch
+// against two: 228 tiles 11.0 / 12.8, 442 12.3 / 14.1, 504 14.5 / 13.6, 992 19.3 / 16.9).
+static bool tile_fin(const itr_ctx* ctx, long long tiles) { return tiles <= 3LL * ctx->sm_count; }
+
+// Predicted time per step of the 16x16 tiles: within 5 % of 9.7 .. 50 us on grids of 60x50 .. 1980x8 and 1 .. 32 designs.
+static double tile_step_us(const itr_ctx* ctx, int nx, int ny, int n, bool locked) {
+  const long long tiles = (long long)n * ((nx + kTile - 1) / kTile) * ((ny + kTile - 1) / kTile);
+  const bool fin = tile_fin(ctx, tiles) && !locked;
+  return (fin ? 9.8 : locked ? 15.0 : 11.5) + tiles * (148.0 / ctx->sm_count) * (fin ? 0.0055 : 0.0083);
 }
 
 // ------------------------------------------------------------------ input checks ------
@@ -731,14 +755,15 @@ int itr_gpu_last_timing(itr_ctx* ctx, double* kernel_ms, double* total_ms, uint6
 // ------------------------------------------------------------------ plain path ------
 // One step's update kernel of the tiled path: the ghost rule with stage and inflow cells
 // only where the grid has them.
+template <bool FIN = false>
 static void launch_update(const PlainArgs& A, dim3 grid, cudaStream_t st) {
   const bool bnd = A.bh != nullptr || A.P.inflow.n > 0;
   if (A.mode == 1) {
-    if (bnd) k_plain_update<true, true><<<grid, kTileThreads, 0, st>>>(A);
-    else k_plain_update<true, false><<<grid, kTileThreads, 0, st>>>(A);
+    if (bnd) k_plain_update<true, true, FIN><<<grid, kTileThreads, 0, st>>>(A);
+    else k_plain_update<true, false, FIN><<<grid, kTileThreads, 0, st>>>(A);
   } else {
-    if (bnd) k_plain_update<false, true><<<grid, kTileThreads, 0, st>>>(A);
-    else k_plain_update<false, false><<<grid, kTileThreads, 0, st>>>(A);
+    if (bnd) k_plain_update<false, true, FIN><<<grid, kTileThreads, 0, st>>>(A);
+    else k_plain_update<false, false, FIN><<<grid, kTileThreads, 0, st>>>(A);
   }
 }
 
@@ -758,8 +783,8 @@ static void launch_band(const PlainArgs& A, dim3 grid, cudaStream_t st, int fin)
 }
 
 // Blocks per design of the tiled path's update (the finalize's partials).
-static dim3 tiled_grid(const itr_ctx* ctx, int nx, int ny, int n) {
-  if (!ctx->band) return dim3((nx + kTile - 1) / kTile, (ny + kTile - 1) / kTile);
+static dim3 tiled_grid(const itr_ctx* ctx, int nx, int ny, int n, bool band) {
+  if (!band) return dim3((nx + kTile - 1) / kTile, (ny + kTile - 1) / kTile);
   const BandGeom bg = band_geom(nx, ny, band_rows_for(nx, ny, n, ctx->sm_count));
   return dim3((unsigned)bg.gx, (unsigned)bg.gy);
 }
@@ -806,7 +831,8 @@ struct Vjp {
   double* gy2 = nullptr;
 };
 
-static int run_tiled_batch(itr_ctx* ctx, PlainArgs& A, int n, dim3 tgrid, int* launches) {
+// band: row bands (k_band), else 16x16 tiles.
+static int run_tiled_batch(itr_ctx* ctx, PlainArgs& A, int n, dim3 tgrid, bool band, int* launches) {
   const int nb = (int)(tgrid.x * tgrid.y);
   const dim3 grid(tgrid.x, tgrid.y, (unsigned)n);
   const cudaStream_t st = ctx->stream;
@@ -828,11 +854,12 @@ static int run_tiled_batch(itr_ctx* ctx, PlainArgs& A, int n, dim3 tgrid, int* l
   }
   *launches += 2;
   const int K = tape ? tape->K : ctx->steps_per_submit;
+  const bool fin = !locked && (band || tile_fin(ctx, (long long)n * nb));   // the step's kernel advances the integrators too
   if (tape) { tape->dt.assign(n, std::vector<double>()); tape->blocks = 0; }
   auto block = [&]() {
     for (int s = 0; s < K; ++s) {
-      const bool fin = ctx->band && !locked;   // the band kernel advances the integrators too
-      if (ctx->band) launch_band<false>(A, grid, st, fin ? 1 : 0);
+      if (band) launch_band<false>(A, grid, st, fin ? 1 : 0);
+      else if (fin) launch_update<true>(A, grid, st);
       else launch_update(A, grid, st);
       if (fin) continue;
       if (locked) {
@@ -881,7 +908,7 @@ static int run_tiled_batch(itr_ctx* ctx, PlainArgs& A, int n, dim3 tgrid, int* l
     }
     if (ge) { const cudaError_t e = cudaGraphLaunch(ge, st); if (e != cudaSuccess) { rc = fail(ctx, ITR_DEVICE_ERROR, "cudaGraphLaunch: %s", cudaGetErrorString(e)); break; } }
     else block();
-    *launches += (locked ? 3 : ctx->band ? 1 : 2) * K;
+    *launches += (locked ? 3 : fin ? 1 : 2) * K;
     cudaError_t e = cudaMemcpyAsync(hc, A.ctl, (size_t)n * sizeof(PlainCtl), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) { rc = fail(ctx, ITR_DEVICE_ERROR, "tiled run: %s", cudaGetErrorString(e)); break; }
@@ -1556,7 +1583,9 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
 
   // impl 2, or a grid no cluster shape can hold: the tiled batched path (state in HBM)
   bool tiled = ctx->impl == 2 || ctx->vjp != nullptr;
-  dim3 tgrid = tiled_grid(ctx, nx, ny, n);   // blocks per design of the tiled path's update
+  bool tiles = false;             // ... where the rule takes it, on 16x16 tiles
+  bool band = ctx->band != 0;   // the tiled path's kernel
+  dim3 tgrid = tiled_grid(ctx, nx, ny, n, band);   // blocks per design of the tiled path's update
   int n_tiles = (int)(tgrid.x * tgrid.y);
   const int max_tiles = std::max((nx + kTile - 1) / kTile * ((ny + kTile - 1) / kTile), n_tiles);
   const bool bnd_grid = has_stage || P.inflow.n > 0;   // stage or inflow ghosts
@@ -1626,16 +1655,16 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
       ctx->locked_run = true;
     }
     A.band_rows = band_rows_for(nx, ny, n, ctx->sm_count);
-    if ((ctx->band || (ctx->vjp && (adj_band_bits(ctx, N) & 1))) && e == cudaSuccess) {   // k_band runs the steps or their replay
+    if ((band || (ctx->vjp && (adj_band_bits(ctx, N) & 1))) && e == cudaSuccess) {   // k_band runs the steps or their replay
       PackArgs K;
       e = pack_inputs(K);
       A.G = K.G; A.J = K.J; A.J2 = K.J2;
     }
-    if (ctx->band && e == cudaSuccess) {
+    if (e == cudaSuccess) {
       e = ctx->tArr.ensure((size_t)n * 4);
       A.arrive = ctx->tArr.as<unsigned>();
     }
-    if (ctx->band && P.skip_dry && e == cudaSuccess) {   // dry-row skipping (the storm leaves a rain-free step)
+    if (band && P.skip_dry && e == cudaSuccess) {   // dry-row skipping (the storm leaves a rain-free step)
       const size_t R = (size_t)ny + 2;
       e = ctx->tRow.ensure((size_t)n * 2 * R * 4);
       if (e == cudaSuccess && bnd_grid) e = ctx->tGw.ensure((size_t)n * R);
@@ -1677,7 +1706,8 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
       return e;
     };
     // (a kept shape holds for all that its rule reads: the grid, the population, the kernels open to the batch)
-    auto key = std::make_tuple(nx, ny, n, (int)g->mode + (bnd ? 2 : 0) + (ctx->band ? 4 : 0) + (ctx->defer ? 8 : 0));
+    auto key = std::make_tuple(nx, ny, n, (int)g->mode + (bnd ? 2 : 0) + (ctx->band ? 4 : 0) + (ctx->defer ? 8 : 0) + (locked ? 16 : 0) +
+                               (P.skip_dry ? 32 : 0));
     if (ctx->cluster > 0 || ctx->threads > 0) {
       const int C = ctx->cluster > 0 ? ctx->cluster : 1, T = ctx->threads > 0 ? ctx->threads : 512;
       if (!shape_accepted(ctx, nx, ny, C, T, crest, bnd))
@@ -1688,18 +1718,24 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
       if (!tiled) CU(pack());
     } else if (ctx->tuned.count(key)) {
       cfg = ctx->tuned[key];
-      tiled = cfg.tiled;
+      tiled = cfg.tiled; tiles = cfg.tiles;
       if (!tiled) CU(pack());
     } else {
       cfg = batched_shape(ctx, nx, ny, n, crest, bnd);
       // A design needs more shared memory than 8 CTAs hold, or its strips are so tall (a band of five windows has
-      // one strip) that the whole device sweeping each step is the shorter way: by a margin above both models'
-      // errors. Kernel ms, cluster against tiled, about 600 steps: 250x230 x1 17.0 / 10.1, x16 33.5 / 15.8 (tiled);
-      // 240x192 x1 7.8 / 9.7, x32 22.9 / 22.0, 300x180 x1 10.8 / 9.8, x8 10.9 / 17.9 (cluster). A ladder's groups
-      // are branches of one graph and stay on the cluster kernel.
-      if (!cfg.ok || (!ctx->defer && ctx->band && n <= 65535 && tiled_step_us(ctx, nx, ny, n) < 0.85 * cfg.us)) cfg.tiled = true;
+      // one strip) that the whole device sweeping each step is the shorter way: few designs on 16x16 tiles, which
+      // spread a step over the most threads, more on row bands, by margins for the models' errors. us a step, cluster /
+      // bands / tiles: 300x180 x1 18.9 / 17.1 / 10.9, x4 19.1 / 18.1 / 18.4, x8 19.2 / 31.2 / 26.6; 250x230 x1 29.2 / 16.8 /
+      // 10.7, x16 58.5 / 26.4 / 44.2; 60x900 x1 16.1 / 20.8 / 10.8; 180x140 x1 9.0 / 17.1 / 9.9. A ladder's groups are
+      // branches of one graph and stay on the cluster kernel; the tiles do not skip dry rows.
+      const bool open = !ctx->defer && n <= 65535;
+      const double cl = cfg.ok ? cluster_step_us(ctx, cfg, ny, n, std::max(1, max_active_clusters(ctx, cfg, crest))) : HUGE_VAL;
+      const double bd = ctx->band ? tiled_step_us(ctx, nx, ny, n, locked) : HUGE_VAL;
+      const double tl = P.skip_dry ? HUGE_VAL : tile_step_us(ctx, nx, ny, n, locked);
+      cfg.tiled = !cfg.ok || (open && std::min(bd / 0.85, tl / 0.96) < cl);
+      cfg.tiles = cfg.tiled && (!ctx->band || (open && tl < 0.92 * bd && tl < 0.96 * cl));
       ctx->tuned[key] = cfg;
-      tiled = cfg.tiled;
+      tiled = cfg.tiled; tiles = cfg.tiles;
       if (!tiled) CU(pack());
     }
     if (!tiled) {
@@ -1744,6 +1780,8 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
   }
   if (tiled) {
     PlainArgs A;
+    band = ctx->band && !tiles;
+    tgrid = tiled_grid(ctx, nx, ny, n, band);
     CU(tiled_args(A));
     if (ctx->vjp) {
       const int K = ctx->vjp->K;
@@ -1755,8 +1793,8 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
       A.max_log = 2 * K;
     }
     CU(cudaEventRecord(ctx->ev[1], ctx->stream));
-    rc = run_tiled_batch(ctx, A, n, tgrid, &launches);
-    ctx->last_band = ctx->band;
+    rc = run_tiled_batch(ctx, A, n, tgrid, band, &launches);
+    ctx->last_band = band;
     if (rc != ITR_OK) return rc;
     k_plain_outputs<<<dim3((unsigned)plain_blocks(nx, ny, n), (unsigned)n), 256, 0, ctx->stream>>>(A, ctx->out.as<DesignOut>(), ctx->depth.as<float>());
     launches += 1;
@@ -2296,10 +2334,7 @@ extern "C" int itr_gpu_rerun_resident(itr_ctx* ctx) {
   CU(cudaEventRecord(ctx->ev[1], ctx->stream));
   if (ctx->last_was_tiled) {
     PlainArgs A = ctx->last_tiled;
-    const int band = ctx->band;
-    ctx->band = ctx->last_band;   // the kernel its partials were laid out for
-    int rc = run_tiled_batch(ctx, A, A.n_designs, ctx->last_tgrid, &launches);
-    ctx->band = band;
+    int rc = run_tiled_batch(ctx, A, A.n_designs, ctx->last_tgrid, ctx->last_band != 0, &launches);
     if (rc != ITR_OK) return rc;
   } else if (!ctx->last_was_plain) {
     int rc = launch_batched(ctx, ctx->last_args, ctx->last_cfg, ctx->last_args.n_designs);

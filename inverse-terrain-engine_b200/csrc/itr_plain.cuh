@@ -205,8 +205,13 @@ ITR_DEV void plain_load(const PlainArgs& A, const PlainDesign& D, int par, int g
   }
 }
 
-template <bool CREST, bool BND = false>
-__global__ void __launch_bounds__(kTileThreads, 6) k_plain_update(const PlainArgs A) {
+template <bool LOCKED>
+ITR_DEV void plain_finalize_body(const PlainArgs& A, int d, int n_blocks, int first);
+
+// One step's update of every design: 16x16 tiles x designs. FIN: the last block of a design to finish also
+// advances its integrator, as k_band's does (3 blocks an SM for the registers that takes: for batches of few tiles).
+template <bool CREST, bool BND = false, bool FIN = false>
+__global__ void __launch_bounds__(kTileThreads, FIN ? 3 : 6) k_plain_update(const PlainArgs A) {
   __shared__ float sh[18 * 18], su[18 * 18], sv[18 * 18], sc[18 * 18], sqx[18 * 18], sqy[18 * 18];
   __shared__ FaceF fx[16 * 17], fy[17 * 16];
   __shared__ float wmax[kTileThreads / 32];
@@ -308,6 +313,20 @@ __global__ void __launch_bounds__(kTileThreads, 6) k_plain_update(const PlainArg
     double* p = D.part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kPart;
     for (int j = 0; j < 5; ++j) p[j] = ss[j];
     p[5] = yt; p[6] = yb;
+  }
+  if constexpr (FIN) {
+    // the design's last block: the block's writes are in memory before the count (those of the other threads
+    // were ordered before this thread's by the barrier above)
+    __shared__ unsigned s_last;
+    const unsigned nblk = gridDim.x * gridDim.y;
+    if (li == 0) {
+      __threadfence();
+      s_last = atomicInc(A.arrive + blockIdx.z, nblk - 1u) == nblk - 1u ? 1u : 0u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    plain_finalize_body<false>(A, blockIdx.z, (int)nblk, 0);
   }
 }
 

@@ -164,30 +164,28 @@ def test_storms_at_the_ends_of_the_number_range(gpu, name, impl):
     with_options(gpu, {"impl": impl}, lambda: check(gpu, base, p, [PreparedTerrain(base)], f"{name} impl {impl}"))
 
 
-def test_launch_shape_follows_option_band(gpu):
+def test_launch_shape_follows_option_band():
     """The kernel of a batch follows from its sizes and the options, not from the calls before it: a grid that takes the
-    row bands runs elsewhere once option band is 0, as on a solver that never had it at 1."""
+    row bands, on solvers that had option band at 0 or 1 before."""
     base = synthetic_terrain(250, 230, 5.0, lambda x, y: 5.0 + 0.01 * x + 0.1 * math.sin(y / 9.0), n=0.03, segments=[Segment("transmissive", "west")])
     p = SolverParams(20.0, 10.0, rain=Hyetograph.from_mm_h([(0, 100)]), initial_depth=0.05)
-    terrs, mon = [PreparedTerrain(base)], MonitorSet(np.arange(0, 250 * 230, 991))
-    last = lambda g: g.adapter_info().split("last batch:")[1]
+    terrs, mon = [PreparedTerrain(base)] * 4, MonitorSet(np.arange(0, 250 * 230, 991))
 
-    def run(g):
-        r = g.run_batch(p, terrs, mon, ledger_rows=4)[0]
-        return last(g), r
+    def run(bands):
+        g = GpuSolver()
+        try:
+            for b in bands:
+                g.set_option("band", b)
+                r = g.run_batch(p, terrs, mon, ledger_rows=4)[0]
+            return g.adapter_info().split("last batch:")[1], r
+        finally:
+            g.close()
 
-    fresh = GpuSolver()
-    try:
-        fresh.set_option("band", 0)
-        want, a = run(fresh)
-    finally:
-        fresh.close()
-    first, _ = run(gpu)
-    assert "row bands" in first
-    got, b = with_options(gpu, {"band": 0}, lambda: run(gpu), {"band": 1})
-    assert got == want
-    np.testing.assert_array_equal(a.ledger, b.ledger)
-    assert run(gpu)[0] == first
+    for bands in ((0,), (1,)):
+        want, a = run(bands)
+        got, b = run((1 - bands[0],) + bands)
+        assert got == want and ("row bands" in want) == (bands == (1,))
+        np.testing.assert_array_equal(a.ledger, b.ledger)
 
 
 @pytest.mark.parametrize("nx,ny", [(161, 133), (40, 300), (1, 40)])
@@ -252,3 +250,70 @@ def test_single_column_on_the_cluster_kernel(gpu, ny, cluster, level, rain):
         # (time, volume, rain, inflow, outflow: f64 sums; the infiltration of a step is summed in f32, in another order)
         np.testing.assert_allclose(r.ledger[:, :5], a.ledger[:, :5], rtol=1e-12, atol=1e-12)
         assert np.all(r.ledger[:, 3:5] > 0.0)
+
+
+@pytest.mark.parametrize("level", [1, 2])
+@pytest.mark.parametrize("nx,ny,n", [(16, 16, 1), (17, 15, 5), (16, 16, 444), (16, 16, 445), (300, 33, 2)])
+def test_tiles_that_advance_the_integrator(gpu, nx, ny, n, level):
+    """One launch a step on 16x16 tiles (up to 444 of them) and two (above): the oracle's bits, the row bands' ledgers."""
+    dx = 2.0
+    segs = [Segment("inflow", "west", (0.0, 0.6 * ny * dx), hydrograph=[(0.0, 0.02), (12.0, 0.1)]), Segment("stage", "east", stage_m=3.15),
+            Segment("transmissive", "south")]
+    base = synthetic_terrain(nx * level, ny * level, dx / level, lambda x, y: 3.0 + 0.02 * math.sin(x / 5.0) * math.cos(y / 7.0), n=0.035, segments=segs, level=level)
+    p = SolverParams(12.0, 4.0, rain=Hyetograph.from_mm_h([(0, 100), (5, 300), (12, 50)]), infil_capacity=2e-6, initial_depth=0.12)
+    mon = MonitorSet(np.arange(0, nx * ny, 5))
+    terrs = []
+    for i in range(n):
+        t = PreparedTerrain(base)
+        t.dzx = t.dzx.copy()
+        t.dzx.flat[(7 * i + 3) % t.dzx.size] += np.float32(0.01 * (i + 1) / n)
+        terrs.append(t)
+    go = lambda: gpu.run_batch(p, terrs, mon, want_peak=True, ledger_rows=4)
+    got = with_options(gpu, {"impl": 2, "band": 0}, go, {"band": 1})
+    ref = with_options(gpu, {"impl": 2}, go)
+    for i, (a, b) in enumerate(zip(got, ref)):
+        assert a.steps == b.steps and np.array_equal(a.depth, b.depth) and np.array_equal(a.peak, b.peak)
+        np.testing.assert_allclose(a.ledger[:, :5], b.ledger[:, :5], rtol=1e-12, atol=1e-12)
+        if i % 89 == 0:
+            o = orc.flat_run(base_arrays(base), design_dict(terrs[i], p), p, mon, want_peak=True, bnd=orc.bnd_dict(base, terrs[i]))
+            compare_run(a, o, f"{nx}x{ny} design {i}")
+
+
+def test_aborts_on_tiles_that_advance_the_integrator(gpu):
+    from test_gpu_parity import small_valley
+    sc = small_valley(1200.0)
+    terrs = [t for _, _, t in sc.designs(6)]
+    baseline = gpu.run_batch(sc.params, [PreparedTerrain(sc.base)], sc.monitors)[0].monitor_max
+    sc.objective.d.guard_tolerance_m = 0.0005
+    inc = sorted(r.j for r in gpu.run_batch(sc.params, terrs, sc.monitors, objective=sc.objective))[2]
+    statuses = set()
+    for kw in (dict(guard_abort=True), dict(incumbent=inc), dict(guard_abort=True, incumbent=inc)):
+        go = lambda: gpu.run_batch(sc.params, terrs, sc.monitors, objective=sc.objective, baseline_max=baseline, **kw)
+        want, got = go(), with_options(gpu, {"impl": 2, "band": 0}, go, {"band": 1})
+        statuses |= {r.status for r in want}
+        for a, b in zip(got, want):
+            assert (a.status, a.steps, a.t_end, a.breach_cell, a.breach_sync, a.violation, a.lower_bound) == \
+                   (b.status, b.steps, b.t_end, b.breach_cell, b.breach_sync, b.violation, b.lower_bound)
+            assert np.array_equal(a.depth, b.depth)
+    assert len(statuses) > 1
+
+
+@pytest.mark.parametrize("nx,ny,n,rain,where", [(300, 180, 1, 60, "16x16 tiles"), (300, 180, 1, 0, "row bands|cluster"), (60, 900, 1, 60, "16x16 tiles"),
+                                                (900, 40, 2, 60, "16x16 tiles"), (180, 140, 1, 60, "cluster"), (250, 230, 16, 60, "row bands"),
+                                                (1000, 8, 4, 60, "16x16 tiles|cluster")])
+def test_few_designs_of_large_grids(gpu, nx, ny, n, rain, where):
+    """The kernel that the rule on sizes takes, dry rows not on the tiles, and the oracle's bits there, with locked dt too."""
+    base = synthetic_terrain(nx, ny, 5.0, lambda x, y: 5.0 + 0.01 * x + 0.1 * math.sin(y / 9.0), n=0.03, segments=[Segment("transmissive", "west")])
+    p = SolverParams(20.0, 10.0, rain=Hyetograph.from_mm_h([(0, rain), (20, rain)]), initial_depth=0.05)
+    terrs, mon = [PreparedTerrain(base)] * n, MonitorSet(np.arange(0, nx * ny, 97))
+    r = gpu.run_batch(p, terrs, mon, want_peak=True)
+    assert any(w in gpu.adapter_info() for w in where.split("|")), gpu.adapter_info()
+    o = orc.flat_run(base_arrays(base), design_dict(terrs[0], p), p, mon, want_peak=True, bnd=orc.bnd_dict(base, terrs[0]))
+    for i in range(n):
+        compare_run(r[i], o, f"{nx}x{ny} design {i}")
+        assert r[i].rows_skipped == o["rows_skipped"]
+    p.locked_dt = np.full(1000, 0.3)   # kept, or refused where it breaks the limit: the same on every path
+    lock = gpu.run_batch(p, terrs, mon)
+    ref = with_options(gpu, {"impl": 2}, lambda: gpu.run_batch(p, terrs, mon))
+    for a, b in zip(lock, ref):
+        assert a.steps == b.steps and np.array_equal(a.depth, b.depth)
