@@ -197,8 +197,9 @@ int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_grid* g, int3
  *              take the tiled path), 1 = plain one-design-per-launch kernel, 2 = tiled
  *              batched path: all designs per launch, state in HBM, a CUDA graph per
  *              steps_per_submit steps
- *   "threads"  threads per CTA of the batched kernel, at most 512 used (0 = by the grid and population)
- *   "cluster"  CTAs per design of the batched kernel (0 = by the grid and population, 1 .. 8)
+ *   "threads"  threads per CTA of the batched kernel, at most 512 used, 768 on grids wider than 960 columns
+ *              (0 = by the grid and population)
+ *   "cluster"  CTAs per design of the batched kernel: 1, 2, 4 or 8 (0 = by the grid and population)
  *   "graph"    tiled path: 1 = replay each block of steps as one CUDA graph (default 1)
  *   "steps_per_submit"  plain and tiled paths: steps between host polls (default 64)
  *   "warm_start"  1 = start each design from the baseline record (itr_gpu_record_baseline) where

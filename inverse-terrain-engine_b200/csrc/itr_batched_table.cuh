@@ -1,8 +1,8 @@
 // itr_batched_table.cuh — the instantiations of k_batched for one (CREST, BND) pair.
 //
-// k_batched has 96 instantiations: crest faces, stage/inflow ghosts, cluster use, three block
+// k_batched has 128 instantiations: crest faces, stage/inflow ghosts, cluster use, four block
 // size buckets, locked dt and dry-row skipping. Each of the translation units itr_kb_<c><b>.cu
-// instantiates the 24 of one (CREST, BND) pair through ITR_BATCHED_TABLE, so the library
+// instantiates the 32 of one (CREST, BND) pair through ITR_BATCHED_TABLE, so the library
 // compiles in parallel; the self-checking build (-DITR_CHECKED) instantiates all four pairs
 // in itr_capi.cu, one translation unit, so its error record g_itr_err is a single array.
 #pragma once
@@ -16,7 +16,8 @@ template <bool CR, bool CL, bool BD, bool LK, bool SK>
 BatchedFn batched_by_maxt(int maxt) {
   if (maxt <= 256) return k_batched<CR, CL, 256, BD, LK, SK>;
   if (maxt <= 384) return k_batched<CR, CL, 384, BD, LK, SK>;
-  return k_batched<CR, CL, 512, BD, LK, SK>;
+  if (maxt <= 512) return k_batched<CR, CL, 512, BD, LK, SK>;
+  return k_batched<CR, CL, 768, BD, LK, SK>;
 }
 
 template <bool CR, bool BD>

@@ -233,7 +233,7 @@ static BatchedFn batched_fn(bool crest, bool clustered, int maxt, bool bnd, bool
   return bnd ? batched_fn_01(clustered, maxt, locked, skip) : batched_fn_00(clustered, maxt, locked, skip);
 }
 
-static int maxt_bucket(int T) { return T <= 256 ? 256 : T <= 384 ? 384 : 512; }
+static int maxt_bucket(int T) { return T <= 256 ? 256 : T <= 384 ? 384 : T <= 512 ? 512 : 768; }
 
 // Geometry of the batched kernel for (nx, ny) with C CTAs per design and about T threads.
 static LaunchCfg make_cfg(const itr_ctx* ctx, int nx, int ny, int C, int T_target, bool bnd) {
@@ -243,12 +243,13 @@ static LaunchCfg make_cfg(const itr_ctx* ctx, int nx, int ny, int C, int T_targe
   c.W = windows(nx);   // warps per strip row
   if (C < 1 || ny < C) return c;
   const int nr_min = ny / C, nr_max = (ny + C - 1) / C;
-  int S = std::min(T_target, 512) / (32 * c.W);   // (more threads leave too few registers each: below)
+  const int most = c.W > 16 ? 768 : 512;   // (more threads leave too few registers each: batched_shape)
+  int S = std::min(T_target, most) / (32 * c.W);
   if (S > nr_min) S = nr_min;
   if (S < 1) return c;
   c.S = S;
   c.T = S * 32 * c.W;
-  if (c.T > 512) return c;
+  if (c.T > most) return c;
   c.smem = smem_plan(nr_max, nx, S, c.W, c.T / 32, bnd ? 1 : 0, ny).total;
   c.ok = c.smem <= ctx->smem_optin;
   return c;
@@ -311,6 +312,13 @@ static int max_active_clusters(itr_ctx* ctx, const LaunchCfg& cfg, bool crest) {
   return n;
 }
 
+// Predicted time per round and step of a block above 512 threads (grids of 961 to 1440 columns). Such grids with few
+// rows take the device's other kernels longer: us a step, this / the best of tiles and bands, 1000x8 x1 7.8 / 10.4,
+// x16 11.4 / 18.2, 1200x8 x32 12.2 / 22.1, 1440x8 x8 10.4 / 15.0. Fitted within 6 % to 961x4 .. 1440x16.
+static double wide_step_us(const LaunchCfg& c, int ny) {
+  return (c.C > 1 ? 1.5 : 0.9) + (std::ceil((double)ny / c.C) + 0.9) * 0.19 * c.W;
+}
+
 // The launch shape of the cluster kernel for n designs of an nx x ny grid: the least predicted time per
 // step over all cluster sizes and block sizes. A rule on sizes alone, so that the same batch always
 // runs in the same shape (its ledger sums to the same bits); it replaces timing a few candidates on
@@ -321,13 +329,14 @@ static int max_active_clusters(itr_ctx* ctx, const LaunchCfg& cfg, bool crest) {
 // each: the shape chosen is the fastest or within 6 % of it on all but one (45x35 x64: 12 %), 0.8 %
 // on average. Blocks above 256 threads hold 168 registers a thread, too few for the sweep that runs the
 // faces a row ahead (x 1.15 per row), but three windows divide 12 warps and not 8; above 384 (128
-// registers) only for grids that need more windows than 12.
+// registers) only for grids that need more windows than 12, and above 512 (80 registers, a kilobyte of them in local
+// memory) for one strip of 17 to 24: wide_step_us.
 static LaunchCfg batched_shape(itr_ctx* ctx, int nx, int ny, int n, bool crest, bool bnd) {
   LaunchCfg best;
   double best_us = 1e300;
   for (int C = 1; C <= 8; ++C) {
     int last_S = 0;
-    for (int T = 32; T <= 512; T += 32) {
+    for (int T = 32; T <= 768; T += 32) {
       if (T > 384 && 32 * windows(nx) <= 384) break;
       const LaunchCfg c = make_cfg(ctx, nx, ny, C, T, bnd);
       if (!c.ok || c.S == last_S) continue;
@@ -338,7 +347,7 @@ static LaunchCfg batched_shape(itr_ctx* ctx, int nx, int ny, int n, bool crest, 
       const int ctas = std::min(n, act) * C, per_sm = (ctas + ctx->sm_count - 1) / ctx->sm_count;
       const double w = std::max(1.0, per_sm * c.T / 128.0), rows = std::ceil(std::ceil((double)ny / C) / c.S);
       const double r = c.T <= 256 ? 0.75 * (1.0 + 0.25 * (w - 1.0)) : 0.8625 * (1.0 + 0.3 * (w - 1.0));
-      const double us = waves * ((C > 1 ? 1.5 : 0.9) + (rows + 0.5) * r);
+      const double us = waves * (c.T > 512 ? wide_step_us(c, ny) : (C > 1 ? 1.5 : 0.9) + (rows + 0.5) * r);
       if (us < best_us) { best_us = us; best = c; best.us = us; }
     }
   }
@@ -352,7 +361,7 @@ static double cluster_step_us(const itr_ctx* ctx, const LaunchCfg& c, int ny, in
   const int ctas = std::min(n, act) * c.C, per_sm = (ctas + ctx->sm_count - 1) / ctx->sm_count;
   const double w = std::max(1.0, std::ceil(per_sm * c.T / 128.0)), rows = std::ceil(std::ceil((double)ny / c.C) / c.S);
   const double r = c.T <= 256 ? 0.75 * (1.0 + 0.25 * (w - 1.0)) : (c.T <= 384 ? 0.8625 : 1.104) * (1.0 + 0.3 * (w - 1.0));
-  return std::ceil((double)n / act) * ((c.C > 1 ? 1.5 : 0.9) + (rows + 0.5) * r);
+  return std::ceil((double)n / act) * (c.T > 512 ? wide_step_us(c, ny) : (c.C > 1 ? 1.5 : 0.9) + (rows + 0.5) * r);
 }
 
 // Predicted time per step of the row bands: a launch and the integrator's chain (longer where a block has one warp),

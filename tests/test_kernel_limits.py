@@ -317,3 +317,30 @@ def test_few_designs_of_large_grids(gpu, nx, ny, n, rain, where):
     ref = with_options(gpu, {"impl": 2}, lambda: gpu.run_batch(p, terrs, mon))
     for a, b in zip(lock, ref):
         assert a.steps == b.steps and np.array_equal(a.depth, b.depth)
+
+
+@pytest.mark.parametrize("nx,ny,level,cluster", [(961, 4, 1, 0), (1000, 8, 2, 0), (1020, 3, 1, 2), (1021, 5, 2, 2), (1100, 1, 1, 1), (1439, 9, 1, 8), (1440, 8, 1, 4), (1441, 4, 1, 0)])
+@pytest.mark.parametrize("rain", [True, False])
+def test_blocks_above_512_threads(gpu, nx, ny, level, cluster, rain):
+    """Grids of 17 to 24 windows on the cluster kernel, widths on both sides of a window; 25 windows on the tiled path."""
+    dx = 2.0
+    segs = [Segment("inflow", "west", hydrograph=[(0.0, 0.02), (30.0, 0.1)]), Segment("stage", "east", stage_m=3.1),
+            Segment("inflow", "north", (0.3 * nx * dx, 0.7 * nx * dx), hydrograph=[(0.0, 0.01), (3.0, 0.3)])]
+    base = synthetic_terrain(nx * level, ny * level, dx / level, lambda x, y: 3.0 + 0.02 * math.sin(x / 5.0) - 0.01 * y, n=0.035, segments=segs, level=level)
+    p = SolverParams(8.0, 4.0, dt_max_s=0.2, rain=Hyetograph.from_mm_h([(0, 100), (5, 300), (8, 50)] if rain else []), infil_capacity=2e-6,
+                     initial_depth=0.12 if rain else 0.0)
+    terrs, mon = [PreparedTerrain(base)] * 2, MonitorSet(np.arange(0, nx * ny, 5))
+    o = orc.flat_run(base_arrays(base), design_dict(terrs[0], p), p, mon, want_peak=True, bnd=orc.bnd_dict(base, terrs[0]))
+
+    def run():
+        r = gpu.run_batch(p, terrs, mon, want_peak=True)
+        assert ("cluster kernel" if nx <= 1440 else "tiled path") in gpu.adapter_info()
+        return r
+
+    opts = {"cluster": cluster, "threads": 768 if cluster else 0}
+    for r in with_options(gpu, opts, run):
+        compare_run(r, o, f"{nx}x{ny} cluster {cluster}")
+    p.locked_dt = np.full(1000, 0.05)
+    ref = with_options(gpu, {"impl": 2}, lambda: gpu.run_batch(p, terrs, mon))
+    for a, b in zip(with_options(gpu, opts, run), ref):
+        assert a.steps == b.steps and np.array_equal(a.depth, b.depth)
