@@ -68,7 +68,8 @@ ITR_DEV float sqrt_rn(float x) {
 // bits for operands in the ranges that rcp2 and sqrt2 (below) state, which hold in a step from a
 // bounded state (StepK::exact == 0). Fast::div: a y with y = 1 / b rounded, corrected twice by the
 // exact residual (as div_rn), b in rcp2's range and not above 2^62; a small |a| (adjoints at the fringe of their domain
-// of dependence) is scaled by 2^64 and back, which keeps the residual a normal number. A quotient
+// of dependence) is scaled by 2^64 and back, which keeps the residual a normal number (|a / b| below 2^63 there:
+// the derivative of u at h = 0 reaches 2 / h_eps^2). A quotient
 // that overflows, or of an infinity or NaN, is returned before the correction (infinity - infinity); one
 // below 2^-126 is rounded a second time on its way back, and may then lie one 2^-149 beside the IEEE
 // result. The adjoint's divisors: celerities and |q|, 2^-76 .. 2^40; h^2 above h_eps^2; and h_eps^4 up
@@ -585,7 +586,7 @@ ITR_DEV B2 gt2(float2 a, float b) { return B2{a.x > b, a.y > b}; }
 // 1/x for |x| in [2^-125, 2^126): one Newton step from the hardware estimate (textbook FMA
 // refinement: P. Markstein, IBM J. Res. Dev. 34(1), 1990; J.-M. Muller et al., Handbook of
 // Floating-Point Arithmetic, 2nd ed., 2018, ch. 4): y = est(1/x); e = fma(-x, y, 1); y + y e.
-// Equal to CUDA's IEEE reciprocal on every 32-bit input of that range (checked on the B200).
+// Equal to CUDA's IEEE reciprocal on every 32-bit input of that range (tests/test_special_ops.py).
 ITR_DEV float2 rcp2(float2 x) {
   const float2 y = make_float2(rcp_est(x.x), rcp_est(x.y));
   const float2 e = make_float2(__fmaf_rn(-x.x, y.x, 1.0f), __fmaf_rn(-x.y, y.y, 1.0f));
@@ -595,8 +596,8 @@ ITR_DEV float2 rcp2(float2 x) {
 // 1/sqrt (same sources: s = x y, d = fma(-s, s, x), s + d (y / 2)), on x 2^48 so that the
 // residual d is exact for the smallest subnormals too (wetting fronts have depths down to them).
 // The 2^-126 added for the estimate alone keeps it finite at 0 and vanishes in rounding
-// elsewhere. Equal to CUDA's IEEE square root on every 32-bit input of that range (checked on the
-// B200); about half its time, and without the branch that would end the basic block.
+// elsewhere. Equal to CUDA's IEEE square root on every 32-bit input of that range (tests/test_special_ops.py);
+// about half its time, and without the branch that would end the basic block.
 ITR_DEV float2 sqrt2(float2 x) {
   const float2 xs = mulc2(0x1p48f, x);
   const float2 xt = addc2(xs, 0x1p-126f);
