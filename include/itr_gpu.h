@@ -193,10 +193,10 @@ int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_grid* g, int3
                       const itr_objective* obj, itr_result* results);
 
 /* Options (GpuSolver::steps_per_submit, lib.rs:70, is the reference's one knob):
- *   "impl"     0 = batched cluster kernel (default; grids too large for 8 CTAs' shared memory
- *              take the tiled path), 1 = plain one-design-per-launch kernel, 2 = tiled
- *              batched path: all designs per launch, state in HBM, a CUDA graph per
- *              steps_per_submit steps
+ *   "impl"     0 = batched cluster kernel (default; grids too large for 8 CTAs' shared memory, and
+ *              those where it is predicted to be faster, take the tiled path), 1 = plain
+ *              one-design-per-launch kernel, 2 = tiled batched path: all designs per launch,
+ *              state in HBM, a CUDA graph per steps_per_submit steps
  *   "threads"  threads per CTA of the batched kernel, at most 512 used, 768 on grids wider than 960 columns
  *              (0 = by the grid and population)
  *   "cluster"  CTAs per design of the batched kernel: 1, 2, 4 or 8 (0 = by the grid and population)
@@ -207,8 +207,8 @@ int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_grid* g, int3
  *   "exact_special"     1 = the batched kernel computes every reciprocal and square root
  *                       with the IEEE-exact library routines instead of its own branch-free
  *                       ones (identical results; for checking, default 0)
- *   "band"     tiled path update kernel: 1 = row-band sweep (default), 0 = 16x16 tiles with a
- *              halo (identical results; for comparison)
+ *   "band"     tiled path update kernel: 1 = row-band sweep, or with impl 0 the tiles where they are
+ *              predicted to be faster (default), 0 = 16x16 tiles with a halo (identical results)
  *   "adj_band" adjoint kernels on row-band sweeps instead of 16x16 tiles with a halo: bit 0
  *              the replay of each segment, bit 1 the backward step; -1 (default) = the replay
  *              on bands, the backward step on bands for grids of 2^18 cells or more
@@ -221,6 +221,7 @@ int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_grid* g, int3
  *   "stall_wait_test"   1 = that barrier expects one arrival more than the CTA makes, so every
  *                       such wait runs to its limit and the call returns ITR_DEVICE_TIMEOUT with
  *                       the context still usable (test of the timeout path; default 0)
+ *   "autotune", "probe_steps"  accepted, without effect (the launch shape follows from the sizes)
  * Returns ITR_INVALID_ARG for an unknown key. */
 int itr_gpu_set_option(itr_ctx* ctx, const char* key, int64_t value);
 

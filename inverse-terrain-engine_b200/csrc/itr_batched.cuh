@@ -209,17 +209,6 @@ ITR_DEV double warp_sum_d(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-ITR_DEV float warp_sum_f(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-ITR_DEV float warp_max_f(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = rmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
 // Barrier over the design: the cluster's, or the CTA's for single-CTA designs.
 template <bool CLUSTERED>
 ITR_DEV void design_bar() {

@@ -822,10 +822,11 @@ static int run_plain_design(itr_ctx* ctx, PlainArgs& A, int n_blocks, dim3 grid,
 }
 
 // ------------------------------------------------------------------ tiled batch ------
-// All designs per launch: one update (tiles x designs) and one finalize (a warp per design)
-// per step, driven entirely by the control blocks on the device, so a block of
+// All designs per launch: per step one launch, whose last block of a design advances its integrator, or an
+// update and a finalize, driven entirely by the control blocks on the device, so a block of
 // steps_per_submit steps is captured once in a CUDA graph and replayed until every design
 // is done (the host reads the control blocks between replays).
+
 // The adjoint's kernels on row bands: bit 0 the replay, bit 1 the backward step (option adj_band).
 static int adj_band_bits(const itr_ctx* ctx, size_t N) { return ctx->adj_band >= 0 ? ctx->adj_band : (N >= (size_t(1) << 18) ? 3 : 1); }
 
