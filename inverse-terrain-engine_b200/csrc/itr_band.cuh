@@ -21,8 +21,8 @@
 //   * the old state is read-only during a step (ping-pong), so warps never synchronise with
 //     each other inside a step: row r + 1 is loaded while row r is updated, and the only
 //     block barrier is the final reduction of the per-block partials.
-// What bounds it: the row arithmetic (56 % of the issue slots, register-file reads; a step of 16 designs
-// of 1024 x 1024 moves 48 B per cell in 0.29 ms, 2.7 TB/s). So a row's inputs come as two records
+// What bounds it: the row arithmetic, issue and dependent instructions at 12 warps an SM (61 % of the issue
+// slots; a step of 16 designs of 1024 x 1024 moves 48 B per cell in 0.30 ms, 2.7 TB/s). So a row's inputs come as two records
 // (jumps, wet | g n^2) of 16 B per pair, the columns past the grid are masked once per step instead of
 // once per row, a row's ghosts are filled in when it is used (filled in at the load they made every
 // row wait for memory: 285 ms against 238 ms of 16 designs x 959 steps; the layout with separate arrays
