@@ -499,6 +499,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
   double sum_infil = 0.0, sum_fix = 0.0, sum_in = 0.0, sum_out = 0.0;
 
   const float2* inf_cur = sm.INF;   // this step's inflow group values (parity slot)
+  unsigned gw_even = ~0u, gw_odd = ~0u;   // inflow groups that flow (a bit each) in the ghost wetness of each parity slot; ~0: not known
   const int top_odd = row_odd(lr0, nr), bot_odd = row_odd(lr0 + L - 1, nr);
   // The lane's pair in the rows above the strip's first and below its last, on even and odd steps: in
   // this CTA or the next one (unused at the domain's edges). B lies nab words after A everywhere.
@@ -602,7 +603,10 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
           if (BND && wid == nwarps - 1) {
             if (lane < P.inflow.n) sm.INF[par * kMaxInflow + lane] = inflow_values(P.inflow, lane, t, P.g);
             __syncwarp();
-            if (SKIP) ghost_row_wet(A.bc, nx, ny, bh, sm.INF + par * kMaxInflow, sm.GWF + par * (ny + 2), lane);
+            if (SKIP) {
+              ghost_row_wet(A.bc, nx, ny, bh, sm.INF + par * kMaxInflow, sm.GWF + par * (ny + 2), lane);
+              gw_even = gw_odd = ~0u;
+            }
           }
           if (SKIP) {
             __syncthreads();   // the restored rows complete before their flags are taken
@@ -673,8 +677,14 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
       if (wid == nwarps - 1) {
         if (lane < P.inflow.n) sm.INF[(sp ^ 1) * kMaxInflow + lane] = inflow_values(P.inflow, lane, pl.t_new, P.g);
         if (SKIP) {
+          // (the ghosts' wetness changes only with the groups that flow: going over the edge cells again each step
+          // was up to 17 us of it on wide grids)
           __syncwarp();
-          ghost_row_wet(A.bc, nx, ny, bh, sm.INF + (sp ^ 1) * kMaxInflow, sm.GWF + (sp ^ 1) * (ny + 2), lane);
+          const unsigned flows = __ballot_sync(0xffffffffu, lane < P.inflow.n && sm.INF[(sp ^ 1) * kMaxInflow + (lane & (kMaxInflow - 1))].y > 0.0f);
+          if (flows != (sp ? gw_even : gw_odd)) {
+            ghost_row_wet(A.bc, nx, ny, bh, sm.INF + (sp ^ 1) * kMaxInflow, sm.GWF + (sp ^ 1) * (ny + 2), lane);
+            (sp ? gw_even : gw_odd) = flows;
+          }
         }
       }
     }
