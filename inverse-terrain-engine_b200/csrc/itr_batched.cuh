@@ -54,7 +54,7 @@ namespace cg = cooperative_groups;
 struct LockedSnap {
   double t, dt_cfl, s_cur, acc_rain, volume, rel_res;
   double led[4];
-  unsigned long long step;
+  unsigned long long step, skipped;   // skipped: dry rows of this CTA so far
   unsigned sync_index;
   int n_rows;
 };
@@ -274,7 +274,7 @@ ITR_DEV void locked_save(const BatchArgs& A, const Smem& sm, int n16, size_t rec
     LockedSnap& o = A.snap_s[rec];
     o.t = t; o.dt_cfl = dt_cfl; o.s_cur = s_cur; o.acc_rain = acc_rain; o.volume = volume; o.rel_res = rel_res;
     for (int j = 0; j < 4; ++j) o.led[j] = sm.LED[j];
-    o.step = step; o.sync_index = sync_index; o.n_rows = n_rows;
+    o.step = step; o.skipped = *sm.NSK; o.sync_index = sync_index; o.n_rows = n_rows;
   }
   __syncthreads();
 }
@@ -595,6 +595,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_batched(const BatchArgs A) {
           t = o.t; dt_cfl = o.dt_cfl; s_cur = o.s_cur; acc_rain = o.acc_rain; volume = o.volume; rel_res = o.rel_res;
           step = o.step; sync_index = o.sync_index; n_rows = o.n_rows;
           if (tid < 4) sm.LED[tid] = o.led[tid];
+          if (SKIP && tid == 0) *sm.NSK = o.skipped;
           if (tid < 3) sm.slot[tid] = make_uint2(0u, 0u);
           sum_infil = sum_fix = sum_in = sum_out = 0.0;
           seg = 0; have_smax = false;

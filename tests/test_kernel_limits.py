@@ -344,3 +344,23 @@ def test_blocks_above_512_threads(gpu, nx, ny, level, cluster, rain):
     ref = with_options(gpu, {"impl": 2}, lambda: gpu.run_batch(p, terrs, mon))
     for a, b in zip(with_options(gpu, opts, run), ref):
         assert a.steps == b.steps and np.array_equal(a.depth, b.depth)
+
+
+@pytest.mark.parametrize("impl", [0, 2])
+def test_dry_rows_of_steps_taken_back(gpu, impl):
+    """A locked run that returns to its last snapshot takes back the count of dry rows with the steps."""
+    nx, ny, dx = 60, 50, 2.0
+    segs = [Segment("inflow", "north", (0.3 * nx * dx, 0.8 * nx * dx), hydrograph=[(0.0, 0.0), (3.0, 0.0), (4.0, 1.5)]),
+            Segment("stage", "south", (0.0, 0.5 * nx * dx), stage_m=0.6)]
+    base = synthetic_terrain(nx, ny, dx, lambda x, y: 0.02 * y + 0.1 * math.sin(x / 7.0) + 0.1, n=0.03, segments=segs)
+    p = SolverParams(10.0, 5.0, dt_max_s=0.1, rain=Hyetograph([]), initial_depth=0.0)
+    t, mon = PreparedTerrain(base), MonitorSet(np.arange(0, nx * ny, 5))
+    p.locked_dt = np.full(60, 0.1)
+    o = orc.locked(lambda: orc.flat_run(base_arrays(base), design_dict(t, p), p, mon, want_peak=True, bnd=orc.bnd_dict(base, t)),
+                   p.locked_dt, p.cfl_hard)
+    back = o["dt_fallback_t"]
+    assert back > 0.0 and o["rows_skipped"] > 0
+    r = with_options(gpu, {"impl": impl}, lambda: gpu.run_batch(p, [t, t], mon, want_peak=True))
+    for a in r:
+        compare_run(a, o, f"impl {impl}")
+        assert (a.dt_fallback_t, a.rows_skipped) == (back, o["rows_skipped"])
