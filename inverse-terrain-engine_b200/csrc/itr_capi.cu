@@ -761,19 +761,23 @@ int itr_gpu_last_timing(itr_ctx* ctx, double* kernel_ms, double* total_ms, uint6
 
 }  // extern "C"
 
+// go(crest, bnd, skip) with the three as compile-time constants.
+template <class Go>
+static void by_flags(bool crest, bool bnd, bool skip, Go go) {
+  using T = std::true_type;
+  using F = std::false_type;
+  if (crest) { if (bnd) { if (skip) go(T(), T(), T()); else go(T(), T(), F()); } else { if (skip) go(T(), F(), T()); else go(T(), F(), F()); } }
+  else { if (bnd) { if (skip) go(F(), T(), T()); else go(F(), T(), F()); } else { if (skip) go(F(), F(), T()); else go(F(), F(), F()); } }
+}
+
 // ------------------------------------------------------------------ plain path ------
 // One step's update kernel of the tiled path: the ghost rule with stage and inflow cells
 // only where the grid has them.
 template <bool FIN = false>
 static void launch_update(const PlainArgs& A, dim3 grid, cudaStream_t st) {
-  const bool bnd = A.bh != nullptr || A.P.inflow.n > 0;
-  if (A.mode == 1) {
-    if (bnd) k_plain_update<true, true, FIN><<<grid, kTileThreads, 0, st>>>(A);
-    else k_plain_update<true, false, FIN><<<grid, kTileThreads, 0, st>>>(A);
-  } else {
-    if (bnd) k_plain_update<false, true, FIN><<<grid, kTileThreads, 0, st>>>(A);
-    else k_plain_update<false, false, FIN><<<grid, kTileThreads, 0, st>>>(A);
-  }
+  const bool bnd = A.bh != nullptr || A.P.inflow.n > 0, skip = A.rowwet != nullptr;
+  auto go = [&](auto crest, auto b, auto s) { k_plain_update<decltype(crest)::value, decltype(b)::value, FIN, decltype(s)::value><<<grid, kTileThreads, 0, st>>>(A); };
+  by_flags(A.mode == 1, bnd, skip, go);
 }
 
 // One step of the tiled batched path: the row-band sweep (itr_band.cuh) over (segment groups, bands,
@@ -785,10 +789,7 @@ static void launch_band(const PlainArgs& A, dim3 grid, cudaStream_t st, int fin)
   const BandGeom bg = band_geom(A.nx, A.ny, A.band_rows);
   const dim3 block((unsigned)(32 * bg.wpb));
   auto go = [&](auto crest, auto b, auto s) { k_band<decltype(crest)::value, decltype(b)::value, TAPE, decltype(s)::value && !TAPE><<<grid, block, 0, st>>>(A, fin); };
-  using T = std::true_type;
-  using F = std::false_type;
-  if (A.mode == 1) { if (bnd) { if (skip) go(T(), T(), T()); else go(T(), T(), F()); } else { if (skip) go(T(), F(), T()); else go(T(), F(), F()); } }
-  else { if (bnd) { if (skip) go(F(), T(), T()); else go(F(), T(), F()); } else { if (skip) go(F(), F(), T()); else go(F(), F(), F()); } }
+  by_flags(A.mode == 1, bnd, skip, go);
 }
 
 // Blocks per design of the tiled path's update (the finalize's partials).
@@ -1674,7 +1675,7 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
       e = ctx->tArr.ensure((size_t)n * 4);
       A.arrive = ctx->tArr.as<unsigned>();
     }
-    if (band && P.skip_dry && e == cudaSuccess) {   // dry-row skipping (the storm leaves a rain-free step)
+    if ((band || tiles) && P.skip_dry && e == cudaSuccess) {   // dry-row skipping (the storm leaves a rain-free step)
       const size_t R = (size_t)ny + 2;
       e = ctx->tRow.ensure((size_t)n * 2 * R * 4);
       if (e == cudaSuccess && bnd_grid) e = ctx->tGw.ensure((size_t)n * R);
@@ -1737,13 +1738,15 @@ extern "C" int itr_gpu_run_batch(itr_ctx* ctx, const itr_params* p, const itr_gr
       // spread a step over the most threads, more on row bands, by margins for the models' errors. us a step, cluster /
       // bands / tiles: 300x180 x1 18.9 / 17.1 / 10.9, x4 19.1 / 18.1 / 18.4, x8 19.2 / 31.2 / 26.6; 250x230 x1 29.2 / 16.8 /
       // 10.7, x16 58.5 / 26.4 / 44.2; 60x900 x1 16.1 / 20.8 / 10.8; 180x140 x1 9.0 / 17.1 / 9.9. A ladder's groups are
-      // branches of one graph and stay on the cluster kernel; the tiles do not skip dry rows.
+      // branches of one graph and stay on the cluster kernel. The dry-row instantiation of the cluster kernel runs row by
+      // row and takes 1.2 times as long (240x192 x32 without rain 47.8 us a step, on bands 30.4); the row flags cost the tiles
+      // a tenth and 3 us, a step of bands 6 us where few rows are skipped (300x180 x1 15.0 / 24.5, 265x380 x8 45.9 / 39).
       const bool open = !ctx->defer && n <= 65535;
-      const double cl = cfg.ok ? cluster_step_us(ctx, cfg, ny, n, std::max(1, max_active_clusters(ctx, cfg, crest))) : HUGE_VAL;
+      const double cl = cfg.ok ? cluster_step_us(ctx, cfg, ny, n, std::max(1, max_active_clusters(ctx, cfg, crest))) * (P.skip_dry ? 1.2 : 1.0) : HUGE_VAL;
       const double bd = ctx->band ? tiled_step_us(ctx, nx, ny, n, locked) : HUGE_VAL;
-      const double tl = P.skip_dry ? HUGE_VAL : tile_step_us(ctx, nx, ny, n, locked);
+      const double tl = tile_step_us(ctx, nx, ny, n, locked) * (P.skip_dry ? 1.1 : 1.0) + (P.skip_dry ? 3.0 : 0.0);
       cfg.tiled = !cfg.ok || (open && std::min(bd / 0.85, tl / 0.96) < cl);
-      cfg.tiles = cfg.tiled && (!ctx->band || (open && tl < 0.92 * bd && tl < 0.96 * cl));
+      cfg.tiles = cfg.tiled && (!ctx->band || (open && tl < 0.92 * (bd + (P.skip_dry ? 6.0 : 0.0)) && tl < 0.96 * cl));
       ctx->tuned[key] = cfg;
       tiled = cfg.tiled; tiles = cfg.tiles;
       if (!tiled) CU(pack());

@@ -210,7 +210,9 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int d, int n_blocks, int fi
 
 // One step's update of every design: 16x16 tiles x designs. FIN: the last block of a design to finish also
 // advances its integrator, as k_band's does (3 blocks an SM for the registers that takes: for batches of few tiles).
-template <bool CREST, bool BND = false, bool FIN = false>
+// SKIP: rows that hold water are flagged, from which the finalize counts the rows that could be skipped; the tiles
+// compute them all the same (zero faces, the zero state kept).
+template <bool CREST, bool BND = false, bool FIN = false, bool SKIP = false>
 __global__ void __launch_bounds__(kTileThreads, FIN ? 3 : 6) k_plain_update(const PlainArgs A) {
   __shared__ float sh[18 * 18], su[18 * 18], sv[18 * 18], sc[18 * 18], sqx[18 * 18], sqy[18 * 18];
   __shared__ FaceF fx[16 * 17], fy[17 * 16];
@@ -263,7 +265,7 @@ __global__ void __launch_bounds__(kTileThreads, FIN ? 3 : 6) k_plain_update(cons
   }
   __syncthreads();
   float smax = 0.0f;
-  bool bad = false, uns = false;
+  bool bad = false, uns = false, wet = false;
   double acc[5] = {0, 0, 0, 0, 0};
   if (cv) {
     const FaceF w = fx[ly * 17 + lx], e = fx[ly * 17 + lx + 1];
@@ -278,6 +280,7 @@ __global__ void __launch_bounds__(kTileThreads, FIN ? 3 : 6) k_plain_update(cons
     }
     smax = o.s;
     bad = o.bad;
+    wet = o.h > 0.0f;
     uns = !state_safe(A.P, o.s);
     acc[0] = (double)o.infil; acc[1] = (double)o.fix;
     if (hits) acc[4] = (double)o.h;
@@ -286,6 +289,10 @@ __global__ void __launch_bounds__(kTileThreads, FIN ? 3 : 6) k_plain_update(cons
     if (gx == nx - 1) { double v = (double)e.m * dt_dy; if (v > 0.0) acc[3] += v; else acc[2] -= v; }
     if (gy == 0) yedge[0][lx] = (double)n.m;
     if (gy == ny - 1) yedge[1][lx] = (double)s.m;
+  }
+  if constexpr (SKIP) {   // a warp holds two rows of the tile (every writer stores 1)
+    const unsigned w = __ballot_sync(0xffffffffu, wet);
+    if ((li & 15) == 0 && (w >> (li & 16) & 0xffffu)) D.rowwet[(size_t)(par ^ 1) * (ny + 2) + gy + 1] = 1u;
   }
   // block reductions, fixed order
   float m = smax;

@@ -298,11 +298,11 @@ def test_aborts_on_tiles_that_advance_the_integrator(gpu):
     assert len(statuses) > 1
 
 
-@pytest.mark.parametrize("nx,ny,n,rain,where", [(300, 180, 1, 60, "16x16 tiles"), (300, 180, 1, 0, "row bands|cluster"), (60, 900, 1, 60, "16x16 tiles"),
+@pytest.mark.parametrize("nx,ny,n,rain,where", [(300, 180, 1, 60, "16x16 tiles"), (300, 180, 1, 0, "16x16 tiles"), (60, 900, 1, 60, "16x16 tiles"),
                                                 (900, 40, 2, 60, "16x16 tiles"), (180, 140, 1, 60, "cluster"), (250, 230, 16, 60, "row bands"),
                                                 (1000, 8, 4, 60, "16x16 tiles|cluster")])
 def test_few_designs_of_large_grids(gpu, nx, ny, n, rain, where):
-    """The kernel that the rule on sizes takes, dry rows not on the tiles, and the oracle's bits there, with locked dt too."""
+    """The kernel that the rule on sizes takes, and the oracle's bits there, with locked dt too."""
     base = synthetic_terrain(nx, ny, 5.0, lambda x, y: 5.0 + 0.01 * x + 0.1 * math.sin(y / 9.0), n=0.03, segments=[Segment("transmissive", "west")])
     p = SolverParams(20.0, 10.0, rain=Hyetograph.from_mm_h([(0, rain), (20, rain)]), initial_depth=0.05)
     terrs, mon = [PreparedTerrain(base)] * n, MonitorSet(np.arange(0, nx * ny, 97))
@@ -364,3 +364,32 @@ def test_dry_rows_of_steps_taken_back(gpu, impl):
     for a in r:
         compare_run(a, o, f"impl {impl}")
         assert (a.dt_fallback_t, a.rows_skipped) == (back, o["rows_skipped"])
+
+
+@pytest.mark.parametrize("nx,ny,n,level", [(300, 180, 1, 1), (300, 180, 2, 1), (61, 900, 1, 1), (250, 230, 2, 1), (80, 1200, 1, 2)])
+def test_dry_rows_on_tiles(gpu, nx, ny, n, level):
+    """Few designs of a large grid without rain on the 16x16 tiles, which count the dry rows that the other kernels skip:
+    one launch a step (up to 444 tiles) and two, the oracle's count and bits; locked dt and a restored snapshot too."""
+    dx = 2.0
+    segs = [Segment("inflow", "north", (0.3 * nx * dx, 0.8 * nx * dx), hydrograph=[(0.0, 0.0), (3.0, 0.0), (4.0, 1.5)]),
+            Segment("stage", "south", (0.0, 0.5 * nx * dx), stage_m=0.6)]
+    base = synthetic_terrain(nx * level, ny * level, dx / level, lambda x, y: 0.02 * y + 0.1 * math.sin(x / 7.0) + 0.1, n=0.03, segments=segs, level=level)
+    p = SolverParams(10.0, 5.0, dt_max_s=0.1, rain=Hyetograph([]), initial_depth=0.0)
+    terrs, mon = [PreparedTerrain(base)] * n, MonitorSet(np.arange(0, nx * ny, 5))
+    o = orc.flat_run(base_arrays(base), design_dict(terrs[0], p), p, mon, want_peak=True, bnd=orc.bnd_dict(base, terrs[0]))
+    assert o["rows_skipped"] > 0
+
+    def run():
+        r = gpu.run_batch(p, terrs, mon, want_peak=True)
+        return gpu.adapter_info(), r
+
+    info, r = run()
+    assert "16x16 tiles" in info, info
+    for a in r:
+        compare_run(a, o, f"{nx}x{ny}")
+        assert a.rows_skipped == o["rows_skipped"]
+    p.locked_dt = np.full(60, 0.1)   # runs out: back to the last snapshot, adaptive from there
+    _, lock = run()
+    _, ref = with_options(gpu, {"impl": 2}, run)
+    for a, b in zip(lock, ref):
+        assert a.steps == b.steps and a.rows_skipped == b.rows_skipped and np.array_equal(a.depth, b.depth)
