@@ -58,6 +58,8 @@ struct PlainCtl {
   unsigned long long rows_skipped;   // dry rows skipped so far (kernel.rs:605-612)
   int seg;           // the storm's piece at t (RainSeg)
   unsigned unsafe;   // bit 0: the state is not known to be bounded, bit 1: never will be (StepK::exact)
+  unsigned gw_flows;  // the inflow groups that flow in the ghost wetness kept (a bit each; ~0: not known)
+  unsigned pad;
 };
 
 struct PlainArgs {
@@ -393,6 +395,7 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int d, int n_blocks, int fi
   }
   __syncthreads();
   if (first && threadIdx.x == 0) {
+    c.gw_flows = ~0u;
     const WarmStart* W = (A.warm && A.warm[d].state) ? &A.warm[d] : nullptr;
     if (W) {
       c.t = W->t; c.dt_cfl = W->dt_cfl; c.acc_rain = W->acc_rain; c.v0 = W->v0; c.volume = W->volume; c.rel_res = W->rel_res;
@@ -414,9 +417,12 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int d, int n_blocks, int fi
     const int R = A.ny + 2;
     unsigned* rw = D.rowwet + (size_t)c.par * R;
     if (P.skip_dry && !(c.k.rain > 0.0f)) {
-      unsigned cnt = 0u;
-      for (int j = 1 + threadIdx.x; j <= A.ny; j += blockDim.x)
-        cnt += (plain_row_dry(rw, D.gwet, j - 1) && plain_row_dry(rw, D.gwet, j) && plain_row_dry(rw, D.gwet, j + 1)) ? 1u : 0u;
+      unsigned cnt = 0u;   // (rows j - 1, j and j + 1 dry: plain_row_dry of each, the loads side by side)
+#pragma unroll 4
+      for (int j = 1 + threadIdx.x; j <= A.ny; j += blockDim.x) {
+        const unsigned w = rw[j - 1] | rw[j] | rw[j + 1] | (D.gwet ? D.gwet[j - 1] | D.gwet[j] | D.gwet[j + 1] : 0u);
+        cnt += w == 0u ? 1u : 0u;
+      }
       if (cnt) atomicAdd(&s_skip, cnt);
     }
     __syncthreads();
@@ -428,7 +434,15 @@ ITR_DEV void plain_finalize_body(const PlainArgs& A, int d, int n_blocks, int fi
     plain_finalize_steps<LOCKED>(A, D, d, first, c, sums);
   }
   __syncthreads();
-  if (D.gwet && !c.done) plain_ghost_wet(A, D.bh, c.inf, D.gwet);   // what the row-band kernel's dry-row test reads
+  if (D.gwet && !c.done) {   // what the dry-row test reads; it changes only with the groups that flow
+    unsigned flows = 0u;
+    for (int g = 0; g < P.inflow.n; ++g) flows |= c.inf[g].y > 0.0f ? 1u << g : 0u;
+    const bool redo = flows != c.gw_flows;
+    __syncthreads();
+    if (threadIdx.x == 0) c.gw_flows = flows;
+    if (redo) plain_ghost_wet(A, D.bh, c.inf, D.gwet);
+    __syncthreads();
+  }
   unsigned long long* dst = reinterpret_cast<unsigned long long*>(D.ctl);
   for (int i = threadIdx.x; i < kWords; i += blockDim.x) dst[i] = reinterpret_cast<const unsigned long long*>(&c)[i];
 }
@@ -548,6 +562,7 @@ ITR_DEV void plain_finalize_steps(const PlainArgs& A, const PlainDesign& D, int 
         // finalize (save still pending) is the current state: nothing to copy back.
         const int pending_save = c.copy_req;
         c = A.snapctl[d];
+        c.gw_flows = ~0u;   // (the flags are of the steps taken back)
         c.locked_live = 0;
         c.copy_req = pending_save == 1 ? 0 : 2;
         A.fallback_t[d] = c.t;
